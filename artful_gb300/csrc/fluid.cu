@@ -9,14 +9,19 @@
  * Same bytes: this unit is built without contraction and with IEEE division and square root, and each
  * float expression keeps the reference's order of operations.  The reference's cell loops are
  * independent within a pass (each pass reads one copy of the fields and writes the other), so one thread
- * a cell computes what it computes.  Two things are ordered: the eddies, which overlap and so run one
- * after another in one block, each eddy's cells in parallel (an eddy touches each cell once); and each
- * ring's mean density, a sum in cell order, which one thread a ring adds up.  The random draws that place
- * the eddies (a xorshift sequence) are made on the host, in the reference's order, for all the steps of
- * a call at once, and copied to the device with their shapes.
+ * a cell computes what it computes.  Two things are ordered: the eddies, which overlap: each cell takes
+ * them in their order, and an eddy changes a cell by that cell's own values alone, so the cells need not
+ * wait for one another; and each ring's mean density, a sum in cell order, which one thread a ring adds
+ * up.  The random draws that place the eddies (a xorshift sequence) are made on the host, in the
+ * reference's order, and travel with the launches as kernel parameters.
  *
- * Work layout: 7 fields of 256 x 1024 floats (7 MB, L2-resident), one allocation; per step five launches
- * on the context's stream (stir, velocities, densities, shift, balance), and the field after the last. */
+ * Work layout: 7 fields of 256 x 1024 floats (7 MB, L2-resident), one allocation.  A step is two launches
+ * on the context's stream: `velocities`, a thread a cell; and `ringStep`, a block a ring, which does all
+ * that follows within the ring: its new densities, its shift along itself, its mean drawn to 1, the next
+ * step's eddies, and after the last step the field.  What bounds a step is latency: the sum in cell order
+ * (1024 dependent additions, 2.1 us) and the two launches; the fields are read and written once.  One
+ * block working through the eddies, and a launch a pass, took 62 us a step; this takes 11 (24 steps
+ * of a 1024 x 256 gas, a call: 1486 -> 265 us; of that the launches as dependent ones 387 -> 265). */
 #include "nvtxRange.h"
 #include "artful_cuda.h"
 
@@ -37,17 +42,23 @@ constexpr int FW = ARTF_CUDA_FLUID_WIDTH;  /* cells around a ring */
 constexpr int FH = ARTF_CUDA_FLUID_HEIGHT; /* rings */
 constexpr float DT = .2f;                  /* fluid.c:28 */
 #define ARC (6.2831853f / (float)FW)       /* fluid.c:29 */
-constexpr int MAX_STEPS = 48;              /* fluid.c:30 */
 constexpr int WARM_STEPS = 60;             /* fluid.c:31 */
 constexpr float WOUND_TIME = 900.f;        /* fluid.c:32 */
 constexpr int EDDIES_A_STEP = 16;          /* fluid.c:232-234: two large, fourteen small */
 constexpr int START_EDDIES = 200;          /* fluid.c:312 */
+constexpr int EDDIES_A_LAUNCH = 128;       /* a launch's room for them */
+constexpr int RING_THREADS = 512;          /* a ring's block: two cells a thread */
 constexpr int FIELD = FW * FH;
 
-/* Per ring: radius, the row's width in radius, orbital and epicyclic terms, sound speed squared, the
- * ring's shift a step in cells, the envelope and fall-off of what shows (fluid.c:270-287). */
-struct Rings {
-    float radius[FH], rowWidth[FH], angular[FH], epicyclic[FH], sound2[FH], slide[FH], envelope[FH], fall[FH];
+/* What a cell's passes take from its ring alone (fluid.c:98-106, 128-135, 155-165, 270-287), formed once on
+ * the host in the reference's float operations (IEEE there and here: the same values; on the device each
+ * cell formed them again with five divisions): its radius and its neighbours', orbital and epicyclic
+ * terms, sound speed squared, the gradients' factors, the cubic its shift reads with, and the envelope
+ * and fall-off of what shows. */
+struct Ring {
+    float radius, up, down, angular, epicyclic, sound2, toCells, toRows, invR, invSpan, invArc, keep, refill;
+    float k0, k1, k2, k3, envelope, fall;
+    int shift;
 };
 
 /* One eddy, placed and shaped on the host (fluid.c:188-201). */
@@ -86,7 +97,7 @@ __device__ __forceinline__ float noise(float x, float y, uint32_t period, uint32
 }
 
 /* fluid.c:82-93 (an index never leaves the field: y0 <= FH - 2, columns wrap) */
-__device__ __forceinline__ float bilinear(const float* __restrict__ a, float x, float y) {
+__device__ __forceinline__ float bilinear(const float* a, float x, float y) {
     const float fy = clampF(y, 0.f, (float)(FH - 1) - .001f);
     const int y0 = (int)fy;
     const float py = fy - (float)y0;
@@ -101,11 +112,11 @@ __device__ __forceinline__ float bilinear(const float* __restrict__ a, float x, 
 /* ---- kernels: one thread a cell, unless said otherwise ------------------------------------------ */
 
 /* fluid.c:291-311: the start, clumps the shear has long been drawing out */
-__global__ void __launch_bounds__(256) seedDensity(float* __restrict__ s, const Rings* __restrict__ rings) {
+__global__ void __launch_bounds__(256) seedDensity(float* __restrict__ s, const Ring* __restrict__ rings) {
     const int cell = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (cell >= FIELD) return;
     const int j = cell / FW, i = cell - j * FW;
-    const float rho = (float)j / (float)(FH - 1), wound = rings->angular[j] * WOUND_TIME / 6.2831853f;
+    const float rho = (float)j / (float)(FH - 1), wound = rings[j].angular * WOUND_TIME / 6.2831853f;
     float turn = (float)i / (float)FW - wound;
     turn -= floorf(turn);
     float sum = 0, amplitude = .5f, total = 0, across = 14.f;
@@ -121,142 +132,198 @@ __global__ void __launch_bounds__(256) seedDensity(float* __restrict__ s, const 
     s[cell] = .06f + 3.4f * ease(.34f, .68f, v) * ease(.34f, .68f, v);
 }
 
-/* fluid.c:202-218: eddies one after another (they overlap), each one's cells at once; one block.  The
- * rows an eddy can reach (its radial test passed) are found first and only they are visited: the test
- * still runs on each, so every cell gets the update the reference gives it. */
-__global__ void __launch_bounds__(1024) stir(float* __restrict__ s, float* __restrict__ vr, float* __restrict__ w,
-                                             const Rings* __restrict__ rings, const Eddy* __restrict__ eddies,
-                                             int count) {
-    __shared__ int lo, hi;
-    for (int e = 0; e < count; ++e) {
-        const Eddy q = eddies[e];
-        if (threadIdx.x == 0) lo = FH, hi = -1;
-        __syncthreads();
-        if ((int)threadIdx.x < FH) {
-            const float dr = rings->radius[threadIdx.x] - q.r0;
-            if (!(dr * dr > 6.25f * q.size * q.size)) {
-                atomicMin(&lo, (int)threadIdx.x);
-                atomicMax(&hi, (int)threadIdx.x);
-            }
+/* A launch's eddies, in their order, as a kernel parameter: a step's 16, or 128 (3.6 KB, under the 4 KB
+ * every driver takes) of a gas's start. */
+template <int N> struct Eddies {
+    int count;
+    Eddy e[N];
+};
+
+/* The launches of a run follow one another at once (programmatic dependent launch): a kernel may start
+ * while the one before it drains, fetches what no kernel writes, and waits here, before its first read of
+ * the fields, until that one has finished and its writes are visible.  The fields' pointers are not
+ * __restrict__: their reads stay below the wait. */
+__device__ __forceinline__ void startNext() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void waitBefore() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+/* How strongly an eddy's shape reaches the cell (ring radius r, column i), fluid.c:202-214: whether it does,
+ * and there its shape and the offsets from its middle.  Columns -reach .. reach: fewer than FW, so a cell
+ * is at one offset at most. */
+__device__ __forceinline__ bool eddyAt(const Eddy& q, float r, int i, float& shape, float& dr, float& dx) {
+    dr = r - q.r0;
+    if (dr * dr > 6.25f * q.size * q.size) return false;
+    const int di = ((i - q.i0 + FW / 2) & (FW - 1)) - FW / 2;
+    if (di > q.reach || di < -q.reach) return false;
+    dx = (float)di * r * ARC;
+    const float d2 = (dr * dr + dx * dx) * q.invSize2;
+    if (d2 > 6.25f) return false;
+    const float g = 1.f - d2 * .16f;
+    shape = g * g * g;
+    return true;
+}
+
+/* What an eddy does to a cell it reaches (fluid.c:215-217): to its velocities, and to its density. */
+__device__ __forceinline__ void stirFlow(const Eddy& q, float r, int i, float& vr, float& w) {
+    float shape, dr, dx;
+    if (!eddyAt(q, r, i, shape, dr, dx)) return;
+    vr -= q.strength * shape * dx / q.size;
+    w += q.strength * shape * dr / q.size;
+}
+
+__device__ __forceinline__ void stirDensity(const Eddy& q, float r, int i, float& s) {
+    float shape, dr, dx;
+    if (eddyAt(q, r, i, shape, dr, dx)) s = clampF(s * (1.f + q.clump * shape), .03f, 8.f);
+}
+
+/* Eddies on their own (those of a gas's start, and of a run's first step): a block a ring, so that an eddy
+ * out of the ring's reach costs the block one uniform test. */
+__global__ void __launch_bounds__(RING_THREADS) stir(float* s, float* vr, float* w, const Ring* __restrict__ rings,
+                                                     const __grid_constant__ Eddies<EDDIES_A_LAUNCH> eddies) {
+    const int j = (int)blockIdx.x;
+    const float r = rings[j].radius;
+    startNext();
+    waitBefore();
+    for (int i = (int)threadIdx.x; i < FW; i += RING_THREADS) {
+        const size_t at = (size_t)j * FW + (size_t)i;
+        float cellS = s[at], cellR = vr[at], cellW = w[at];
+        for (int e = 0; e < eddies.count; ++e) {
+            stirFlow(eddies.e[e], r, i, cellR, cellW);
+            stirDensity(eddies.e[e], r, i, cellS);
         }
-        __syncthreads();
-        const int span = 2 * q.reach + 1; /* columns -reach .. reach: fewer than FW, so each cell once */
-        const int rows = hi - lo + 1;     /* (none reached: not positive) */
-        for (int k = (int)threadIdx.x; k < rows * span; k += (int)blockDim.x) {
-            const int row = k / span, j = lo + row, di = k - row * span - q.reach;
-            const float dr = rings->radius[j] - q.r0;
-            if (dr * dr > 6.25f * q.size * q.size) continue;
-            const float dx = (float)di * rings->radius[j] * ARC;
-            const float d2 = (dr * dr + dx * dx) * q.invSize2;
-            if (d2 > 6.25f) continue;
-            const float g = 1.f - d2 * .16f, shape = g * g * g;
-            const size_t at = (size_t)j * FW + (size_t)((q.i0 + di) & (FW - 1));
-            vr[at] -= q.strength * shape * dx / q.size;
-            w[at] += q.strength * shape * dr / q.size;
-            s[at] = clampF(s[at] * (1.f + q.clump * shape), .03f, 8.f);
-        }
-        __syncthreads();
+        s[at] = cellS, vr[at] = cellR, w[at] = cellW;
     }
 }
 
 /* fluid.c:96-124 */
-__global__ void __launch_bounds__(256) velocities(const float* __restrict__ s, const float* __restrict__ vr,
-                                                  const float* __restrict__ w, float* __restrict__ outR,
-                                                  float* __restrict__ outW, const Rings* __restrict__ rings) {
-    const int cell = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (cell >= FIELD) return;
-    const int j = cell / FW, i = cell - j * FW;
-    const float r = rings->radius[j], invR = 1.f / r, c2 = rings->sound2[j], om = rings->angular[j];
-    const float sw = rings->epicyclic[j];
-    const float toCells = DT / (r * ARC), toRows = DT / rings->rowWidth[j];
+__global__ void __launch_bounds__(256) velocities(const float* s, const float* vr, const float* w, float* outR,
+                                                  float* outW, const Ring* __restrict__ rings) {
+    const int cell = (int)(blockIdx.x * 256 + threadIdx.x); /* (256 divides the field) */
+    const int j = (int)(blockIdx.x * 256) / FW, i = cell - j * FW; /* (a block's cells are of one ring) */
+    const Ring g = rings[j];
+    startNext();
+    waitBefore();
     const int up = atMost(j + 1, FH - 1), down = atLeast(j - 1, 0);
-    const float invSpan = 1.f / (rings->radius[up] - rings->radius[down]), invArc = 1.f / (2.f * r * ARC);
-    const float keep = 1.f - DT * .04f * om;
-    const float x = (float)i - w[cell] * toCells, y = (float)j - vr[cell] * toRows;
+    const float x = (float)i - w[cell] * g.toCells, y = (float)j - vr[cell] * g.toRows;
     const float v0 = bilinear(vr, x, y), w0 = bilinear(w, x, y);
     const float inv = 1.f / s[cell];
-    const float gradR = (s[(size_t)up * FW + i] - s[(size_t)down * FW + i]) * invSpan * inv;
+    const float gradR = (s[(size_t)up * FW + i] - s[(size_t)down * FW + i]) * g.invSpan * inv;
     const float gradPhi = (s[(size_t)j * FW + ((i + 1) & (FW - 1))] - s[(size_t)j * FW + ((i - 1) & (FW - 1))]) *
-                          invArc * inv;
-    const float w1 = w0 + DT * (-sw * v0 - v0 * w0 * invR - c2 * gradPhi);
-    const float v1 = v0 + DT * (2.f * om * w1 + w1 * w1 * invR - c2 * gradR);
-    outW[cell] = clampF(w1 * keep, -.4f, .4f);
-    outR[cell] = clampF(v1 * keep, -.4f, .4f);
+                          g.invArc * inv;
+    const float w1 = w0 + DT * (-g.epicyclic * v0 - v0 * w0 * g.invR - g.sound2 * gradPhi);
+    const float v1 = v0 + DT * (2.f * g.angular * w1 + w1 * w1 * g.invR - g.sound2 * gradR);
+    outW[cell] = clampF(w1 * g.keep, -.4f, .4f);
+    outR[cell] = clampF(v1 * g.keep, -.4f, .4f);
 }
 
-/* fluid.c:126-151 */
-__global__ void __launch_bounds__(256) densities(const float* __restrict__ s, const float* __restrict__ vr,
-                                                 const float* __restrict__ w, float* __restrict__ out,
-                                                 const Rings* __restrict__ rings) {
-    const int cell = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (cell >= FIELD) return;
-    const int j = cell / FW, i = cell - j * FW;
-    const float r = rings->radius[j], invR = 1.f / r;
-    const float toCells = DT / (r * ARC), toRows = DT / rings->rowWidth[j];
+/* fluid.c:126-151: a cell's new density */
+__device__ __forceinline__ float densityAt(const float* s, const float* vr, const float* w, const Ring& g, int j, int i) {
+    const int cell = j * FW + i;
     const int up = atMost(j + 1, FH - 1), down = atLeast(j - 1, 0);
-    const float rUp = rings->radius[up], rDown = rings->radius[down], invSpan = 1.f / (rUp - rDown);
-    const float invArc = 1.f / (2.f * r * ARC);
-    const float drift = -.004f, refill = DT * .002f * rings->angular[j];
-    const float x = (float)i - w[cell] * toCells, y = (float)j - (vr[cell] + drift) * toRows;
+    const float drift = -.004f;
+    const float x = (float)i - w[cell] * g.toCells, y = (float)j - (vr[cell] + drift) * g.toRows;
     const float moved = bilinear(s, x, y);
-    const float spread = (rUp * vr[(size_t)up * FW + i] - rDown * vr[(size_t)down * FW + i]) * invSpan * invR +
-                         (w[(size_t)j * FW + ((i + 1) & (FW - 1))] - w[(size_t)j * FW + ((i - 1) & (FW - 1))]) * invArc;
+    const float spread = (g.up * vr[(size_t)up * FW + i] - g.down * vr[(size_t)down * FW + i]) * g.invSpan * g.invR +
+                         (w[(size_t)j * FW + ((i + 1) & (FW - 1))] - w[(size_t)j * FW + ((i - 1) & (FW - 1))]) * g.invArc;
     const float next = moved * (1.f - DT * clampF(spread, -2.f, 2.f));
-    out[cell] = clampF(next + (1.f - next) * refill, .03f, 8.f);
+    return clampF(next + (1.f - next) * g.refill, .03f, 8.f);
 }
 
-/* fluid.c:153-173: each ring moved along itself by its orbit, a Catmull-Rom cubic held within its two
- * middle neighbours, for the three fields, from the new copies back into the current ones */
-__device__ __forceinline__ float slideCell(const float* __restrict__ in, int i, int b, float k0, float k1, float k2,
-                                           float k3) {
-    const float p0 = in[(i + b - 1) & (FW - 1)], p1 = in[(i + b) & (FW - 1)];
-    const float p2 = in[(i + b + 1) & (FW - 1)], p3 = in[(i + b + 2) & (FW - 1)];
-    return clampF(k0 * p0 + k1 * p1 + k2 * p2 + k3 * p3, lesser(p1, p2), greater(p1, p2));
+/* fluid.c:153-173: a ring moved along itself by its orbit, a Catmull-Rom cubic held within its two middle
+ * neighbours */
+__device__ __forceinline__ float slideCell(const float* in, int i, const Ring& g) {
+    const int at = i + g.shift;
+    const float p0 = in[(at - 1) & (FW - 1)], p1 = in[at & (FW - 1)];
+    const float p2 = in[(at + 1) & (FW - 1)], p3 = in[(at + 2) & (FW - 1)];
+    return clampF(g.k0 * p0 + g.k1 * p1 + g.k2 * p2 + g.k3 * p3, lesser(p1, p2), greater(p1, p2));
 }
 
-__global__ void __launch_bounds__(256) slide(const float* __restrict__ s, const float* __restrict__ vr,
-                                             const float* __restrict__ w, float* __restrict__ outS,
-                                             float* __restrict__ outR, float* __restrict__ outW,
-                                             const Rings* __restrict__ rings) {
-    const int cell = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (cell >= FIELD) return;
-    const int j = cell / FW, i = cell - j * FW;
-    const float cells = rings->slide[j];
-    const float whole = floorf(cells), t = 1.f - (cells - whole), t2 = t * t, t3 = t2 * t;
-    const int b = -(int)whole - 1;
-    const float k0 = -.5f * t + t2 - .5f * t3, k1 = 1.f - 2.5f * t2 + 1.5f * t3;
-    const float k2 = .5f * t + 2.f * t2 - 1.5f * t3, k3 = -.5f * t2 + .5f * t3;
-    const size_t row = (size_t)j * FW;
-    outS[cell] = slideCell(s + row, i, b, k0, k1, k2, k3);
-    outR[cell] = slideCell(vr + row, i, b, k0, k1, k2, k3);
-    outW[cell] = slideCell(w + row, i, b, k0, k1, k2, k3);
-}
-
-/* fluid.c:221-229: a block a ring; its sum in cell order by one thread, as the reference adds it */
-__global__ void __launch_bounds__(256) balance(float* __restrict__ s) {
-    __shared__ float ring[FW];
+/* The rest of a step, within a ring: the new densities from the old (s) and the new velocities (vr, w),
+ * the shift of the three fields along the ring, the mean drawn to 1 (fluid.c:221-229: a sum in cell order,
+ * by one thread, while the others stir the velocities), the next step's eddies, and, when `field` is
+ * given, what shows of the ring (fluid.c:175-186).  Rings read their neighbours' old density and new
+ * velocities and write neither. */
+__global__ void __launch_bounds__(RING_THREADS) ringStep(const float* s, const float* vr, const float* w, float* outS,
+                                                         float* outR, float* outW, const Ring* __restrict__ rings,
+                                                         float* field,
+                                                         const __grid_constant__ Eddies<EDDIES_A_STEP> eddies) {
+    constexpr int CELLS = FW / RING_THREADS;
+    __shared__ __align__(16) float ringS[FW];
+    __shared__ float ringR[FW], ringW[FW];
+    __shared__ uint32_t reaching; /* the eddies that reach the ring at all, a bit each */
     __shared__ float scale;
-    float* row = s + (size_t)blockIdx.x * FW;
-    for (int i = (int)threadIdx.x; i < FW; i += (int)blockDim.x) ring[i] = row[i];
+    const int j = (int)blockIdx.x;
+    const Ring g = rings[j];
+    const size_t row = (size_t)j * FW;
+    if (threadIdx.x < 32) {
+        const int e = (int)threadIdx.x;
+        const float dr = e < eddies.count ? g.radius - eddies.e[e & (EDDIES_A_STEP - 1)].r0 : 0.f;
+        const float size = eddies.e[e & (EDDIES_A_STEP - 1)].size;
+        const uint32_t bits = __ballot_sync(0xFFFFFFFFu, e < eddies.count && !(dr * dr > 6.25f * size * size));
+        if (e == 0) reaching = bits;
+    }
+    startNext();
+    waitBefore();
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) {
+        const int i = (int)threadIdx.x + c * RING_THREADS;
+        ringS[i] = densityAt(s, vr, w, g, j, i);
+        ringR[i] = vr[row + i], ringW[i] = w[row + i];
+    }
+    __syncthreads();
+    float slidS[CELLS], slidR[CELLS], slidW[CELLS];
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) {
+        const int i = (int)threadIdx.x + c * RING_THREADS;
+        slidS[c] = slideCell(ringS, i, g);
+        slidR[c] = slideCell(ringR, i, g);
+        slidW[c] = slideCell(ringW, i, g);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) ringS[threadIdx.x + c * RING_THREADS] = slidS[c];
     __syncthreads();
     if (threadIdx.x == 0) {
         float sum = 0;
-        for (int i = 0; i < FW; ++i) sum += ring[i];
+        const float4* four = reinterpret_cast<const float4*>(ringS);
+#pragma unroll 16
+        for (int i = 0; i < FW / 4; ++i) {
+            const float4 q = four[i];
+            sum += q.x;
+            sum += q.y;
+            sum += q.z;
+            sum += q.w;
+        }
         const float mean = sum * (1.f / (float)FW);
         scale = 1.f + .03f * (1.f / mean - 1.f);
     }
+    /* The eddies near each cell: of the 16 some four reach a ring, and each a few dozen of its 1024 columns,
+     * so most cells are done with a test of columns an eddy. */
+    uint32_t near[CELLS];
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) {
+        const int i = (int)threadIdx.x + c * RING_THREADS;
+        near[c] = 0;
+        for (uint32_t bits = reaching; bits; bits &= bits - 1) {
+            const Eddy& q = eddies.e[__ffs((int)bits) - 1];
+            if (((i - q.i0 + q.reach) & (FW - 1)) <= 2 * q.reach) near[c] |= bits & (0u - bits);
+        }
+        for (uint32_t bits = near[c]; bits; bits &= bits - 1)
+            stirFlow(eddies.e[__ffs((int)bits) - 1], g.radius, i, slidR[c], slidW[c]);
+        outR[row + i] = slidR[c], outW[row + i] = slidW[c];
+    }
     __syncthreads();
-    for (int i = (int)threadIdx.x; i < FW; i += (int)blockDim.x) row[i] = clampF(ring[i] * scale, .03f, 8.f);
-}
-
-/* fluid.c:175-186 */
-__global__ void __launch_bounds__(256) showField(const float* __restrict__ s, float* __restrict__ out,
-                                                 const Rings* __restrict__ rings) {
-    const int cell = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (cell >= FIELD) return;
-    const int j = cell / FW;
-    const float v = s[cell] * rings->envelope[j];
-    out[cell] = rings->fall[j] * ease(.1f, 1.1f, v) * lesser(v, 2.2f);
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) {
+        const int i = (int)threadIdx.x + c * RING_THREADS;
+        float v = clampF(slidS[c] * scale, .03f, 8.f);
+        if (field) {
+            const float shown = v * g.envelope;
+            field[row + i] = g.fall * ease(.1f, 1.1f, shown) * lesser(shown, 2.2f);
+        }
+        for (uint32_t bits = near[c]; bits; bits &= bits - 1)
+            stirDensity(eddies.e[__ffs((int)bits) - 1], g.radius, i, v);
+        outS[row + i] = v;
+    }
 }
 
 }  // namespace
@@ -270,11 +337,9 @@ struct ArtfCudaFluid {
     float* radial[2];
     float* orbital[2];
     float* field;
-    Rings* rings;          /* device copy */
-    Eddy* eddies;          /* device: a call's eddies, in order */
-    Eddy* staged;          /* pinned host: the same */
-    int eddyRoom;
-    Rings host;
+    int cur;               /* which density copy is the current one (the velocities' is always 0) */
+    Ring* rings;           /* device copy */
+    Ring host[FH];
     uint32_t state;        /* fluid.c:49 xorshift32 */
     double time;
 };
@@ -296,11 +361,15 @@ Eddy placeEddy(ArtfCudaFluid* f, bool small) {
     Eddy q;
     const float u = uniform(f);
     q.r0 = f->inner + (f->outer - f->inner) * u * u;
-    int j0 = 0;
-    while (j0 < FH - 1 && f->host.radius[j0] < q.r0) ++j0;
+    int j0 = 0; /* the first ring at or past r0, or the last (the rings' radii ascend) */
+    for (int past = FH - 1; j0 < past;) {
+        const int mid = (j0 + past) / 2;
+        if (f->host[mid].radius < q.r0) j0 = mid + 1;
+        else past = mid;
+    }
     q.i0 = (int)(draw(f) & (FW - 1));
     q.size = q.r0 * (small ? .006f + .02f * uniform(f) : .02f + .1f * uniform(f));
-    const float c = sqrtf(f->host.sound2[j0]);
+    const float c = sqrtf(f->host[j0].sound2);
     q.strength = 0.f;
     if (!small) {
         const float sign = uniform(f) < .5f ? -1.f : 1.f;
@@ -312,54 +381,48 @@ Eddy placeEddy(ArtfCudaFluid* f, bool small) {
     return q;
 }
 
-int reserveEddies(ArtfCudaFluid* f, int count) {
-    if (count <= f->eddyRoom) return ARTF_CUDA_OK;
-    if (cudaStreamSynchronize(f->stream) != cudaSuccess) return artf::failWith(ARTF_CUDA_ELAUNCH, "fluid: sync");
-    cudaFree(f->eddies);
-    cudaFreeHost(f->staged);
-    f->eddies = nullptr, f->staged = nullptr, f->eddyRoom = 0;
-    if (cudaMalloc(&f->eddies, sizeof(Eddy) * count) != cudaSuccess ||
-        cudaMallocHost(&f->staged, sizeof(Eddy) * count) != cudaSuccess)
-        return artf::failWith(ARTF_CUDA_ENOMEM, "fluid: eddy table allocation");
-    f->eddyRoom = count;
-    return ARTF_CUDA_OK;
+/* The next `large` large and `small` small eddies, drawn in that order. */
+template <int N> void drawEddies(ArtfCudaFluid* f, Eddies<N>& q, int large, int small) {
+    q.count = 0;
+    for (int e = 0; e < large; ++e) q.e[q.count++] = placeEddy(f, false);
+    for (int e = 0; e < small; ++e) q.e[q.count++] = placeEddy(f, true);
 }
 
-/* `steps` steps (fluid.c:231-241), after `extra` eddies of the start, and the field after them. */
-int advanceSteps(ArtfCudaFluid* f, int extra, int steps) {
-    const int count = extra + steps * EDDIES_A_STEP;
-    if (int s = reserveEddies(f, count)) return s;
-    /* (the previous call's copy may still read the staging) */
-    if (cudaStreamSynchronize(f->stream) != cudaSuccess) return artf::failWith(ARTF_CUDA_ELAUNCH, "fluid: sync");
-    int n = 0;
-    for (int e = 0; e < extra; ++e) f->staged[n++] = placeEddy(f, false);
-    for (int k = 0; k < steps; ++k) {
-        for (int e = 0; e < 2; ++e) f->staged[n++] = placeEddy(f, false);
-        for (int e = 0; e < 14; ++e) f->staged[n++] = placeEddy(f, true);
-    }
-    cudaError_t e = n ? cudaMemcpyAsync(f->eddies, f->staged, sizeof(Eddy) * n, cudaMemcpyHostToDevice, f->stream)
-                      : cudaSuccess;
-    const int cur = 0; /* each step's shift writes back into the current copies */
-    const unsigned blocks = (FIELD + 255) / 256;
-    if (e == cudaSuccess && extra > 0) {
-        stir<<<1, 1024, 0, f->stream>>>(f->dens[cur], f->radial[cur], f->orbital[cur], f->rings, f->eddies, extra);
-        e = cudaGetLastError();
-    }
-    for (int k = 0; k < steps && e == cudaSuccess; ++k) {
-        stir<<<1, 1024, 0, f->stream>>>(f->dens[cur], f->radial[cur], f->orbital[cur], f->rings,
-                                         f->eddies + extra + k * EDDIES_A_STEP, EDDIES_A_STEP);
-        velocities<<<blocks, 256, 0, f->stream>>>(f->dens[cur], f->radial[cur], f->orbital[cur], f->radial[cur ^ 1],
-                                                  f->orbital[cur ^ 1], f->rings);
-        densities<<<blocks, 256, 0, f->stream>>>(f->dens[cur], f->radial[cur ^ 1], f->orbital[cur ^ 1],
-                                                 f->dens[cur ^ 1], f->rings);
-        slide<<<blocks, 256, 0, f->stream>>>(f->dens[cur ^ 1], f->radial[cur ^ 1], f->orbital[cur ^ 1], f->dens[cur],
-                                             f->radial[cur], f->orbital[cur], f->rings);
-        balance<<<FH, 256, 0, f->stream>>>(f->dens[cur]);
-        e = cudaGetLastError();
+/* A kernel that may start while the stream's work before it drains, for those that wait in waitBefore. */
+template <typename... P, typename... A>
+cudaError_t follow(ArtfCudaFluid* f, void (*kernel)(P...), unsigned blocks, unsigned threads, const A&... args) {
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(blocks), c.blockDim = dim3(threads), c.stream = f->stream, c.attrs = &early, c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+/* `steps` steps, one at least (fluid.c:231-241), after `extra` eddies of the start, and the field after them. */
+int advanceSteps(ArtfCudaFluid* f, int extra, int64_t steps) {
+    Eddies<EDDIES_A_LAUNCH> first;
+    Eddies<EDDIES_A_STEP> q;
+    cudaError_t e = cudaSuccess;
+    for (int left = extra; left > 0 && e == cudaSuccess; left -= EDDIES_A_LAUNCH) {
+        drawEddies(f, first, atMost(left, EDDIES_A_LAUNCH), 0);
+        e = follow(f, stir, FH, RING_THREADS, f->dens[f->cur], f->radial[0], f->orbital[0], f->rings, first);
     }
     if (e == cudaSuccess) {
-        showField<<<blocks, 256, 0, f->stream>>>(f->dens[cur], f->field, f->rings);
-        e = cudaGetLastError();
+        drawEddies(f, first, 2, EDDIES_A_STEP - 2);
+        e = follow(f, stir, FH, RING_THREADS, f->dens[f->cur], f->radial[0], f->orbital[0], f->rings, first);
+    }
+    for (int64_t k = 0; k < steps && e == cudaSuccess; ++k) {
+        const bool last = k == steps - 1;
+        if (last) q.count = 0;
+        else drawEddies(f, q, 2, EDDIES_A_STEP - 2);
+        float *old = f->dens[f->cur], *next = f->dens[f->cur ^ 1];
+        e = follow(f, velocities, FIELD / 256, 256, old, f->radial[0], f->orbital[0], f->radial[1], f->orbital[1],
+                   f->rings);
+        if (e == cudaSuccess)
+            e = follow(f, ringStep, FH, RING_THREADS, old, f->radial[1], f->orbital[1], next, f->radial[0], f->orbital[0],
+                       f->rings, last ? f->field : (float*)nullptr, q);
+        f->cur ^= 1;
     }
     if (e != cudaSuccess) return artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
     return ARTF_CUDA_OK;
@@ -372,8 +435,6 @@ extern "C" void artfCudaFluidFree(ArtfCudaFluid* f) {
     cudaStreamSynchronize(f->stream);
     cudaFree(f->block);
     cudaFree(f->rings);
-    cudaFree(f->eddies);
-    cudaFreeHost(f->staged);
     free(f);
 }
 
@@ -391,7 +452,7 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
     f->ctx = ctx, f->stream = stream, f->inner = inner, f->outer = outer;
     f->state = 0x9E3779B9u, f->time = time;
     if (cudaMalloc(&f->block, sizeof(float) * FIELD * 7) != cudaSuccess ||
-        cudaMalloc(&f->rings, sizeof(Rings)) != cudaSuccess) {
+        cudaMalloc(&f->rings, sizeof f->host) != cudaSuccess) {
         artfCudaFluidFree(f);
         return artf::failWith(ARTF_CUDA_ENOMEM, "fluid: device allocation");
     }
@@ -400,24 +461,33 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
         f->orbital[k] = f->block + FIELD * (3 * k + 2);
     f->field = f->block + FIELD * 6;
     /* the rings (fluid.c:270-290), on the host in float as the reference has them */
-    Rings& g = f->host;
     const float k = 1.f - inner / outer;
     for (int j = 0; j < FH; ++j) {
+        Ring& g = f->host[j];
         const float rho = (float)j / (float)(FH - 1), r = inner / (1.f - rho * k);
-        g.radius[j] = r;
+        g.radius = r;
         const float root = sqrtf(r), om = 1.f / (r * root + spin);
-        g.angular[j] = om;
+        g.angular = om;
         const float kappa2 = om * om * (1.f - 6.f / r + 8.f * spin / (r * root) - 3.f * spin * spin / (r * r));
-        g.epicyclic[j] = greater(kappa2, -.5f * om * om) / (2.f * om);
+        g.epicyclic = greater(kappa2, -.5f * om * om) / (2.f * om);
         const float c = .03f * r * om;
-        g.sound2[j] = c * c;
-        g.slide[j] = om * DT / ARC;
-        g.envelope[j] = ease(inner + .5f, inner + 2.2f, r) * (1.f - .86f * ease(outer * .12f, outer * .8f, r));
-        g.fall[j] = sqrtf(inner / r);
+        g.sound2 = c * c;
+        g.toCells = DT / (r * ARC), g.invR = 1.f / r, g.invArc = 1.f / (2.f * r * ARC);
+        g.keep = 1.f - DT * .04f * om, g.refill = DT * .002f * om;
+        const float cells = om * DT / ARC, whole = floorf(cells), t = 1.f - (cells - whole), t2 = t * t, t3 = t2 * t;
+        g.shift = -(int)whole - 1;
+        g.k0 = -.5f * t + t2 - .5f * t3, g.k1 = 1.f - 2.5f * t2 + 1.5f * t3;
+        g.k2 = .5f * t + 2.f * t2 - 1.5f * t3, g.k3 = -.5f * t2 + .5f * t3;
+        g.envelope = ease(inner + .5f, inner + 2.2f, r) * (1.f - .86f * ease(outer * .12f, outer * .8f, r));
+        g.fall = sqrtf(inner / r);
     }
-    for (int j = 0; j < FH; ++j)
-        g.rowWidth[j] = (g.radius[atMost(j + 1, FH - 1)] - g.radius[atLeast(j - 1, 0)]) * (j == 0 || j == FH - 1 ? 1.f : .5f);
-    cudaError_t e = cudaMemcpyAsync(f->rings, &f->host, sizeof(Rings), cudaMemcpyHostToDevice, stream);
+    for (int j = 0; j < FH; ++j) {
+        Ring& g = f->host[j];
+        g.up = f->host[atMost(j + 1, FH - 1)].radius, g.down = f->host[atLeast(j - 1, 0)].radius;
+        g.invSpan = 1.f / (g.up - g.down);
+        g.toRows = DT / ((g.up - g.down) * (j == 0 || j == FH - 1 ? 1.f : .5f));
+    }
+    cudaError_t e = cudaMemcpyAsync(f->rings, f->host, sizeof f->host, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(f->block, 0, sizeof(float) * FIELD * 7, stream);
     if (e == cudaSuccess) {
         seedDensity<<<(FIELD + 255) / 256, 256, 0, stream>>>(f->dens[0], f->rings);
@@ -455,12 +525,8 @@ extern "C" int artfCudaFluidStep(ArtfCudaFluid* f, int64_t steps, double time) {
     if (!f || steps < 0 || !isfinite(time)) return artf::failWith(ARTF_CUDA_EINVAL, "fluid step: no fluid, or bad steps or time");
     cudaStream_t stream = nullptr;
     if (int s = artf::contextStream(f->ctx, &stream)) return s;
-    /* in runs of at most 4 x 48 steps, so that the eddy staging stays small */
-    for (int64_t done = 0; done < steps;) {
-        const int run = (int)(steps - done < 4 * MAX_STEPS ? steps - done : 4 * MAX_STEPS);
-        if (int s = advanceSteps(f, 0, run)) return s;
-        done += run;
-    }
+    if (steps > 0)
+        if (int s = advanceSteps(f, 0, steps)) return s;
     f->time = time;
     return ARTF_CUDA_OK;
 }

@@ -148,3 +148,17 @@ def test_counted_steps_equal_the_advances(lib, ctx):
     finally:
         a.free()
         b.free()
+
+
+@pytest.mark.parametrize("inner,outer,spin", [(6.0, 7.0, 0.0), (1.3, 80.0, 0.99), (9.0, 34.0, -0.9)])
+def test_each_run_of_steps_equals_the_oracle(lib, ctx, oracle_lib, inner, outer, spin):
+    """Runs of one step, of two and of a whole call's 48, each ending in a field: a narrow disc, whose
+    eddies are wider than it is; a wide one, whose rings the largest reach around column 0; a retrograde one."""
+    a = GpuFluid(lib, ctx, inner, outer, spin, 0.0)
+    b = binding.Fluid(oracle_lib, "oracle", inner, outer, spin, 0.0)
+    for target in (None, 0.25, 0.65, 10.3):
+        if target is not None:
+            assert a.advance(target) == b.advance(target)
+        np.testing.assert_array_equal(a.read()[0].view(np.uint32), b.read()[0].view(np.uint32))
+    a.free()
+    b.free()
