@@ -452,7 +452,7 @@ static const int64_t kRaysApart = 64000000, kRaysABand = 8000000;
  * list, in the given precision. */
 static int launchBand(ArtfCuda* ctx, artf::TraceLaunch& l, int precision) {
     if (precision == ARTF_CUDA_MIXED) {
-        if (int s = reserveTable(ctx, 1)) return s;
+        alignas(16) unsigned char view[artf::kMixedViewBytesMax];
         const int height = (int)l.frame.size[1];
         const int rowBegin = l.tileRows > 0 ? l.tileRowBegin * 4 : 0;
         const int rows = l.tileRows > 0 ? (rowBegin + l.tileRows * 4 < height ? l.tileRows * 4 : height - rowBegin)
@@ -461,14 +461,11 @@ static int launchBand(ArtfCuda* ctx, artf::TraceLaunch& l, int precision) {
         const size_t np = l.rayCount > 0 ? 0 : artf::mixedRayPlanes(l, l.frame);
         if (np)
             if (int s = reservePlanes(ctx, pixels * np)) return s;
-        if (int s = waitStaging(ctx)) return s;
         int tiles = 0;
         const int units = artf::mixedFillView(l, l.frame, l.frame64, l.map, l.fluid, l.hdr, l.ends,
-                                              np ? ctx->planes : nullptr, 0, 0, ctx->stage, &tiles);
+                                              np ? ctx->planes : nullptr, 0, 0, view, &tiles);
         if (int s = reserveOrder(ctx, tiles, units)) return s;
-        if (int s = sendTable(ctx, 1)) return s;
-        const cudaError_t e = artf::launchMixedTable(l, ctx->table, 1, units, np ? pixels : 0, tiles, ctx->order,
-                                                     ctx->stage);
+        const cudaError_t e = artf::launchMixedTable(l, nullptr, 1, units, np ? pixels : 0, tiles, ctx->order, view);
         if (e != cudaSuccess) return fail(ARTF_CUDA_ELAUNCH, "mixed trace launch: %s", cudaGetErrorString(e));
         return ARTF_CUDA_OK;
     }
@@ -1035,26 +1032,23 @@ extern "C" int artfCudaAutotune(ArtfCuda* ctx, const ArtfCudaView* views, int co
 
     /* coordinate descent over the launch shape, from the defaults */
     static const int blocks[] = {64, 128, 192, 256};
-    static const int waits[] = {16, 32, 64, 128, 256};
-    static const int batches[] = {16, 24, 28, 32};
-    static const int refills[] = {16, 24, 28, 32};
-    int best[4] = {128, 64, 32, 32};
-    const int* values[4] = {blocks, waits, batches, refills};
-    const int counts[4] = {4, 5, 4, 4};
+    static const int refills[] = {4, 8, 16, 32};
+    int best[2] = {128, 32};
+    const int* values[2] = {blocks, refills};
     const int repeats = 3;
     float bestMs = 0.f;
     int trials = 0;
-    l.blockSize = best[0], l.compactEvery = best[1], l.fp64Batch = best[2], l.refillBatch = best[3];
+    l.blockSize = best[0], l.refillBatch = best[1];
     if ((status = timeBatch(ctx, l, count, units, combine, tiles, repeats, &bestMs))) return status;
     const float defaultMs = bestMs;
     ++trials;
     for (int pass = 0; pass < 2; ++pass)
-        for (int d = 0; d < 4; ++d)
-            for (int c = 0; c < counts[d]; ++c) {
-                int trial[4] = {best[0], best[1], best[2], best[3]};
+        for (int d = 0; d < 2; ++d)
+            for (int c = 0; c < 4; ++c) {
+                int trial[2] = {best[0], best[1]};
                 if (values[d][c] == best[d]) continue;
                 trial[d] = values[d][c];
-                l.blockSize = trial[0], l.compactEvery = trial[1], l.fp64Batch = trial[2], l.refillBatch = trial[3];
+                l.blockSize = trial[0], l.refillBatch = trial[1];
                 float ms = 0.f;
                 if ((status = timeBatch(ctx, l, count, units, combine, tiles, repeats, &ms))) return status;
                 ++trials;
@@ -1064,9 +1058,9 @@ extern "C" int artfCudaAutotune(ArtfCuda* ctx, const ArtfCudaView* views, int co
                 }
             }
     ctx->tuned.blockSize = best[0];
-    ctx->tuned.compactEvery = best[1];
-    ctx->tuned.fp64Batch = best[2];
-    ctx->tuned.refillBatch = best[3];
+    ctx->tuned.compactEvery = 256; /* (nothing waits for a round any more: the two have one value) */
+    ctx->tuned.fp64Batch = 32;
+    ctx->tuned.refillBatch = best[1];
     ctx->tuned.ms = bestMs;
     ctx->tuned.defaultMs = defaultMs;
     ctx->tuned.trials = trials;

@@ -116,6 +116,20 @@ ARTF_HD double rootR(double x) { return sqrt(x); }
 #endif
 ARTF_HD float rootR(float x) { return sqrtf(x); }
 
+/* Two products summed, and a product that stands by itself.  Where multiply-adds may be fused there are
+ * two ways to round a b + c d, and the compiler's choice moves with the code around it, and with it the
+ * last bits of an image.  A unit that defines ARTF_PINNED_FMA has them settled: sum2 and diff2 fuse the
+ * first product, and `apart` rounds a product that a fused sum could swallow.  Elsewhere they are the
+ * plain expressions (the exact trace fuses nothing; in double the choice is far below float's rounding). */
+template <typename R> ARTF_HD R sum2(R a, R b, R c, R d) { return a * b + c * d; }
+template <typename R> ARTF_HD R diff2(R a, R b, R c, R d) { return a * b - c * d; }
+template <typename R> ARTF_HD R apart(R a, R b) { return a * b; }
+#if defined(__CUDA_ARCH__) && defined(ARTF_PINNED_FMA)
+template <> __device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+template <> __device__ __forceinline__ float diff2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+template <> __device__ __forceinline__ float apart(float a, float b) { return __fmul_rn(a, b); }
+#endif
+
 /* ---- the debug build's bounds checks -------------------------------------------------------------
  * Built with ARTF_CUDA_DEBUG_BOUNDS, every table row or entry the shading reads is checked against its
  * own region of the map or fluid (not only the buffer, which the clamps below keep every read inside),
@@ -498,7 +512,7 @@ template <typename R> ARTF_HD R turnsOf(R y, R x) {
     if (ay > ax) r = KF(1.57079633) - r;
     if (x < R(0)) r = KF(3.14159265) - r;
     if (y < R(0)) r = R(0) - r;
-    return r * KF(.15915494);
+    return apart(r, KF(.15915494));
 }
 
 /* lens.inc:44-54: sine of an angle in turns, folded to a quarter turn, odd polynomial. */
@@ -537,7 +551,7 @@ ARTF_HD uint32_t cubeHash(uint32_t x, uint32_t y, uint32_t z) {
 
 /* lens.inc:69-86: one layer of hashed-cube stars at direction dir, added to rgb. */
 template <typename R> ARTF_HD void starLayer(const R* dir, R cells, int32_t density, float size, R gain, R* rgb) {
-    const R px = dir[0] * cells, py = dir[1] * cells, pz = dir[2] * cells;
+    const R px = apart(dir[0], cells), py = apart(dir[1], cells), pz = apart(dir[2], cells);
     const R cx = floorR(px), cy = floorR(py), cz = floorR(pz);
     const uint32_t h = cubeHash((uint32_t)truncI(cx), (uint32_t)truncI(cy), (uint32_t)truncI(cz));
     if (!(density > (int32_t)(h & 255u))) return;
@@ -545,7 +559,7 @@ template <typename R> ARTF_HD void starLayer(const R* dir, R cells, int32_t dens
     const R ex = px - cx - R(float((h >> 8) & 255u)) * inv255;
     const R ey = py - cy - R(float((h >> 16) & 255u)) * inv255;
     const R ez = pz - cz - R(float((h >> 24) & 255u)) * inv255;
-    const R d2 = ex * ex + ey * ey + ez * ez;
+    const R d2 = sum2(ex, ex, ey, ey) + ez * ez;
     R light = maxX(R(1) - d2 * R(1.f / (size * size)), R(0));
     light = light * light * gain;
     const R warm = R(float((h >> 3) & 255u)) * inv255;
@@ -559,11 +573,11 @@ template <typename R> ARTF_HD void starLayer(const R* dir, R cells, int32_t dens
 template <typename R> ARTF_HD R shadeCrossing(const Frame<R>& f, R rhoScale, const float* map, const float* fluid,
                                               const RayConst<R>& c, const Crossing<R>& x, R& through, R* sum,
                                               R* turnOut) {
-    const R turn = turnsOf(x.cy, x.cx) + x.psiC * KF(.15915494);
-    const R rate = (divR(x.cx * x.vy - x.cy * x.vx, maxX(x.cx * x.cx + x.cy * x.cy, KF(1e-6))) + x.dragC) * KF(.15915494);
+    const R turn = x.psiC * KF(.15915494) + turnsOf(x.cy, x.cx);
+    const R rate = (divR(diff2(x.cx, x.vy, x.cy, x.vx), maxX(sum2(x.cx, x.cx, x.cy, x.cy), KF(1e-6))) + x.dragC) * KF(.15915494);
     /* gas seen at a slant is deeper */
     const R slope = divR(x.wc, x.uc);
-    const R speed2 = x.vx * x.vx + x.vy * x.vy + (x.vz * x.vz + slope * slope);
+    const R speed2 = sum2(x.vx, x.vx, x.vy, x.vy) + sum2(slope, slope, x.vz, x.vz);
     const R mu = maxX(divSqrtR(absR(x.vz), speed2), KF(.02));
     const R slant = divR(divR(f.thickness, R(3)), mu);
     const R reach = minX(divR(f.discHeight, maxX(absR(x.vz), KF(1e-5))), c.step * KF(1.5));
@@ -578,18 +592,18 @@ template <typename R> ARTF_HD R shadeCrossing(const Frame<R>& f, R rhoScale, con
         const R uk = x.uc + x.wc * ds;
         const R rhoK = (R(1) - f.inner * uk) * rhoScale;
         const bool inside = rhoK > R(0) && rhoK < R(1);
-        const R rowPos = (inside ? rhoK : R(0)) * R(ARTF_CUDA_MAP_HEIGHT - 1);
+        const R rowPos = apart(inside ? rhoK : R(0), R(ARTF_CUDA_MAP_HEIGHT - 1));
         const R rowFloor = minX(floorR(rowPos), R(ARTF_CUDA_MAP_HEIGHT - 2));
         const R rowPart = rowPos - rowFloor;
         const int32_t row0 = truncI(rowFloor), row1 = row0 + 1;
         inBounds(f.fault, kBoundsGasRow, row0, ARTF_CUDA_MAP_HEIGHT - 1); /* (row0 and row1) */
         const R speed0 = ringSpeedAt(f, map, row0), speed1 = ringSpeedAt(f, map, row1);
-        const R turnK = turn + (inside ? rate * ds : R(0));
+        const R turnK = turn + (inside ? apart(rate, ds) : R(0));
         const R d0 = rowAt(map, mapCount, 0, ARTF_CUDA_MAP_WIDTH, row0, turnK - speed0 * c.time);
         const R d1 = rowAt(map, mapCount, 0, ARTF_CUDA_MAP_WIDTH, row1, turnK - speed1 * c.time);
         R density = d0 + (d1 - d0) * rowPart;
         /* the fluid, each ring turned on since it was stepped */
-        const R fluidPos = (inside ? rhoK : R(0)) * R(ARTF_CUDA_FLUID_HEIGHT - 1);
+        const R fluidPos = apart(inside ? rhoK : R(0), R(ARTF_CUDA_FLUID_HEIGHT - 1));
         const R fluidFloor = minX(floorR(fluidPos), R(ARTF_CUDA_FLUID_HEIGHT - 2));
         const int32_t fluidRow = truncI(fluidFloor);
         inBounds(f.fault, kBoundsFluidRow, fluidRow, ARTF_CUDA_FLUID_HEIGHT - 1); /* (and the row after) */
@@ -648,12 +662,12 @@ template <typename R> ARTF_HD R shadeCrossing(const Frame<R>& f, R rhoScale, con
 
 /* The escape direction in the sky's frame: the last chord's end turned by psi (lens.inc:316-321). */
 template <typename R> ARTF_HD void skyDirection(const R* away, R awayPsi, R* dir) {
-    const R invAway = invSqrtR(maxX(away[0] * away[0] + away[1] * away[1] + away[2] * away[2], KF(1e-12)));
+    const R invAway = invSqrtR(maxX(sum2(away[0], away[0], away[1], away[1]) + away[2] * away[2], KF(1e-12)));
     const R psiTurns = awayPsi * KF(.15915494);
     const R sine = sineOf(psiTurns), cosine = sineOf(psiTurns + KF(.25));
     const R x = away[0] * invAway, y = away[1] * invAway, m = away[2] * invAway;
-    dir[0] = x * cosine - y * sine;
-    dir[1] = x * sine + y * cosine;
+    dir[0] = diff2(x, cosine, y, sine);
+    dir[1] = sum2(x, sine, y, cosine);
     dir[2] = m;
 }
 
@@ -664,7 +678,7 @@ template <typename R> ARTF_HD void shadeSky(const Frame<R>& f, const float* map,
     starLayer(dir, KF(90.), 26, .1f, KF(1.6), rgb);
     starLayer(dir, KF(240.), 70, .17f, KF(.22), rgb);
     const R skyTurn = turnsOf(dir[1], dir[0]);
-    const R heightPos = (dir[2] * KF(.5) + KF(.5)) * R(ARTF_CUDA_SKY_HEIGHT - 1);
+    const R heightPos = apart(dir[2] * KF(.5) + KF(.5), R(ARTF_CUDA_SKY_HEIGHT - 1));
     const R skyFloor = minX(floorR(heightPos), R(ARTF_CUDA_SKY_HEIGHT - 2));
     const int32_t skyRow = truncI(skyFloor);
     inBounds(f.fault, kBoundsSkyRow, skyRow, ARTF_CUDA_SKY_HEIGHT - 1); /* (and the row after) */

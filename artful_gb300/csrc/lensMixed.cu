@@ -18,18 +18,26 @@
  *   PSI      psi, the frame-drag angle, is summed with a compensated (two-sum) accumulator, and the
  *            endpoint's Mino time is formed in FP64 from the step count: neither drifts over 192 steps.
  * The radial and polar sub-steps are independent (u'' depends on u alone, n'' on n alone), so a guard
- * costs wide work only for the part that needs it.  The disc and sky shading stay in FP32.  Built with
- * the fast FP32 flags; in double, + - * are IEEE and / and sqrt are refined hardware estimates (within
- * an ulp or two, lensCore.cuh), as in the plain FP64 trace.  At the headline frame the double-float
- * sub-steps give the FP64 ones' bits, rounded to float, for every pixel.
+ * costs wide work only for the part that needs it; and u'' and n_z'' are the same cubic with other
+ * coefficients, so one wide step in the code serves both turning points, and a warp runs it once for the
+ * lanes at either.  The disc and sky shading stay in FP32.  Built with the fast FP32 flags; in double,
+ * + - * are IEEE and / and sqrt are refined hardware estimates (within an ulp or two, lensCore.cuh), as in
+ * the plain FP64 trace.  At the headline frame the double-float sub-steps give the FP64 ones' bits, rounded
+ * to float, for every pixel.
  *
- * Scheduling (traceMixedQueue): a warp pays for a wide sub-step whatever number of its lanes take part.
- * So wide work runs in warp-wide rounds: lanes that need a wide sub-step (or a new ray's set-up) wait,
- * keeping their FP32 results, while the others keep stepping in FP32; a round runs when `batch` lanes
- * wait, when no lane can move without one, or after a bounded wait.  Pixels of every view of a batch
- * come from one device queue (work stealing across views of uneven size), a lane at a time, by warp
- * ballot and shuffle.  Every lane computes exactly what the per-ray path (traceRayMixed) computes, in
- * the same order: the schedule changes when, never what.  A single frame is a batch of one view. */
+ * Scheduling (mixedTiles): a persistent grid of warps takes slots from one device queue (a slot: one ray of
+ * each pixel of an 8 x 4 tile; heavy tiles first; views of uneven size share the queue), and a warp traces
+ * its 32 rays together, each step's wide sub-steps at once.  Neighbouring rays turn within a step or two of
+ * one another, so a wide step serves most of a warp at a time, and a ray's step costs nothing for the
+ * schedule's sake.  (Lanes that waited for full rounds of wide steps and were refilled one by one, as an
+ * FP64 wide step wanted, paid 80 thread instructions a step in votes and flags: 2.15 against 1.61 ms for the
+ * 1080p x 4 frame, 7.63 against 5.51 for 64 views.)  What a step costs is issue slots (71 % of them used, FMA
+ * pipe 50 % busy), so the FP32 step runs its coordinates in pairs with packed instructions (mixedStep: 1.86
+ * -> 1.76 ms), the wide step is one code path (1.74 -> 1.61 with the counts out of registers) and each float
+ * rounding is written out or pinned (ARTF_PINNED_FMA): whatever registers a kernel is given, its images are
+ * the same bits.  A frame of fewer rays than the GPU's warps could take is bound by its longest ray's
+ * latency; there warps take fewer rays each (mixedGrid). */
+#define ARTF_PINNED_FMA 1 /* every float sum of two products rounds the same in every kernel (lensCore.cuh) */
 #define ARTF_FAST_FP64 1 /* FP64 division and square roots by refined hardware estimates (lensCore.cuh) */
 #define ARTF_FP64_NEWTON_STEPS 1 /* one refinement: ~40 bits, far below float's rounding (3.4 % faster) */
 #include "lensKernel.cuh"
@@ -90,23 +98,22 @@ struct MixedParams {
     unsigned long long* counters;
     float stepScale;
     int maxSteps;
+    int lanesLog2;    /* a warp's rays at a time: 2^lanesLog2 of its lanes */
     uint32_t guards;  /* ARTF_CUDA_GUARD_* */
-    int batch;        /* lanes waiting before a warp runs an FP64 round */
-    int refill;       /* idle lanes before a warp starts new rays (an FP64 set-up each) */
-    int maxWait;      /* iterations a lane waits at most */
 };
 
 /* One ray's state between steps. */
 struct MixedRay {
     RayConst<float> c;
-    Ff big, uA, uB, uC, xiA;           /* the coefficients the wide sub-steps use, as double-float pairs */
-    double step;
+    float stepLo, uALo, uBLo, uCLo, xiALo; /* the low halves of the coefficients the wide sub-steps use */
     RayState<float> s;                 /* s.psi stays 0: a step returns psi's increment */
-    float psiHi, psiLo, through, sum[3], hitR, hitPhi;
+    float psiHi, psiLo, through, sum[3];
     int i;
-    unsigned crossings, wide;
-    bool lit;
+    unsigned crossings;                /* and bit 31 once the disc lit the ray */
+    unsigned wide, turns;              /* wide steps and those in the horizon's band, radial and polar turning
+                                        * points: two counts a word, a ray's 384 steps at most */
 };
+constexpr unsigned kLit = 0x80000000u;
 
 /* Float <-> double conversions on the integer pipe.  On this GPU a conversion to double costs an FP64
  * instruction and one to float two, on the narrow FP64 pipe, while the integer pipe idles: these take a
@@ -144,15 +151,6 @@ __device__ __noinline__ float narrow(double d) {
         bits = 0x7f800000u; /* too large, or infinite */
     }
     return __uint_as_float(sign | bits);
-}
-
-__device__ __forceinline__ double ffWide(Ff a);
-__device__ __forceinline__ RayConst<double> wideConst(const MixedRay& r) {
-    RayConst<double> c;
-    c.big = ffWide(r.big), c.step = r.step, c.uA = ffWide(r.uA), c.uB = ffWide(r.uB), c.uC = ffWide(r.uC);
-    c.xiA = ffWide(r.xiA);
-    c.invEnergy = c.xi = c.moved = c.time = 0.0; /* (not read by the sub-steps) */
-    return c;
 }
 
 /* ---- double-float arithmetic --------------------------------------------------------------------------
@@ -201,63 +199,118 @@ __device__ __forceinline__ Ff ffProd(float a, float b) {
 }
 __device__ __forceinline__ Ff ffScale(Ff a, float powerOfTwo) { return Ff{a.hi * powerOfTwo, a.lo * powerOfTwo}; }
 
-/* The step's terms (stepTerms in lensCore.cuh) in double-float from the float step: its square is exact
- * as a pair, the halves and eighth exact, the sixths products by the float 1/6 as there. */
-struct StepTermsFf {
-    Ff half, eighth, halfSquare, sixthSquare, sixth;
+/* x (A + x (B + x C)): what u'' is of u, and n_z'' of n_z with B = 0 and C = -2 a^2
+ * (a^2 n_z - (K + 2 a^2 n_z^2) n_z, and A is a^2 - K for both). */
+struct Cubic {
+    Ff A, B, C;
 };
-__device__ __forceinline__ StepTermsFf stepTermsFf(float step) {
-    const Ff step2 = ffProd(step, step);
-    StepTermsFf t;
-    t.half = Ff{step * .5f, 0.f}, t.eighth = ffScale(step2, .125f), t.halfSquare = ffScale(step2, .5f);
-    t.sixthSquare = ffMulF(step2, 1.f / 6.f), t.sixth = ffProd(step, 1.f / 6.f);
-    return t;
+__device__ __forceinline__ Ff ffCubic(const Cubic& f, Ff x) {
+    return ffMul(x, ffAdd(f.A, ffMul(x, ffAdd(f.B, ffMul(x, f.C)))));
 }
-__device__ __forceinline__ StepTerms<double> wideTerms(const StepTermsFf& t) {
-    StepTerms<double> w;
-    w.half = ffWide(t.half), w.eighth = ffWide(t.eighth), w.halfSquare = ffWide(t.halfSquare);
-    w.sixthSquare = ffWide(t.sixthSquare), w.sixth = ffWide(t.sixth);
-    return w;
+/* One Nystrom step (lens.inc:165-192) of x'' = cubic(x) in double-float, from x and its rate v in float:
+ * the motion of u at a radial turning point and of n_z at a polar one are this same step, so a warp runs
+ * it once for the lanes at either. */
+__device__ __forceinline__ void motionFf(const Cubic& f, float step, float x, float v, Ff& nextX, Ff& nextV, Ff& k1) {
+    const Ff step2 = ffProd(step, step), xf{x, 0.f};
+    k1 = ffCubic(f, xf);
+    const Ff mid = ffAdd(ffAdd(xf, ffProd(step * .5f, v)), ffMul(ffScale(step2, .125f), k1));
+    const Ff k2 = ffCubic(f, mid);
+    const Ff xv = ffAdd(xf, ffProd(step, v));
+    const Ff k3 = ffCubic(f, ffAdd(xv, ffMul(ffScale(step2, .5f), k2)));
+    nextX = ffAdd(xv, ffMul(ffMulF(step2, 1.f / 6.f), ffAdd(k1, ffScale(k2, 2.f))));
+    nextV = ffAdd(Ff{v, 0.f}, ffMul(ffProd(step, 1.f / 6.f), ffAdd(ffAdd(k1, k3), ffScale(k2, 4.f))));
 }
-/* bendAt: x (uA + x (uB + x uC)) */
-__device__ __forceinline__ Ff ffBend(const MixedRay& r, Ff x) {
-    return ffMul(x, ffAdd(r.uA, ffMul(x, ffAdd(r.uB, ffMul(x, r.uC)))));
+
+/* ---- the FP32 step ------------------------------------------------------------------------------------
+ * Blackwell's packed instructions do two float operations in one issue slot, each rounded as by itself.
+ * The step's four coordinates, u and n, go through the same Nystrom stages with the same factors, so they
+ * ride in two pairs, (n_x, n_y) and (u, n_z), and the two drag rates in one. */
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 pack(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
-/* radialMotionWith (lensCore.cuh) in double-float, in its order of operations. */
-__device__ __forceinline__ void radialMotionFf(const MixedRay& r, const StepTermsFf& t, float u, float w, Ff& nextU,
-                                               Ff& nextW, Ff& k1) {
-    const Ff uf{u, 0.f};
-    k1 = ffBend(r, uf);
-    const Ff midU = ffAdd(ffAdd(uf, ffMulF(t.half, w)), ffMul(t.eighth, k1));
-    const Ff k2 = ffBend(r, midU);
-    const Ff uw = ffAdd(uf, ffProd(r.c.step, w));
-    const Ff endU = ffAdd(uw, ffMul(t.halfSquare, k2));
-    const Ff k3 = ffBend(r, endU);
-    nextU = ffAdd(uw, ffMul(t.sixthSquare, ffAdd(k1, ffAdd(k2, k2))));
-    nextW = ffAdd(Ff{w, 0.f}, ffMul(t.sixth, ffAdd(ffAdd(k1, k3), ffMulF(k2, 4.f))));
+__device__ __forceinline__ void unpack(F2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
-/* polarAxisWith (lensCore.cuh) in double-float, in its order of operations. */
-__device__ __forceinline__ void polarAxisFf(Ff a2, const MixedRay& r, const StepTermsFf& t, float nz, float vz,
-                                            Ff& nextNz, Ff& nextVz, Ff& a1) {
-    const Ff twoA2 = ffScale(a2, 2.f), nzf{nz, 0.f};
-    const Ff c1 = ffAdd(r.big, ffMul(twoA2, ffProd(nz, nz)));
-    a1 = ffSub(ffMulF(a2, nz), ffMulF(c1, nz));
-    const Ff midN = ffAdd(ffAdd(nzf, ffMulF(t.half, vz)), ffMul(t.eighth, a1));
-    const Ff c2 = ffAdd(r.big, ffMul(twoA2, ffMul(midN, midN)));
-    const Ff a2s = ffSub(ffMul(a2, midN), ffMul(c2, midN));
-    const Ff nv = ffAdd(nzf, ffProd(r.c.step, vz));
-    const Ff endN = ffAdd(nv, ffMul(t.halfSquare, a2s));
-    const Ff c3 = ffAdd(r.big, ffMul(twoA2, ffMul(endN, endN)));
-    const Ff a3 = ffSub(ffMul(a2, endN), ffMul(c3, endN));
-    nextNz = ffAdd(nv, ffMul(t.sixthSquare, ffAdd(a1, ffAdd(a2s, a2s))));
-    nextVz = ffAdd(Ff{vz, 0.f}, ffMul(t.sixth, ffAdd(ffAdd(a1, a3), ffMulF(a2s, 4.f))));
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 both(float a) { return pack(a, a); }
+
+__device__ __forceinline__ float bendPoly(const RayConst<float>& c, float x) {
+    return __fmaf_rn(x, __fmaf_rn(x, c.uC, c.uB), c.uA);
+}
+__device__ __forceinline__ float axisAccel(float a2, float c, float z) { return __fmaf_rn(a2, z, -__fmul_rn(c, z)); }
+
+/* nystromStep (lensCore.cuh), each rounding written out as the scalar code's compiles: x + (y + y) is
+ * fma(2, y, x), which rounds the same. */
+__device__ __forceinline__ void mixedStep(float a, const RayConst<float>& c, const RayState<float>& s, StepOut<float>& o) {
+    const StepTerms<float> t = stepTerms(c.step);
+    const float a2 = a * a, twoA2 = 2.f * a2;
+    const F2 h = both(c.step), half = both(t.half), eighth = both(t.eighth), halfSq = both(t.halfSquare);
+    const F2 sixthSq = both(t.sixthSquare), sixth = both(t.sixth), two = both(2.f), four = both(4.f);
+    const F2 n = pack(s.n[0], s.n[1]), v = pack(s.v[0], s.v[1]), q = pack(s.u, s.n[2]), w = pack(s.w, s.v[2]);
+    const float k1 = __fmul_rn(s.u, bendPoly(c, s.u));
+    const float c1 = __fmaf_rn(twoA2, __fmul_rn(s.n[2], s.n[2]), c.big);
+    const float a1z = axisAccel(a2, c1, s.n[2]);
+    const F2 a1 = mul2(both(-c1), n), r1 = pack(k1, a1z);
+    const F2 midN = fma2(eighth, a1, fma2(half, v, n)), midQ = fma2(eighth, r1, fma2(half, w, q));
+    float midU, midZ;
+    unpack(midQ, midU, midZ);
+    const float k2 = __fmul_rn(midU, bendPoly(c, midU));
+    const float c2 = __fmaf_rn(twoA2, __fmul_rn(midZ, midZ), c.big);
+    const F2 a2s = mul2(both(-c2), midN), r2 = pack(k2, axisAccel(a2, c2, midZ));
+    const F2 nv = fma2(h, v, n), qw = fma2(h, w, q);
+    const F2 endN = fma2(halfSq, a2s, nv), endQ = fma2(halfSq, r2, qw);
+    float endU, endZ;
+    unpack(endQ, endU, endZ);
+    const float c3 = __fmaf_rn(twoA2, __fmul_rn(endZ, endZ), c.big);
+    /* (the product against zero: a bare one would be fused into the sum after it) */
+    const F2 a13 = add2(a1, fma2(both(-c3), endN, both(0.f)));
+    const F2 r13 = pack(__fmaf_rn(endU, bendPoly(c, endU), k1), __fadd_rn(a1z, axisAccel(a2, c3, endZ)));
+    const F2 nextN = fma2(sixthSq, fma2(two, a2s, a1), nv), nextQ = fma2(sixthSq, fma2(two, r2, r1), qw);
+    const F2 nextV = fma2(sixth, fma2(four, a2s, a13), v), nextW = fma2(sixth, fma2(four, r2, r13), w);
+    unpack(nextN, o.next.n[0], o.next.n[1]);
+    unpack(nextQ, o.next.u, o.next.n[2]);
+    unpack(nextV, o.next.v[0], o.next.v[1]);
+    unpack(nextW, o.next.w, o.next.v[2]);
+    unpack(a1, o.a1[0], o.a1[1]);
+    o.k1 = k1, o.a1[2] = a1z;
+    o.next.drag = o.next.psi = 0.f;
+    if (a != 0.f) {
+        const F2 x = pack(midU, o.next.u);
+        float m0, m1, d0, d1;
+        unpack(mul2(mul2(both(-a), x), fma2(both(-c.xiA), x, two)), m0, m1);
+        unpack(fma2(mul2(both(a2), x), x, fma2(both(-2.f), x, both(1.f))), d0, d1);
+        const float dragMid = __fdividef(m0, fmaxf(d0, 1e-3f));
+        o.next.drag = __fdividef(m1, fmaxf(d1, 1e-3f));
+        o.next.psi = __fmul_rn(t.sixth, __fmaf_rn(4.f, dragMid, __fadd_rn(s.drag, o.next.drag)));
+    }
+}
+
+/* The wide coefficients, their high halves the FP32 ones. */
+__device__ __forceinline__ void setWide(MixedRay& r, Ff uA, Ff uB, Ff uC, Ff xiA) {
+    r.c.uA = uA.hi, r.c.uB = uB.hi, r.c.uC = uC.hi, r.c.xiA = xiA.hi;
+    r.uALo = uA.lo, r.uBLo = uB.lo, r.uCLo = uC.lo, r.xiALo = xiA.lo;
 }
 
 /* The constants of motion alone, for an eye at rest (lens.inc:125-142 without the aberration of
  * 110-122), in double-float, in rayStartWith's order of operations with the direction normalised first: E,
  * the axial momentum xi, eta and K = eta + xi^2 and the radial equation's coefficients, rounded to float
- * (a pair's hi is its value rounded to nearest) into r.c, the five the wide sub-steps take into r as
- * pairs, and the factors the first state is made of (d_x, 1 / (|d| E), across and the axial component
+ * (a pair's hi is its value rounded to nearest) into r.c, the low halves of those the wide sub-steps take
+ * into r, and the factors the first state is made of (d_x, 1 / (|d| E), across and the axial component
  * of the direction over E), which the caller forms in FP32 as the reference's integrator has them. */
 __device__ __forceinline__ void motionConstantsFf(const MotionTermsFf& t, float nx, float ny, MixedRay& r,
                                                   float& dx, float& over, float& across, float& xiAxis) {
@@ -277,9 +330,8 @@ __device__ __forceinline__ void motionConstantsFf(const MotionTermsFf& t, float 
     const Ff uB = ffMulF(ffAdd(eta, ffMul(xiOff, xiOff)), 3.f);
     const Ff uC = ffMul(t.minusTwoA2, eta);
     const Ff xiA = ffMul(xi, t.a);
-    r.c.invEnergy = invEnergy.hi, r.c.xi = xi.hi, r.c.moved = 1.f;
-    r.c.big = big.hi, r.c.uA = uA.hi, r.c.uB = uB.hi, r.c.uC = uC.hi, r.c.xiA = xiA.hi;
-    r.big = big, r.uA = uA, r.uB = uB, r.uC = uC, r.xiA = xiA;
+    r.c.invEnergy = invEnergy.hi, r.c.xi = xi.hi, r.c.moved = 1.f, r.c.big = big.hi;
+    setWide(r, uA, uB, uC, xiA);
     dx = d[0].hi, over = overFf.hi, across = acrossFf.hi, xiAxis = xiAxisFf.hi;
 }
 
@@ -295,26 +347,25 @@ __device__ __forceinline__ void mixedStart(const MixedParams& p, uint32_t guards
         RayState<double> sd;
         rayStartWith(v.d, v.start64, widen(nx), widen(ny), widen(time), cd, sd);
         r.c.invEnergy = narrow(cd.invEnergy), r.c.xi = narrow(cd.xi), r.c.moved = narrow(cd.moved);
-        r.c.big = narrow(cd.big), r.c.step = narrow(cd.step), r.c.uA = narrow(cd.uA), r.c.uB = narrow(cd.uB);
-        r.c.uC = narrow(cd.uC), r.c.xiA = narrow(cd.xiA);
-        r.big = ffSplit(cd.big), r.step = cd.step, r.uA = ffSplit(cd.uA), r.uB = ffSplit(cd.uB);
-        r.uC = ffSplit(cd.uC), r.xiA = ffSplit(cd.xiA);
+        r.c.big = narrow(cd.big);
+        const Ff step = ffSplit(cd.step);
+        r.c.step = step.hi, r.stepLo = step.lo;
+        setWide(r, ffSplit(cd.uA), ffSplit(cd.uB), ffSplit(cd.uC), ffSplit(cd.xiA));
         r.s.u = v.startNarrow[3], r.s.w = narrow(sd.w);
         for (int k = 0; k < 3; ++k) r.s.n[k] = v.startNarrow[k], r.s.v[k] = narrow(sd.v[k]);
     } else if (guards & ARTF_CUDA_GUARD_MOTION) {
         float dx, over, across, xiAxis;
         motionConstantsFf(v.motion, nx, ny, r, dx, over, across, xiAxis);
         r.c.step = divSqrtR(v.stepBaseNarrow, maxX(r.c.big, 4.f));
-        r.step = widen(r.c.step);
+        r.stepLo = 0.f;
         /* (u and n start at the eye's: the view's, narrowed once) */
         r.s.u = v.startNarrow[3];
         r.s.w = v.wScaleNarrow * dx * over;
         for (int k = 0; k < 3; ++k)
-            r.s.n[k] = v.startNarrow[k], r.s.v[k] = across * v.f.etheta[k] + xiAxis * v.f.ephi[k];
+            r.s.n[k] = v.startNarrow[k], r.s.v[k] = sum2(across, v.f.etheta[k], xiAxis, v.f.ephi[k]);
     } else {
         rayStart(v.f, nx, ny, time, p.stepScale, r.c, r.s);
-        r.big = Ff{r.c.big, 0.f}, r.step = r.c.step, r.uA = Ff{r.c.uA, 0.f}, r.uB = Ff{r.c.uB, 0.f};
-        r.uC = Ff{r.c.uC, 0.f}, r.xiA = Ff{r.c.xiA, 0.f};
+        r.stepLo = r.uALo = r.uBLo = r.uCLo = r.xiALo = 0.f;
     }
     r.c.time = time;
     r.s.psi = 0.f;
@@ -322,71 +373,73 @@ __device__ __forceinline__ void mixedStart(const MixedParams& p, uint32_t guards
     r.psiHi = r.psiLo = 0.f;
     r.through = 1.f;
     r.sum[0] = r.sum[1] = r.sum[2] = 0.f;
-    r.hitR = r.hitPhi = NAN;
     r.i = 0;
-    r.crossings = r.wide = 0;
-    r.lit = false;
+    r.crossings = r.wide = r.turns = 0;
 }
 
-/* Which sub-steps of this FP32 step must run again wide. */
-__device__ __forceinline__ void mixedNeeds(uint32_t guards, const MixedView& v, const MixedRay& r,
-                                           const StepOut<float>& o, bool& radial, bool& polar, unsigned& reason) {
+/* The sub-steps of an FP32 step that its guards ask for again, wide.  Radial, in the horizon's band: the
+ * whole sub-step in FP64 (the frame-drag rate's Delta / r^2 cancels there, and it divides).  At a turning
+ * point, of u or of n_z, that coordinate's motion in double-float: psi and its rate, and the components
+ * about the axis, smooth there, stay the FP32 step's.  A step that turns both runs the motion twice. */
+__device__ __forceinline__ void mixedGuards(uint32_t guards, const MixedView& v, MixedRay& r, StepOut<float>& o,
+                                            unsigned& rounds) {
     const bool band = (guards & ARTF_CUDA_GUARD_HORIZON) && r.s.u > v.uGuard;
-    const bool turnR = (guards & ARTF_CUDA_GUARD_RADIAL) && ((r.s.w > 0.f) != (o.next.w > 0.f));
-    polar = (guards & ARTF_CUDA_GUARD_POLAR) && ((r.s.v[2] > 0.f) != (o.next.v[2] > 0.f));
-    radial = band || turnR;
-    reason = (band ? 1u : 0u) | (turnR && !band ? 2u : 0u) | (polar ? 4u : 0u);
-}
-
-/* The wide sub-steps, with the ray's step terms (stepTermsFf, formed once a ray).  Radial: in the
- * horizon's band the whole sub-step in FP64 (the frame-drag rate's Delta / r^2 cancels there, and it
- * divides), from the pairs widened; at a turning point of u the motion (u, du/ds) alone in double-float,
- * psi and its rate staying the FP32 step's. */
-__device__ __forceinline__ void radialWide(const MixedView& v, const MixedRay& r, const StepTermsFf& t, bool band,
-                                           StepOut<float>& o) {
+    bool turnR = (guards & ARTF_CUDA_GUARD_RADIAL) && ((r.s.w > 0.f) != (o.next.w > 0.f)) && !band;
+    bool turnP = (guards & ARTF_CUDA_GUARD_POLAR) && ((r.s.v[2] > 0.f) != (o.next.v[2] > 0.f));
+    if (!(band || turnR || turnP)) return;
+    r.wide += 1u | (band ? 0x10000u : 0u);
+    r.turns += (turnR ? 1u : 0u) | (turnP ? 0x10000u : 0u);
+    const unsigned first = (threadIdx.x & 31) == __ffs((int)__activemask()) - 1;
+    rounds += first;
     if (band) {
-        const RayConst<double> c = wideConst(r);
+        RayConst<double> c;
+        c.step = ffWide(Ff{r.c.step, r.stepLo}), c.uA = ffWide(Ff{r.c.uA, r.uALo}), c.uB = ffWide(Ff{r.c.uB, r.uBLo});
+        c.uC = ffWide(Ff{r.c.uC, r.uCLo}), c.xiA = ffWide(Ff{r.c.xiA, r.xiALo});
+        c.invEnergy = c.xi = c.moved = c.time = c.big = 0.0; /* (not read by the sub-step) */
         double k1;
         RayState<double> s, next;
         s.u = widen(r.s.u), s.w = widen(r.s.w), s.psi = 0.0, s.drag = widen(r.s.drag);
-        radialStepWith(v.d.a, v.wideA2, c, wideTerms(t), s, next, k1);
+        const double step = widen(r.c.step);
+        radialStepWith(v.d.a, v.wideA2, c, stepTerms(step), s, next, k1);
         o.next.u = narrow(next.u), o.next.w = narrow(next.w), o.next.psi = narrow(next.psi);
         o.next.drag = narrow(next.drag);
         o.k1 = narrow(k1);
-    } else {
-        Ff u, w, k1;
-        radialMotionFf(r, t, r.s.u, r.s.w, u, w, k1);
-        o.next.u = u.hi, o.next.w = w.hi, o.k1 = k1.hi;
     }
-}
-
-/* Polar: at the turning point of n_z, the axis component (n_z, dn_z/ds); the components about the axis
- * stay the FP32 step's. */
-__device__ __forceinline__ void polarWide(const MixedView& v, const MixedRay& r, const StepTermsFf& t,
-                                          StepOut<float>& o) {
-    Ff nz, vz, a1z;
-    polarAxisFf(v.motion.a2, r, t, r.s.n[2], r.s.v[2], nz, vz, a1z);
-    o.next.n[2] = nz.hi, o.next.v[2] = vz.hi, o.a1[2] = a1z.hi;
+    while (turnR || turnP) {
+        Cubic f{Ff{r.c.uA, r.uALo}, Ff{0.f, 0.f}, ffScale(v.motion.a2, -2.f)};
+        if (turnR) f.B = Ff{r.c.uB, r.uBLo}, f.C = Ff{r.c.uC, r.uCLo};
+        Ff x, rate, k1;
+        motionFf(f, r.c.step, turnR ? r.s.u : r.s.n[2], turnR ? r.s.w : r.s.v[2], x, rate, k1);
+        if (turnR) {
+            o.next.u = x.hi, o.next.w = rate.hi, o.k1 = k1.hi;
+            turnR = false;
+        } else {
+            o.next.n[2] = x.hi, o.next.v[2] = rate.hi, o.a1[2] = k1.hi;
+            turnP = false;
+        }
+    }
 }
 
 /* After a step: the disc crossing, escape, horizon, opacity and the step cap.  Returns the end's kind
  * (ARTF_CUDA_END_*) + 1, or 0 when the ray goes on. */
 __device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t guards, const MixedView& v,
-                                                 MixedRay& r, const StepOut<float>& o) {
+                                                 MixedRay& r, const StepOut<float>& o, ArtfCudaRayEnd* end) {
     const Frame<float>& f = v.f;
     const bool compensated = guards & ARTF_CUDA_GUARD_PSI;
     const float increment = o.next.psi;
     Crossing<float> x;
+    bool opaque = false;
     if (crossingOf(f, v.rhoScale, r.c, r.s, o, x)) {
         x.psiC = compensated ? r.psiHi + (r.psiLo + x.part * increment) : r.psiHi + x.part * increment;
         ++r.crossings;
         float turn;
         const float light = shadeCrossing(f, v.rhoScale, v.map, v.fluid, r.c, x, r.through, r.sum, &turn);
-        if (light > 0.f && !r.lit) {
-            r.lit = true;
-            r.hitR = 1.f / x.uc;
-            r.hitPhi = turn - floorf(turn);
+        if (light > 0.f && !(r.crossings & kLit)) {
+            r.crossings |= kLit;
+            if (end) end->hitR = 1.f / x.uc, end->hitPhi = turn - floorf(turn);
         }
+        /* (the transmission only changes here) */
+        opaque = !(r.through > .004f);
     }
     ++r.i;
     if (0.f > o.next.u) {
@@ -402,7 +455,7 @@ __device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t 
         return ARTF_CUDA_END_SKY + 1;
     }
     if (o.next.u > f.uHorizon) return ARTF_CUDA_END_HORIZON + 1;
-    if (!(r.through > .004f)) return ARTF_CUDA_END_OPAQUE + 1;
+    if (opaque) return ARTF_CUDA_END_OPAQUE + 1;
     if (compensated) {
         const float sumHi = r.psiHi + increment, back = sumHi - r.psiHi;
         r.psiLo += (r.psiHi - (sumHi - back)) + (increment - back);
@@ -415,82 +468,68 @@ __device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t 
     return r.i >= p.maxSteps ? ARTF_CUDA_END_CAP + 1 : 0u;
 }
 
+/* What a thread counts over its rays, in shared memory: touched once a ray, it would hold ten registers
+ * through the stepping loop. */
+enum { kTallyRays, kTallySteps, kTallyCrossings, kTallyEscapes, kTallyWide, kTallyBand, kTallyRadial, kTallyPolar, kTallyCount };
+
 /* The end record of a finished ray, and its tallies. */
-__device__ __forceinline__ unsigned mixedFinish(const MixedRay& r, unsigned ended, ArtfCudaRayEnd* end, Tally& t) {
+__device__ __forceinline__ unsigned mixedFinish(const MixedRay& r, unsigned ended, ArtfCudaRayEnd* end,
+                                                unsigned (*tally)[256]) {
     unsigned kind = ended - 1;
-    if (r.lit) kind |= ARTF_CUDA_END_LIT;
-    t.rays += 1;
-    t.steps += (unsigned)r.i;
-    t.crossings += r.crossings;
+    if (r.crossings & kLit) kind |= ARTF_CUDA_END_LIT;
+    const unsigned crossings = r.crossings & ~kLit;
     const bool sky = (kind & 15u) == ARTF_CUDA_END_SKY;
-    t.escapes += sky;
+    const unsigned add[kTallyCount] = {1u, (unsigned)r.i, crossings, sky ? 1u : 0u, r.wide & 0xFFFFu, r.wide >> 16,
+                                       r.turns & 0xFFFFu, r.turns >> 16};
+    for (int k = 0; k < kTallyCount; ++k) tally[k][threadIdx.x] += add[k];
     if (end) {
-        ArtfCudaRayEnd e;
-        e.hitR = r.hitR;
-        e.hitPhi = r.hitPhi;
-        for (int k = 0; k < 3; ++k) e.dir[k] = sky ? r.s.n[k] : 0.f;
-        e.mino = (float)(sky ? ((double)(r.i - 1) + (double)r.s.w) * r.step : (double)r.i * r.step);
-        e.steps = (uint16_t)r.i;
-        e.crossings = (uint8_t)(r.crossings > 255u ? 255u : r.crossings);
-        e.kind = (uint8_t)kind;
-        e.fp64Steps = (uint16_t)r.wide;
-        e.reserved = 0;
-        *end = e;
+        const double step = ffWide(Ff{r.c.step, r.stepLo});
+        for (int k = 0; k < 3; ++k) end->dir[k] = sky ? r.s.n[k] : 0.f;
+        end->mino = (float)(sky ? ((double)(r.i - 1) + (double)r.s.w) * step : (double)r.i * step);
+        end->steps = (uint16_t)r.i;
+        end->crossings = (uint8_t)(crossings > 255u ? 255u : crossings);
+        end->kind = (uint8_t)kind;
+        end->fp64Steps = (uint16_t)(r.wide & 0xFFFFu);
+        end->reserved = 0;
     }
     return kind;
 }
 
-struct Reasons {
-    unsigned wide = 0, horizon = 0, radial = 0, polar = 0, rounds = 0;
-};
-
-__device__ __forceinline__ void countReason(unsigned reason, Reasons& n) {
-    n.wide += 1;
-    n.horizon += reason & 1u;
-    n.radial += (reason >> 1) & 1u;
-    n.polar += (reason >> 2) & 1u;
-}
-
-/* The per-ray path: one ray from start to end, each step's wide sub-steps at once. */
+/* One ray from start to end, each step's wide sub-steps at once.  kAll: every guard on (the default), the
+ * step's tests of them as constants. */
+template <bool kAll>
 __device__ __forceinline__ unsigned traceRayMixed(const MixedParams& p, const MixedView& v, float nx, float ny,
-                                                  float time, float* sum, ArtfCudaRayEnd* end, Tally& t, Reasons& n) {
+                                                  float time, float* sum, ArtfCudaRayEnd* end, unsigned (*tally)[256],
+                                                  unsigned& rounds) {
+    const uint32_t guards = kAll ? (uint32_t)ARTF_CUDA_GUARD_ALL : p.guards;
     MixedRay r;
-    mixedStart(p, p.guards, v, nx, ny, time, r);
+    mixedStart(p, guards, v, nx, ny, time, r);
+    if (end) end->hitR = end->hitPhi = NAN;
     unsigned ended = 0;
     while (!ended) {
         StepOut<float> o;
-        nystromStep(v.f.a, r.c, r.s, o);
-        bool radial, polar;
-        unsigned reason;
-        mixedNeeds(p.guards, v, r, o, radial, polar, reason);
-        if (radial || polar) {
-            const StepTermsFf terms = stepTermsFf(r.c.step);
-            if (radial) radialWide(v, r, terms, (reason & 1u) != 0u, o);
-            if (polar) polarWide(v, r, terms, o);
-        }
-        if (radial || polar) {
-            ++r.wide;
-            countReason(reason, n);
-        }
-        ended = mixedAdvance(p, p.guards, v, r, o);
+        mixedStep(v.f.a, r.c, r.s, o);
+        mixedGuards(guards, v, r, o, rounds);
+        ended = mixedAdvance(p, guards, v, r, o, end);
     }
     for (int k = 0; k < 3; ++k) sum[k] = sum[k] + r.sum[k];
-    return mixedFinish(r, ended, end, t);
+    return mixedFinish(r, ended, end, tally);
 }
 
-__device__ __forceinline__ void flushReasons(const Reasons& n, unsigned long long* counters) {
-    const unsigned wide = __reduce_add_sync(0xFFFFFFFFu, n.wide);
-    const unsigned horizon = __reduce_add_sync(0xFFFFFFFFu, n.horizon);
-    const unsigned radial = __reduce_add_sync(0xFFFFFFFFu, n.radial);
-    const unsigned polar = __reduce_add_sync(0xFFFFFFFFu, n.polar);
-    const unsigned rounds = __reduce_add_sync(0xFFFFFFFFu, n.rounds);
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(counters + CFp64Steps, (unsigned long long)wide);
-        atomicAdd(counters + CFp64Horizon, (unsigned long long)horizon);
-        atomicAdd(counters + CFp64Radial, (unsigned long long)radial);
-        atomicAdd(counters + CFp64Polar, (unsigned long long)polar);
-        atomicAdd(counters + CFp64Rounds, (unsigned long long)rounds);
+__device__ __forceinline__ void clearTallies(unsigned (*tally)[256]) {
+    for (int k = 0; k < kTallyCount; ++k) tally[k][threadIdx.x] = 0;
+}
+
+/* A warp's tallies to the launch's counters; the whole warp calls it. */
+__device__ __forceinline__ void flushTallies(unsigned (*tally)[256], unsigned rounds, unsigned long long* counters) {
+    const int to[kTallyCount] = {CRays, CSteps, CCrossings, CEscapes, CFp64Steps, CFp64Horizon, CFp64Radial, CFp64Polar};
+    const bool first = (threadIdx.x & 31) == 0;
+    for (int k = 0; k < kTallyCount; ++k) {
+        const unsigned n = __reduce_add_sync(0xFFFFFFFFu, tally[k][threadIdx.x]);
+        if (first && n) atomicAdd(counters + to[k], (unsigned long long)n);
     }
+    rounds = __reduce_add_sync(0xFFFFFFFFu, rounds);
+    if (first && rounds) atomicAdd(counters + CFp64Rounds, (unsigned long long)rounds);
 }
 
 /* The view a queue unit belongs to: the last whose first unit is at or below it. */
@@ -529,14 +568,15 @@ __device__ __forceinline__ int tileView(const MixedParams& p, int tile) {
 
 /* Each tile's weight class, and each class's count of queue slots (a tile has one a ray plane), counted
  * in the block first so that each class takes one global atomic a block. */
-__global__ void __launch_bounds__(128) probeTiles(const MixedParams p, int totalTiles, int* weights,
-                                                  unsigned* classes) {
+template <bool kOne>
+__device__ __forceinline__ void probeTiles(const MixedParams& p, const MixedView* one, int totalTiles, int* weights,
+                                           unsigned* classes) {
     __shared__ unsigned counts[kWeightClasses];
     if (threadIdx.x < kWeightClasses) counts[threadIdx.x] = 0;
     __syncthreads();
     const int g = (int)(blockIdx.x * 128 + threadIdx.x);
     if (g < totalTiles) {
-        const MixedView& v = p.views[tileView(p, g)];
+        const MixedView& v = kOne ? *one : p.views[tileView(p, g)];
         const int tile = g - v.tileBase;
         const int x = min((tile % v.tilesX) * 8 + 4, (int)v.f.width - 1);
         const int y = min(v.rowBegin + (tile / v.tilesX) * 4 + 2, v.rowBegin + v.rows - 1);
@@ -567,8 +607,10 @@ __global__ void __launch_bounds__(128) probeTiles(const MixedParams p, int total
 /* Each tile's slots into the order, its planes together, heavier classes first (within a class in the
  * order the atomics give): a block reserves each class's run with one global atomic, its tiles take
  * places within the run by shared ones. */
-__global__ void __launch_bounds__(128) placeTiles(const MixedParams p, int totalTiles, const int* weights,
-                                                  const unsigned* classes, unsigned* cursors, uint2* order) {
+template <bool kOne>
+__device__ __forceinline__ void placeTiles(const MixedParams& p, const MixedView* one, int totalTiles,
+                                           const int* weights, const unsigned* classes, unsigned* cursors,
+                                           uint2* order) {
     __shared__ unsigned counts[kWeightClasses], runs[kWeightClasses];
     if (threadIdx.x < kWeightClasses) counts[threadIdx.x] = 0;
     __syncthreads();
@@ -577,9 +619,10 @@ __global__ void __launch_bounds__(128) placeTiles(const MixedParams p, int total
     int vi = 0, w = 0;
     unsigned planes = 0, within = 0;
     if (active) {
-        vi = tileView(p, g);
+        vi = kOne ? 0 : tileView(p, g);
         w = weights[g];
-        planes = p.views[vi].rayOut ? (unsigned)p.views[vi].rays : 1u;
+        const MixedView& v = kOne ? *one : p.views[vi];
+        planes = v.rayOut ? (unsigned)v.rays : 1u;
         within = atomicAdd(counts + w, planes);
     }
     __syncthreads();
@@ -591,202 +634,112 @@ __global__ void __launch_bounds__(128) placeTiles(const MixedParams p, int total
     __syncthreads();
     if (!active) return;
     const unsigned at = runs[w] + within;
-    const unsigned tile = (unsigned)(g - p.views[vi].tileBase);
+    const unsigned tile = (unsigned)(g - (kOne ? one->tileBase : p.views[vi].tileBase));
     for (unsigned k = 0; k < planes; ++k) order[at + k] = make_uint2((unsigned)vi | k << 12, tile);
 }
 
-/* FP32 steps a lane takes between two of the warp's votes on refills and FP64 rounds (measured at
- * 1080p x 4: 3 steps 2.64 ms, 4 steps 2.62, 6 steps 2.60, 8 steps 2.60, 10 steps 2.62; the 64-view batch
- * alike). */
-constexpr int kInnerSteps = 6;
-
-/* This lane's step terms, from the block's table. */
-__device__ __forceinline__ StepTermsFf laneTerms(const Ff (*terms)[256]) {
-    StepTermsFf t;
-    t.half = terms[0][threadIdx.x], t.eighth = terms[1][threadIdx.x], t.halfSquare = terms[2][threadIdx.x];
-    t.sixthSquare = terms[3][threadIdx.x], t.sixth = terms[4][threadIdx.x];
-    return t;
+__global__ void __launch_bounds__(128) probeTable(const MixedParams p, int totalTiles, int* weights, unsigned* classes) {
+    probeTiles<false>(p, nullptr, totalTiles, weights, classes);
+}
+__global__ void __launch_bounds__(128) probeOne(const MixedParams p, const __grid_constant__ MixedView view,
+                                                int totalTiles, int* weights, unsigned* classes) {
+    probeTiles<true>(p, &view, totalTiles, weights, classes);
+}
+__global__ void __launch_bounds__(128) placeTable(const MixedParams p, int totalTiles, const int* weights,
+                                                  const unsigned* classes, unsigned* cursors, uint2* order) {
+    placeTiles<false>(p, nullptr, totalTiles, weights, classes, cursors, order);
+}
+__global__ void __launch_bounds__(128) placeOne(const MixedParams p, const __grid_constant__ MixedView view,
+                                                int totalTiles, const int* weights, const unsigned* classes,
+                                                unsigned* cursors, uint2* order) {
+    placeTiles<true>(p, &view, totalTiles, weights, classes, cursors, order);
 }
 
-/* The warp-scheduled trace (see the file's head).  kOne: a single view, read from `one` (a kernel
- * parameter) rather than from the view table.  kAll: every guard on (the default), the step's tests of
- * them as constants. */
+/* The persistent trace: each warp takes slots from the queue, one ray plane of one 8 x 4 tile of pixels a
+ * slot, and traces a slot's 32 rays together.  kOne: a single view, read from `one` (a kernel parameter)
+ * rather than from the view table. */
 template <bool kOne, bool kAll>
-__device__ __forceinline__ void mixedQueue(const MixedParams& p, const MixedView* one) {
-    const uint32_t guards = kAll ? (uint32_t)ARTF_CUDA_GUARD_ALL : p.guards;
-    /* each lane's ray's step terms as pairs, formed at its set-up: a wide round then loads them where
-     * it would multiply them out again */
-    __shared__ Ff terms[5][256];
-    const unsigned full = 0xFFFFFFFFu;
+__device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView* one) {
+    __shared__ unsigned tally[kTallyCount][256];
     const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    Tally t;
-    Reasons n;
-    int unit = -1, x = 0, y = 0, k = 0, kEnd = 1; /* this lane's unit: rays k .. kEnd - 1 of pixel (x, y) */
-    const MixedView* v = kOne ? one : p.views;
-    bool exhausted = false, live = false, haveStep = false, waitR = false, waitP = false;
-    unsigned reason = 0, bits = 0;
-    float pixel[3] = {0.f, 0.f, 0.f};
-    MixedRay r;
-    StepOut<float> o;
-    int sinceStart = 0, sinceRadial = 0, sincePolar = 0;
-    /* Every iteration either advances some lane's ray by a step, starts rays, or ends the loop: the queue
-     * is finite and a ray ends within maxSteps steps, so the loop ends. */
+    unsigned rounds = 0;
+    clearTallies(tally);
+    const unsigned parts = (unsigned)(p.totalUnits >> p.lanesLog2); /* 2^lanesLog2 rays each */
     for (;;) {
-        /* (1) refill, batched: the set-up of a ray is wide work */
-        const unsigned idle = __ballot_sync(full, !live && !exhausted);
-        const unsigned liveMask = __ballot_sync(full, live);
-        if (idle && (__popc(idle) >= p.refill || liveMask == 0 || sinceStart >= p.maxWait)) {
-            sinceStart = 0;
-            const bool needPixel = !live && !exhausted && (unit < 0 || k >= kEnd);
-            const unsigned fetch = __ballot_sync(full, needPixel);
-            if (fetch) {
-                const int leader = __ffs(fetch) - 1;
-                int base = 0;
-                if (lane == leader) base = (int)atomicAdd(p.counters + CQueue, (unsigned long long)__popc(fetch));
-                base = __shfl_sync(full, base, leader);
-                if (needPixel) {
-                    unit = base + __popc(fetch & below);
-                    k = 0, bits = 0;
-                    pixel[0] = pixel[1] = pixel[2] = 0.f;
-                    if (unit >= p.totalUnits) {
-                        exhausted = true;
-                        unit = -1;
-                    } else {
-                        /* a slot of 32 units is one ray plane of one tile: a warp's lanes take
-                         * neighbouring pixels */
-                        int plane, tile;
-                        const int within = unit & 31; /* (every view's first unit is a multiple of 32) */
-                        if (p.order) {
-                            const uint2 slot = __ldg(p.order + (unit >> 5));
-                            if (!kOne) v = p.views + (slot.x & 4095u);
-                            plane = v->rayOut ? (int)(slot.x >> 12) : 0;
-                            tile = (int)slot.y;
-                        } else {
-                            if (!kOne) v = p.views + viewOf(p, unit);
-                            int local = unit - v->unitBase;
-                            plane = v->rayOut ? local / v->pixelUnits : 0;
-                            local -= plane * v->pixelUnits;
-                            tile = local >> 5;
-                        }
-                        x = (tile % v->tilesX) * 8 + (within & 7);
-                        y = v->rowBegin + (tile / v->tilesX) * 4 + (within >> 3);
-                        k = plane;
-                        kEnd = v->rayOut ? plane + 1 : v->rays;
-                        if (x >= v->f.width || y >= v->rowBegin + v->rows) k = kEnd; /* (off the band: fetch again) */
-                    }
-                }
-            }
-            if (!live && unit >= 0 && k < kEnd) {
+        unsigned part = 0;
+        if (lane == 0) part = (unsigned)atomicAdd(p.counters + CQueue, 1ull);
+        part = __shfl_sync(0xFFFFFFFFu, part, 0);
+        if (part >= parts) break;
+        /* (a tile's rays row by row: 8 x 4 pixels a part, 8 x 2, 8 x 1, 4 x 1 or 2 x 1) */
+        const unsigned first = part << p.lanesLog2, within = (first & 31u) + (unsigned)lane;
+        const int slot = (int)(first >> 5);
+        const MixedView* v = kOne ? one : p.views;
+        int plane, tile;
+        if (p.order) {
+            const uint2 s = __ldg(p.order + slot);
+            if (!kOne) v = p.views + (s.x & 4095u);
+            plane = v->rayOut ? (int)(s.x >> 12) : 0;
+            tile = (int)s.y;
+        } else {
+            const int unit = slot << 5;
+            if (!kOne) v = p.views + viewOf(p, unit);
+            int local = unit - v->unitBase;
+            plane = v->rayOut ? local / v->pixelUnits : 0;
+            local -= plane * v->pixelUnits;
+            tile = local >> 5;
+        }
+        const int x = (tile % v->tilesX) * 8 + (int)(within & 7u);
+        const int y = v->rowBegin + (tile / v->tilesX) * 4 + (int)(within >> 3);
+        if (lane >> p.lanesLog2 == 0 && x < v->f.width && y < v->rowBegin + v->rows) {
+            const size_t index = (size_t)y * (size_t)v->f.width + (size_t)x;
+            const int64_t pixels = (int64_t)v->f.width * v->f.height;
+            float sum[3] = {0.f, 0.f, 0.f};
+            unsigned bits = 0;
+            const int last = v->rayOut ? plane + 1 : v->rays;
+            for (int k = plane; k < last; ++k) {
                 float nx, ny, moment;
                 samplePosition(v->h, v->jitter, v->seed, x, y, k, &nx, &ny, &moment);
-                /* (the set-up keeps its guard test at run time: made constant there too, the batch ran
-                 * 7.61 ms against 7.13, a matter of code layout) */
-                mixedStart(p, p.guards, *v, nx, ny, v->h.disc[2] + v->h.spin[3] * moment, r);
-                const StepTermsFf t = stepTermsFf(r.c.step);
-                terms[0][threadIdx.x] = t.half, terms[1][threadIdx.x] = t.eighth;
-                terms[2][threadIdx.x] = t.halfSquare, terms[3][threadIdx.x] = t.sixthSquare;
-                terms[4][threadIdx.x] = t.sixth;
-                live = true;
+                ArtfCudaRayEnd* end = v->ends && inBounds(v->f.fault, kBoundsRayEnd,
+                                                          (int64_t)(index * (size_t)v->rays + (size_t)k),
+                                                          pixels * v->rays)
+                                          ? v->ends + index * (size_t)v->rays + (size_t)k
+                                          : nullptr;
+                bits |= classBits(traceRayMixed<kAll>(p, *v, nx, ny, v->h.disc[2] + v->h.spin[3] * moment, sum, end, tally,
+                                                    rounds));
             }
-        } else if (idle) {
-            ++sinceStart;
-        }
-        if (__all_sync(full, exhausted && !live)) break;
-
-        /* (2) wide rounds, when enough lanes wait or no other lane can move */
-        const unsigned ready = __ballot_sync(full, live && !waitR && !waitP);
-        const unsigned needR = __ballot_sync(full, waitR), needP = __ballot_sync(full, waitP);
-        if (needR && (__popc(needR) >= p.batch || ready == 0 || sinceRadial >= p.maxWait)) {
-            if (waitR) {
-                radialWide(*v, r, laneTerms(terms), (reason & 1u) != 0u, o);
-                waitR = false;
-            }
-            sinceRadial = 0;
-            n.rounds += lane == 0;
-        } else if (needR) {
-            ++sinceRadial;
-        }
-        if (needP && (__popc(needP) >= p.batch || ready == 0 || sincePolar >= p.maxWait)) {
-            if (waitP) {
-                polarWide(*v, r, laneTerms(terms), o);
-                waitP = false;
-            }
-            sincePolar = 0;
-            n.rounds += lane == 0;
-        } else if (needP) {
-            ++sincePolar;
-        }
-        /* (3) up to kInnerSteps FP32 steps a lane between the warp's votes: a lane commits its complete
-         * step (one a round just finished, or a plain one) and takes the next, until a step needs an FP64
-         * sub-step or the ray ends */
-        for (int j = 0; j < kInnerSteps; ++j) {
-            if (haveStep && !waitR && !waitP) {
-                haveStep = false;
-                const unsigned ended = mixedAdvance(p, guards, *v, r, o);
-                if (ended) {
-                    const size_t index = (size_t)y * (size_t)v->f.width + (size_t)x;
-                    const int64_t pixels = (int64_t)v->f.width * v->f.height;
-                    ArtfCudaRayEnd* end = v->ends && inBounds(v->f.fault, kBoundsRayEnd,
-                                                              (int64_t)(index * (size_t)v->rays + (size_t)k),
-                                                              pixels * v->rays)
-                                              ? v->ends + index * (size_t)v->rays + (size_t)k
-                                              : nullptr;
-                    const unsigned rayBits = classBits(mixedFinish(r, ended, end, t));
-                    live = false;
-                    if (v->rayOut) {
-                        /* (a plane holds the band's pixels) */
-                        const size_t plane = (size_t)v->f.width * (size_t)v->rows;
-                        const size_t inBand = (size_t)(y - v->rowBegin) * (size_t)v->f.width + (size_t)x;
-                        if (inBounds(v->f.fault, kBoundsRayPlane, (int64_t)((size_t)k * plane + inBand),
-                                     (int64_t)plane * v->rays))
-                            v->rayOut[(size_t)k * plane + inBand] =
-                                make_float4(r.sum[0], r.sum[1], r.sum[2], (float)rayBits);
-                        ++k;
-                    } else {
-                        bits |= rayBits;
-                        for (int c = 0; c < 3; ++c) pixel[c] = pixel[c] + r.sum[c];
-                        if (++k == kEnd && inBounds(v->f.fault, kBoundsPixel, (int64_t)index, pixels))
-                            v->hdr[index] = make_float4(pixel[0] * v->share, pixel[1] * v->share,
-                                                        pixel[2] * v->share, (float)bits);
-                    }
-                }
-            }
-            if (live && !haveStep) {
-                nystromStep(v->f.a, r.c, r.s, o);
-                mixedNeeds(guards, *v, r, o, waitR, waitP, reason);
-                haveStep = true;
-                if (waitR || waitP) {
-                    ++r.wide;
-                    countReason(reason, n);
-                }
+            if (v->rayOut) {
+                const size_t planeSize = (size_t)v->f.width * (size_t)v->rows;
+                const size_t inBand = (size_t)(y - v->rowBegin) * (size_t)v->f.width + (size_t)x;
+                if (inBounds(v->f.fault, kBoundsRayPlane, (int64_t)((size_t)plane * planeSize + inBand),
+                             (int64_t)planeSize * v->rays))
+                    v->rayOut[(size_t)plane * planeSize + inBand] = make_float4(sum[0], sum[1], sum[2], (float)bits);
+            } else if (inBounds(v->f.fault, kBoundsPixel, (int64_t)index, pixels)) {
+                v->hdr[index] = make_float4(sum[0] * v->share, sum[1] * v->share, sum[2] * v->share, (float)bits);
             }
         }
+        __syncwarp();
     }
-    flushTally(t, p.counters);
-    flushReasons(n, p.counters);
+    flushTallies(tally, rounds, p.counters);
 }
 
 /* The views from the table (a batch).  The kernels come in pairs: the guards chosen at run time, and all
  * of them as constants, which every trace with all guards runs (frames, bands and batches alike, so that
  * their bits agree): its dead branches fold away and its code is smaller. */
-__global__ void __launch_bounds__(256) traceMixedQueue(const MixedParams p) { mixedQueue<false, false>(p, nullptr); }
-__global__ void __launch_bounds__(256) traceMixedQueueAll(const MixedParams p) { mixedQueue<false, true>(p, nullptr); }
+__global__ void __launch_bounds__(256, 2) traceMixedTable(const MixedParams p) { mixedTiles<false, false>(p, nullptr); }
+__global__ void __launch_bounds__(256, 2) traceMixedTableAll(const MixedParams p) { mixedTiles<false, true>(p, nullptr); }
 
 /* A single view (a frame) as a kernel parameter: its fields are then read from the constant bank where
  * they are used, not loaded from the view table in global memory at every step. */
-__global__ void __launch_bounds__(256) traceMixedQueueOne(const MixedParams p, const __grid_constant__ MixedView view) {
-    mixedQueue<true, false>(p, &view);
+__global__ void __launch_bounds__(256, 2) traceMixedOne(const MixedParams p, const __grid_constant__ MixedView view) {
+    mixedTiles<true, false>(p, &view);
 }
-__global__ void __launch_bounds__(256) traceMixedQueueOneAll(const MixedParams p,
-                                                             const __grid_constant__ MixedView view) {
-    mixedQueue<true, true>(p, &view);
+__global__ void __launch_bounds__(256, 2) traceMixedOneAll(const MixedParams p, const __grid_constant__ MixedView view) {
+    mixedTiles<true, true>(p, &view);
 }
 
 /* Each pixel of the views with ray planes: its rays' radiance summed in ray order and scaled by
  * 1 / rays, and their class bits; the same operations, in the same order, as the per-pixel path. */
-__global__ void __launch_bounds__(256) mixedCombine(const MixedView* views) {
-    const MixedView& v = views[blockIdx.y];
+__device__ __forceinline__ void combinePlanes(const MixedView& v) {
     if (!v.rayOut) return;
     const size_t pixels = (size_t)v.f.width * (size_t)v.rows; /* the band's */
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
@@ -803,20 +756,24 @@ __global__ void __launch_bounds__(256) mixedCombine(const MixedView* views) {
         v.hdr[at] = make_float4(sum[0] * v.share, sum[1] * v.share, sum[2] * v.share, (float)bits);
 }
 
-/* The per-ray entry point: rays at given image positions in the table's first view. */
-__global__ void __launch_bounds__(128) traceMixedList(const MixedParams p, const int count, const float* nx,
-                                                      const float* ny, const float* time, float* rgb) {
+__global__ void __launch_bounds__(256) combineTable(const MixedView* views) { combinePlanes(views[blockIdx.y]); }
+__global__ void __launch_bounds__(256) combineOne(const __grid_constant__ MixedView view) { combinePlanes(view); }
+
+/* The per-ray entry point: rays at given image positions in a view. */
+__global__ void __launch_bounds__(128) traceMixedList(const MixedParams p,
+                                                      const __grid_constant__ MixedView view, const int count,
+                                                      const float* nx, const float* ny, const float* time, float* rgb) {
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    Tally t;
-    Reasons n;
+    __shared__ unsigned tally[kTallyCount][256];
+    unsigned rounds = 0;
+    clearTallies(tally);
     if (i < count) {
         float sum[3] = {0.f, 0.f, 0.f};
-        const MixedView& v = p.views[0];
-        traceRayMixed(p, v, nx[i], ny[i], time[i], sum, v.ends ? v.ends + i : nullptr, t, n);
+        traceRayMixed<false>(p, view, nx[i], ny[i], time[i], sum, view.ends ? view.ends + i : nullptr, tally, rounds);
         for (int k = 0; k < 3; ++k) rgb[3 * i + k] = sum[k];
     }
-    flushTally(t, p.counters);
-    flushReasons(n, p.counters);
+    __syncwarp();
+    flushTallies(tally, rounds, p.counters);
 }
 
 MixedParams paramsOf(const TraceLaunch& l, const void* deviceTable, int viewCount, int totalUnits) {
@@ -828,10 +785,6 @@ MixedParams paramsOf(const TraceLaunch& l, const void* deviceTable, int viewCoun
     p.stepScale = l.stepScale;
     p.maxSteps = l.stepScale < .75f ? 384 : 192;
     p.guards = l.guards ? l.guards : ARTF_CUDA_GUARD_ALL;
-    p.batch = l.fp64Batch > 0 ? (l.fp64Batch > 32 ? 32 : l.fp64Batch) : 32;
-    p.refill = l.refillBatch > 0 ? (l.refillBatch > 32 ? 32 : l.refillBatch) : 32;
-    /* (256 votes: the best of the autotuner's choices on both the 1080p frame and the 64-view batch) */
-    p.maxWait = l.compactEvery > 0 ? l.compactEvery : 256;
     p.order = nullptr;
     return p;
 }
@@ -955,52 +908,79 @@ size_t mixedOrderBytes(int totalTiles, int totalUnits) {
     return kOrderHead + weights + (size_t)(totalUnits / 32) * sizeof(uint2);
 }
 
-int mixedGrid(const TraceLaunch& l, int totalUnits, const void* kernel) {
+/* The persistent grid, and how many rays a warp takes at a time: all of a slot's 32 while that gives every
+ * resident warp one; for a frame too small for that, half as many, and so on, down to two, so that more
+ * warps share the rays and each has fewer that part ways (a warp runs what any of its rays needs, and
+ * rays of a small frame's neighbouring pixels part early: a 101 x 67 frame took 119 us by 32 rays, 84 by
+ * 8, 80 by 4 or 2; at 1920 x 1080 a warp's 32 rays stay together, 30.2 of 32 lanes busy).  refillBatch
+ * sets the most. */
+struct MixedGrid {
+    int blocks, lanesLog2;
+    bool resident; /* every part has a warp at once: the order they start in makes no difference */
+};
+
+static MixedGrid mixedGrid(const TraceLaunch& l, int totalUnits, const void* kernel) {
     const int block = l.blockSize > 0 ? l.blockSize : 128;
     int perSm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, block, 0);
-    int grid = (perSm > 0 ? perSm : 1) * l.smCount;
-    const int needed = (totalUnits + block - 1) / block;
-    return grid > needed ? needed : (grid < 1 ? 1 : grid);
+    const long long grid = (long long)(perSm > 0 ? perSm : 1) * l.smCount, warps = grid * (block / 32);
+    MixedGrid g;
+    g.lanesLog2 = 5;
+    while (l.refillBatch > 0 && 1 << g.lanesLog2 > l.refillBatch) --g.lanesLog2;
+    while (g.lanesLog2 > 1 && (long long)(totalUnits >> g.lanesLog2) * 2 <= warps) --g.lanesLog2;
+    const long long parts = totalUnits >> g.lanesLog2, needed = (parts * 32 + block - 1) / block;
+    g.resident = parts <= warps;
+    g.blocks = (int)(grid > needed ? needed : grid);
+    if (g.blocks < 1) g.blocks = 1;
+    return g;
 }
 
 cudaError_t launchMixedTable(const TraceLaunch& l, const void* deviceTable, int viewCount, int totalUnits,
                              size_t combinePixels, int totalTiles, void* orderScratch, const void* hostView) {
     MixedParams p = paramsOf(l, deviceTable, viewCount, totalUnits);
     const int block = l.blockSize > 0 ? l.blockSize : 128;
+    const bool single = hostView && viewCount == 1, all = p.guards == ARTF_CUDA_GUARD_ALL;
+    MixedView one;
+    if (single) memcpy(&one, hostView, sizeof one);
     if (l.rayCount > 0) {
-        traceMixedList<<<(l.rayCount + 127) / 128, 128, 0, l.stream>>>(p, l.rayCount, l.rayX, l.rayY, l.rayTime,
+        if (!single) return cudaErrorInvalidValue;
+        traceMixedList<<<(l.rayCount + 127) / 128, 128, 0, l.stream>>>(p, one, l.rayCount, l.rayX, l.rayY, l.rayTime,
                                                                        l.rayRgb);
         return cudaGetLastError();
     }
-    if (orderScratch && l.order == ARTF_CUDA_ORDER_HEAVY_FIRST && totalTiles > 0) {
+    const void* kernel = single ? (all ? (const void*)traceMixedOneAll : (const void*)traceMixedOne)
+                                : (all ? (const void*)traceMixedTableAll : (const void*)traceMixedTable);
+    const MixedGrid grid = mixedGrid(l, totalUnits, kernel);
+    p.lanesLog2 = grid.lanesLog2;
+    if (orderScratch && l.order == ARTF_CUDA_ORDER_HEAVY_FIRST && totalTiles > 0 && !grid.resident) {
         unsigned* classes = (unsigned*)orderScratch;
         unsigned* cursors = classes + 32;
         int* weights = (int*)((char*)orderScratch + kOrderHead);
         uint2* order = (uint2*)((char*)weights + (((size_t)totalTiles * sizeof(int) + 15) & ~(size_t)15));
         const cudaError_t e = cudaMemsetAsync(orderScratch, 0, kOrderHead, l.stream);
         if (e != cudaSuccess) return e;
-        const unsigned grid = (unsigned)((totalTiles + 127) / 128);
-        probeTiles<<<grid, 128, 0, l.stream>>>(p, totalTiles, weights, classes);
-        placeTiles<<<grid, 128, 0, l.stream>>>(p, totalTiles, weights, classes, cursors, order);
+        const unsigned tiles = (unsigned)((totalTiles + 127) / 128);
+        if (single) {
+            probeOne<<<tiles, 128, 0, l.stream>>>(p, one, totalTiles, weights, classes);
+            placeOne<<<tiles, 128, 0, l.stream>>>(p, one, totalTiles, weights, classes, cursors, order);
+        } else {
+            probeTable<<<tiles, 128, 0, l.stream>>>(p, totalTiles, weights, classes);
+            placeTable<<<tiles, 128, 0, l.stream>>>(p, totalTiles, weights, classes, cursors, order);
+        }
         p.order = order;
     }
-    const bool all = p.guards == ARTF_CUDA_GUARD_ALL;
-    if (hostView && viewCount == 1) {
-        MixedView one;
-        memcpy(&one, hostView, sizeof one);
-        const void* kernel = all ? (const void*)traceMixedQueueOneAll : (const void*)traceMixedQueueOne;
-        const int grid = mixedGrid(l, totalUnits, kernel);
-        if (all) traceMixedQueueOneAll<<<grid, block, 0, l.stream>>>(p, one);
-        else traceMixedQueueOne<<<grid, block, 0, l.stream>>>(p, one);
+    if (single) {
+        if (all) traceMixedOneAll<<<grid.blocks, block, 0, l.stream>>>(p, one);
+        else traceMixedOne<<<grid.blocks, block, 0, l.stream>>>(p, one);
     } else {
-        const void* kernel = all ? (const void*)traceMixedQueueAll : (const void*)traceMixedQueue;
-        const int grid = mixedGrid(l, totalUnits, kernel);
-        if (all) traceMixedQueueAll<<<grid, block, 0, l.stream>>>(p);
-        else traceMixedQueue<<<grid, block, 0, l.stream>>>(p);
+        if (all) traceMixedTableAll<<<grid.blocks, block, 0, l.stream>>>(p);
+        else traceMixedTable<<<grid.blocks, block, 0, l.stream>>>(p);
     }
-    if (combinePixels > 0)
-        mixedCombine<<<dim3((unsigned)((combinePixels + 255) / 256), (unsigned)viewCount), 256, 0, l.stream>>>(p.views);
+    if (combinePixels > 0) {
+        const unsigned blocks = (unsigned)((combinePixels + 255) / 256);
+        if (single) combineOne<<<blocks, 256, 0, l.stream>>>(one);
+        else combineTable<<<dim3(blocks, (unsigned)viewCount), 256, 0, l.stream>>>(p.views);
+    }
     return cudaGetLastError();
 }
 

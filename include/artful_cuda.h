@@ -196,11 +196,12 @@ typedef struct ArtfCudaTraceOptions {
     float horizonBand;   /* mixed: FP64 radial sub-steps where u > band * (0.995 / r+), i.e. within about
                           * r+ / band of the hole; 0 means the default 0.95 */
     int blockSize;       /* threads a block: 0 picks the tuned value */
-    int compactEvery;    /* steps between warp refills: 0 picks the tuned value */
+    int compactEvery;    /* accepted (0..4096); a warp's rays go from start to end, and it changes nothing */
     int persistent;      /* 1: one block per SM slot, rays pulled from a queue; 0: one ray a thread */
     uint32_t guards;     /* mixed: which FP64 guards run (ARTF_CUDA_GUARD_*); 0 means all */
-    int fp64Batch;       /* mixed: lanes that wait for a wide sub-step before a warp runs them; 0: 32 */
-    int refillBatch;     /* mixed: idle lanes before a warp starts new rays (wide set-ups); 0: 32 */
+    int fp64Batch;       /* accepted (0..32); wide sub-steps run in their step, and it changes nothing */
+    int refillBatch;     /* mixed: the most rays a warp starts at a time (a power of two is used); 0: 32.
+                          * Frames of few rays start fewer, so that every warp has some */
     int64_t bandRays;    /* a frame of more rays than this goes out in bands of whole rows of at most this
                           * many rays, each launched and waited for, so that no launch holds the GPU long
                           * (vulkan.c:1729-1756).  0: the reference's choice, bands of 8e6 rays for frames
@@ -252,7 +253,7 @@ enum {
 typedef struct ArtfCudaTraceStats {
     uint64_t rays, steps, crossings, escapes, fp64Steps;
     uint64_t fp64Horizon, fp64Radial, fp64Polar; /* mixed: the wide (FP64-precision) steps by reason */
-    uint64_t fp64Rounds;                         /* mixed: warp rounds of wide steps */
+    uint64_t fp64Rounds;                         /* mixed: steps in which a warp ran wide work */
     double flops;        /* algorithmic FP32-pipe operations (the counting rule is in lensFlops.h) */
     float ms;            /* device time of the trace kernel(s), CUDA events on the context's stream */
     uint32_t bands;      /* launches the frame went out in (ArtfCudaTraceOptions.bandRays) */
@@ -349,10 +350,9 @@ void artfCudaBatchGraphDestroy(ArtfCudaGraph* graph);
 int artfCudaHoleBatchNoAlloc(const ArtfCudaView* views, int count, const ArtfCudaTraceOptions* options, void* stream,
                              ArtfCudaTraceStats* stats);
 
-/* The autotuner: times the batch under candidate launch shapes (threads a block, steps a lane waits at
- * most before a refill or an FP64 round, the FP64 and refill batch sizes), by coordinate descent from
- * the defaults, and keeps the fastest in the context: later mixed traces whose options leave these at 0
- * use it.  Synchronous; a few hundred launches. */
+/* The autotuner: times the batch under candidate launch shapes (threads a block, the most rays a warp
+ * starts at a time), by coordinate descent from the defaults, and keeps the fastest in the context: later
+ * mixed traces whose options leave these at 0 use it.  Synchronous; some fifty launches. */
 typedef struct ArtfCudaTuning {
     int blockSize, compactEvery, fp64Batch, refillBatch;
     float ms;         /* the best time found */

@@ -261,3 +261,25 @@ def test_integer_conversions_match_the_hardware(lib):
     capi.check(lib.artfCudaCheckConversions(None, 1 << 28, bad))
     assert bad[0] == 0, f"float to double: {bad[0]} differ, first {bad[2]:#010x}"
     assert bad[1] == 0, f"double to float: {bad[1]} differ, first {bad[3]:#018x}"
+
+
+@pytest.mark.parametrize("width,height,samples,moving", [(1, 1, 1, False), (9, 5, 2, True), (33, 18, 1, True), (320, 180, 1, False)])
+def test_mixed_rays_a_warp_do_not_change_the_image(lib, ctx, width, height, samples, moving):
+    """However many rays a warp takes at a time (all sizes a frame of any size can get, odd settings among
+    them), whatever the order and the block: the same bits and the same ends, which are the rays' own."""
+    desc = scenes.hole_desc(0.9, samples=samples, shutter=2.0 if moving else 0.0, time=3.0,
+                            velocity=(0.2, 0.0, 0.1) if moving else (0.0, 0.0, 0.0))
+    view = scenes.Scene("warp", desc, scenes.camera(75.0, 28.0), width, height, seed=3)
+    frame, frame64, clamped = scenes.frame(view)
+    g.set_inputs(lib, ctx, scenes.synth_map(lib, clamped, 3, 3.0), scenes.unit_fluid())
+    base, ends, stats = g.trace(lib, ctx, frame, frame64, capi.MIXED, ends=True)
+    assert stats.rays == width * height * samples ** 2 == len(ends)
+    assert np.all(ends["steps"] > 0) and stats.steps == int(ends["steps"].sum())
+    for refill, block in ((1, 32), (2, 64), (5, 96), (8, 128), (16, 192), (32, 256)):
+        got, e, s = g.trace(lib, ctx, frame, frame64, capi.MIXED, ends=True, refill=refill, block=block)
+        assert np.array_equal(got.view(np.uint32), base.view(np.uint32)), (refill, block)
+        assert e.tobytes() == ends.tobytes() and s.fp64Steps == stats.fp64Steps, (refill, block)
+    if samples == 1 and not moving:
+        nx, ny = g.pixel_centres(frame)
+        rgb, _ = g.trace_rays(lib, ctx, frame, frame64, capi.MIXED, nx, ny, np.float32(frame.disc[2]))
+        assert np.array_equal(rgb.reshape(height, width, 3), base[..., :3])
