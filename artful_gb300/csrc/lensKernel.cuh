@@ -30,6 +30,7 @@ template <typename R> struct KernelParams {
     float share;
     int tilesX, tiles;          /* 8 x 4 pixel tiles: this launch's count */
     int tileBegin;              /* the first (a band of the frame starts further down) */
+    int lanesLog2;              /* a warp takes 2^lanesLog2 of a tile's pixels: a part of it */
 };
 
 /* What a thread counts, reduced over the warp before it reaches the device counters. */
@@ -148,30 +149,33 @@ template <typename R> __device__ __forceinline__ void tracePixel(const KernelPar
         p.hdr[pixel] = make_float4((float)(sum[0] * share), (float)(sum[1] * share), (float)(sum[2] * share), (float)bits);
 }
 
-/* One warp per 8 x 4 tile, one thread per pixel. */
-template <typename R> __global__ void __launch_bounds__(256) traceTiles(const KernelParams<R> p) {
+/* A warp's part of this launch's tiles: pixels row by row, a thread each, 8 x 4 of them or fewer. */
+template <typename R> __device__ __forceinline__ void tracePart(const KernelParams<R>& p, unsigned part, Tally& t) {
     const int lane = threadIdx.x & 31;
-    const int local = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), tile = p.tileBegin + local;
+    const unsigned first = part << p.lanesLog2, within = (first & 31u) + (unsigned)lane;
+    const int tile = p.tileBegin + (int)(first >> 5);
+    const int32_t x = (tile % p.tilesX) * 8 + (int32_t)(within & 7u), y = (tile / p.tilesX) * 4 + (int32_t)(within >> 3);
+    if (lane >> p.lanesLog2 == 0 && x < p.f.width && y < p.f.height) tracePixel(p, x, y, t);
+}
+
+/* One warp per part, one thread per pixel. */
+template <typename R> __global__ void __launch_bounds__(256) traceTiles(const KernelParams<R> p) {
+    const unsigned part = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     Tally t;
-    if (local < p.tiles) {
-        const int32_t x = (tile % p.tilesX) * 8 + (lane & 7), y = (tile / p.tilesX) * 4 + (lane >> 3);
-        if (x < p.f.width && y < p.f.height) tracePixel(p, x, y, t);
-    }
+    if (part < (unsigned)p.tiles << 5 >> p.lanesLog2) tracePart(p, part, t);
     flushTally(t, p.counters);
 }
 
-/* Persistent: a grid of resident warps that pull tiles from the queue counter until none is left. */
+/* Persistent: a grid of resident warps that pull parts from the queue counter until none is left. */
 template <typename R> __global__ void __launch_bounds__(256) traceQueue(const KernelParams<R> p) {
-    const int lane = threadIdx.x & 31;
+    const unsigned parts = (unsigned)p.tiles << 5 >> p.lanesLog2;
     Tally t;
     for (;;) {
-        int local = 0;
-        if (lane == 0) local = (int)atomicAdd(p.counters + CQueue, 1ull);
-        local = __shfl_sync(0xFFFFFFFFu, local, 0);
-        if (local >= p.tiles) break;
-        const int tile = p.tileBegin + local;
-        const int32_t x = (tile % p.tilesX) * 8 + (lane & 7), y = (tile / p.tilesX) * 4 + (lane >> 3);
-        if (x < p.f.width && y < p.f.height) tracePixel(p, x, y, t);
+        unsigned part = 0;
+        if ((threadIdx.x & 31) == 0) part = (unsigned)atomicAdd(p.counters + CQueue, 1ull);
+        part = __shfl_sync(0xFFFFFFFFu, part, 0);
+        if (part >= parts) break;
+        tracePart(p, part, t);
         __syncwarp();
     }
     flushTally(t, p.counters);
@@ -220,20 +224,25 @@ template <typename R> cudaError_t launchUniform(const TraceLaunch& l, const void
     const int bandRows = l.tileRows > 0 ? l.tileRows : tileRows;
     p.tileBegin = bandBegin * p.tilesX;
     p.tiles = p.tilesX * bandRows;
+    p.lanesLog2 = 5;
     const int block = l.blockSize > 0 ? l.blockSize : 128;
     if (l.rayCount > 0) {
         const RayList list = {l.rayCount, l.rayX, l.rayY, l.rayTime, l.rayRgb};
         traceList<R><<<(l.rayCount + block - 1) / block, block, 0, l.stream>>>(p, list);
-    } else if (l.persistent) {
-        int perSm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, traceQueue<R>, block, 0);
-        int grid = (perSm > 0 ? perSm : 1) * l.smCount;
-        const int needed = (p.tiles * 32 + block - 1) / block;
-        if (grid > needed) grid = needed;
-        traceQueue<R><<<grid, block, 0, l.stream>>>(p);
     } else {
-        const int grid = (p.tiles * 32 + block - 1) / block;
-        traceTiles<R><<<grid, block, 0, l.stream>>>(p);
+        const void* kernel = l.persistent ? (const void*)traceQueue<R> : (const void*)traceTiles<R>;
+        int perSm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, block, 0);
+        const long long slots = (long long)(perSm > 0 ? perSm : 1) * l.smCount, warps = slots * (block / 32);
+        /* A frame whose tiles leave half the GPU's warps without one is bound by its longest rays' latency:
+         * its warps take half a tile each, and so on down to two pixels, and have fewer rays that part ways
+         * (exact, 61 x 40: 76 -> 44 us; 200 x 112: 61 -> 54; FP32 160 x 90 x 4: 116 -> 89; parts for more
+         * warps than there are cost more: 200 x 112 66 us).  In double a warp holds the FP64 pipe as long for
+         * two lanes as for 32, so there it keeps them. */
+        while (sizeof(R) == 4 && p.lanesLog2 > 1 && ((long long)p.tiles << 5 >> p.lanesLog2) * 2 <= warps) --p.lanesLog2;
+        const long long blocks = (((long long)p.tiles << 5 >> p.lanesLog2) * 32 + block - 1) / block;
+        if (l.persistent) traceQueue<R><<<(unsigned)(blocks < slots ? blocks : slots), block, 0, l.stream>>>(p);
+        else traceTiles<R><<<(unsigned)blocks, block, 0, l.stream>>>(p);
     }
     return cudaGetLastError();
 }

@@ -32,7 +32,7 @@
  * schedule's sake.  (Lanes that waited for full rounds of wide steps and were refilled one by one, as an
  * FP64 wide step wanted, paid 80 thread instructions a step in votes and flags: 2.15 against 1.61 ms for the
  * 1080p x 4 frame, 7.63 against 5.51 for 64 views.)  What a step costs is issue slots (71 % of them used, FMA
- * pipe 50 % busy), so the FP32 step runs its coordinates in pairs with packed instructions (mixedStep: 1.86
+ * pipe 50 % busy), so the FP32 step runs its coordinates in pairs with packed instructions (nystromStep: 1.86
  * -> 1.76 ms), the wide step is one code path (1.74 -> 1.61 with the counts out of registers) and each float
  * rounding is written out or pinned (ARTF_PINNED_FMA): whatever registers a kernel is given, its images are
  * the same bits.  A frame of fewer rays than the GPU's warps could take is bound by its longest ray's
@@ -221,85 +221,6 @@ __device__ __forceinline__ void motionFf(const Cubic& f, float step, float x, fl
     nextV = ffAdd(Ff{v, 0.f}, ffMul(ffProd(step, 1.f / 6.f), ffAdd(ffAdd(k1, k3), ffScale(k2, 4.f))));
 }
 
-/* ---- the FP32 step ------------------------------------------------------------------------------------
- * Blackwell's packed instructions do two float operations in one issue slot, each rounded as by itself.
- * The step's four coordinates, u and n, go through the same Nystrom stages with the same factors, so they
- * ride in two pairs, (n_x, n_y) and (u, n_z), and the two drag rates in one. */
-typedef unsigned long long F2;
-__device__ __forceinline__ F2 pack(float a, float b) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack(F2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
-    F2 r;
-    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ F2 add2(F2 a, F2 b) {
-    F2 r;
-    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ F2 both(float a) { return pack(a, a); }
-
-__device__ __forceinline__ float bendPoly(const RayConst<float>& c, float x) {
-    return __fmaf_rn(x, __fmaf_rn(x, c.uC, c.uB), c.uA);
-}
-__device__ __forceinline__ float axisAccel(float a2, float c, float z) { return __fmaf_rn(a2, z, -__fmul_rn(c, z)); }
-
-/* nystromStep (lensCore.cuh), each rounding written out as the scalar code's compiles: x + (y + y) is
- * fma(2, y, x), which rounds the same. */
-__device__ __forceinline__ void mixedStep(float a, const RayConst<float>& c, const RayState<float>& s, StepOut<float>& o) {
-    const StepTerms<float> t = stepTerms(c.step);
-    const float a2 = a * a, twoA2 = 2.f * a2;
-    const F2 h = both(c.step), half = both(t.half), eighth = both(t.eighth), halfSq = both(t.halfSquare);
-    const F2 sixthSq = both(t.sixthSquare), sixth = both(t.sixth), two = both(2.f), four = both(4.f);
-    const F2 n = pack(s.n[0], s.n[1]), v = pack(s.v[0], s.v[1]), q = pack(s.u, s.n[2]), w = pack(s.w, s.v[2]);
-    const float k1 = __fmul_rn(s.u, bendPoly(c, s.u));
-    const float c1 = __fmaf_rn(twoA2, __fmul_rn(s.n[2], s.n[2]), c.big);
-    const float a1z = axisAccel(a2, c1, s.n[2]);
-    const F2 a1 = mul2(both(-c1), n), r1 = pack(k1, a1z);
-    const F2 midN = fma2(eighth, a1, fma2(half, v, n)), midQ = fma2(eighth, r1, fma2(half, w, q));
-    float midU, midZ;
-    unpack(midQ, midU, midZ);
-    const float k2 = __fmul_rn(midU, bendPoly(c, midU));
-    const float c2 = __fmaf_rn(twoA2, __fmul_rn(midZ, midZ), c.big);
-    const F2 a2s = mul2(both(-c2), midN), r2 = pack(k2, axisAccel(a2, c2, midZ));
-    const F2 nv = fma2(h, v, n), qw = fma2(h, w, q);
-    const F2 endN = fma2(halfSq, a2s, nv), endQ = fma2(halfSq, r2, qw);
-    float endU, endZ;
-    unpack(endQ, endU, endZ);
-    const float c3 = __fmaf_rn(twoA2, __fmul_rn(endZ, endZ), c.big);
-    /* (the product against zero: a bare one would be fused into the sum after it) */
-    const F2 a13 = add2(a1, fma2(both(-c3), endN, both(0.f)));
-    const F2 r13 = pack(__fmaf_rn(endU, bendPoly(c, endU), k1), __fadd_rn(a1z, axisAccel(a2, c3, endZ)));
-    const F2 nextN = fma2(sixthSq, fma2(two, a2s, a1), nv), nextQ = fma2(sixthSq, fma2(two, r2, r1), qw);
-    const F2 nextV = fma2(sixth, fma2(four, a2s, a13), v), nextW = fma2(sixth, fma2(four, r2, r13), w);
-    unpack(nextN, o.next.n[0], o.next.n[1]);
-    unpack(nextQ, o.next.u, o.next.n[2]);
-    unpack(nextV, o.next.v[0], o.next.v[1]);
-    unpack(nextW, o.next.w, o.next.v[2]);
-    unpack(a1, o.a1[0], o.a1[1]);
-    o.k1 = k1, o.a1[2] = a1z;
-    o.next.drag = o.next.psi = 0.f;
-    if (a != 0.f) {
-        const F2 x = pack(midU, o.next.u);
-        float m0, m1, d0, d1;
-        unpack(mul2(mul2(both(-a), x), fma2(both(-c.xiA), x, two)), m0, m1);
-        unpack(fma2(mul2(both(a2), x), x, fma2(both(-2.f), x, both(1.f))), d0, d1);
-        const float dragMid = __fdividef(m0, fmaxf(d0, 1e-3f));
-        o.next.drag = __fdividef(m1, fmaxf(d1, 1e-3f));
-        o.next.psi = __fmul_rn(t.sixth, __fmaf_rn(4.f, dragMid, __fadd_rn(s.drag, o.next.drag)));
-    }
-}
-
 /* The wide coefficients, their high halves the FP32 ones. */
 __device__ __forceinline__ void setWide(MixedRay& r, Ff uA, Ff uB, Ff uC, Ff xiA) {
     r.c.uA = uA.hi, r.c.uB = uB.hi, r.c.uC = uC.hi, r.c.xiA = xiA.hi;
@@ -436,14 +357,14 @@ __device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t 
         const float light = shadeCrossing(f, v.rhoScale, v.map, v.fluid, r.c, x, r.through, r.sum, &turn);
         if (light > 0.f && !(r.crossings & kLit)) {
             r.crossings |= kLit;
-            if (end) end->hitR = 1.f / x.uc, end->hitPhi = turn - floorf(turn);
+            if (end) end->hitR = recipR(x.uc), end->hitPhi = turn - floorf(turn);
         }
         /* (the transmission only changes here) */
         opaque = !(r.through > .004f);
     }
     ++r.i;
     if (0.f > o.next.u) {
-        const float part = r.s.u / (r.s.u - o.next.u);
+        const float part = divR(r.s.u, r.s.u - o.next.u);
         float away[3], dir[3];
         for (int k = 0; k < 3; ++k) away[k] = r.s.n[k] + part * (o.next.n[k] - r.s.n[k]);
         const float awayPsi = compensated ? r.psiHi + (r.psiLo + part * increment) : r.psiHi + part * increment;
@@ -508,7 +429,7 @@ __device__ __forceinline__ unsigned traceRayMixed(const MixedParams& p, const Mi
     unsigned ended = 0;
     while (!ended) {
         StepOut<float> o;
-        mixedStep(v.f.a, r.c, r.s, o);
+        nystromStep(v.f.a, r.c, r.s, o);
         mixedGuards(guards, v, r, o, rounds);
         ended = mixedAdvance(p, guards, v, r, o, end);
     }

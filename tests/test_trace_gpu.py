@@ -283,3 +283,22 @@ def test_mixed_rays_a_warp_do_not_change_the_image(lib, ctx, width, height, samp
         nx, ny = g.pixel_centres(frame)
         rgb, _ = g.trace_rays(lib, ctx, frame, frame64, capi.MIXED, nx, ny, np.float32(frame.disc[2]))
         assert np.array_equal(rgb.reshape(height, width, 3), base[..., :3])
+
+
+@pytest.mark.parametrize("precision", ["exact", "fp32", "fp64"])
+@pytest.mark.parametrize("width,height", [(1, 1), (9, 5), (61, 40), (200, 112)])
+def test_small_frames_are_their_rays(lib, ctx, precision, width, height):
+    """Small frames, whose warps take parts of a tile: every pixel's ray is the same ray traced by itself, in
+    one launch's order or the queue's."""
+    view = scenes.Scene("small", scenes.hole_desc(0.8), scenes.camera(78.0, 27.0), width, height, seed=5)
+    frame, frame64, clamped = scenes.frame(view)
+    g.set_inputs(lib, ctx, scenes.synth_map(lib, clamped, 5, 3.0), scenes.unit_fluid())
+    p = capi.PRECISIONS[precision]
+    images = [g.trace(lib, ctx, frame, frame64, p, persistent=k)[0] for k in (0, 1)]
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
+    nx, ny = g.pixel_centres(frame)
+    rgb, _ = g.trace_rays(lib, ctx, frame, frame64, p, nx, ny, 0.0)
+    if precision == "fp64":  # (each kernel's doubles may fuse otherwise: a rounding to float apart)
+        np.testing.assert_allclose(images[0][..., :3].reshape(-1, 3), rgb, rtol=2e-7, atol=1e-12)
+    else:
+        assert np.array_equal(images[0][..., :3].reshape(-1, 3), rgb)
