@@ -480,11 +480,13 @@ template <typename R> ARTF_HD void nystromStep(R a, const RayConst<R>& c, const 
     polarStep(a, c, s, o.next, o.a1);
 }
 
-#if defined(__CUDA_ARCH__) && defined(ARTF_PINNED_FMA)
-/* The FP32 step.  Blackwell's packed instructions do two float operations in one issue slot, each rounded
- * as by itself.  The step's four coordinates, u and n, go through the same Nystrom stages with the same
- * factors, so they ride in two pairs, (n_x, n_y) and (u, n_z), and the two drag rates in one: 27 of some
- * 115 instructions a step fewer (the mixed 1080p x 4 frame 1.86 -> 1.76 ms). */
+/* Blackwell's packed instructions do two float operations in one issue slot, each rounded as by itself. */
+#if defined(__CUDA_ARCH__) && (defined(ARTF_PINNED_FMA) || defined(ARTF_EXACT_FLOAT))
+#if defined(ARTF_EXACT_FLOAT)
+#define ARTF_FTZ "" /* (subnormals kept, as the reference keeps them) */
+#else
+#define ARTF_FTZ ".ftz"
+#endif
 typedef unsigned long long F2;
 __device__ __forceinline__ F2 pack(float a, float b) {
     F2 r;
@@ -494,21 +496,26 @@ __device__ __forceinline__ F2 pack(float a, float b) {
 __device__ __forceinline__ void unpack(F2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     F2 r;
-    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    asm("fma.rn" ARTF_FTZ ".f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
 __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
     F2 r;
-    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    asm("mul.rn" ARTF_FTZ ".f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 __device__ __forceinline__ F2 add2(F2 a, F2 b) {
     F2 r;
-    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    asm("add.rn" ARTF_FTZ ".f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 __device__ __forceinline__ F2 both(float a) { return pack(a, a); }
+#endif
 
+#if defined(__CUDA_ARCH__) && defined(ARTF_PINNED_FMA)
+/* The FP32 step, packed.  Its four coordinates, u and n, go through the same Nystrom stages with the same
+ * factors, so they ride in two pairs, (n_x, n_y) and (u, n_z), and the two drag rates in one: 27 of some
+ * 115 instructions a step fewer (the mixed 1080p x 4 frame 1.86 -> 1.76 ms). */
 __device__ __forceinline__ float bendPoly(const RayConst<float>& c, float x) {
     return __fmaf_rn(x, __fmaf_rn(x, c.uC, c.uB), c.uA);
 }
@@ -559,6 +566,63 @@ __device__ __forceinline__ void nystromStep(float a, const RayConst<float>& c, c
         const float dragMid = __fdividef(m0, fmaxf(d0, 1e-3f));
         o.next.drag = __fdividef(m1, fmaxf(d1, 1e-3f));
         o.next.psi = __fmaf_rn(t.sixth, __fmaf_rn(4.f, dragMid, __fadd_rn(s.drag, o.next.drag)), s.psi);
+    }
+}
+#endif
+
+#if defined(__CUDA_ARCH__) && defined(ARTF_EXACT_FLOAT)
+/* A product rounded by itself: against zero, since a bare packed product next to a sum is fused with it
+ * even where scalar ones may not be.  (A product of -0 comes out as +0, which no sum, test or root after
+ * it tells apart.) */
+__device__ __forceinline__ F2 times2(F2 a, F2 b) { return fma2(a, b, both(0.f)); }
+
+/* The exact step, packed as the fast one is, every product and sum rounded by itself in the reference's
+ * order: 2 x and 4 x are exact, so a sum with them may be an FMA, and 0 - c x is one against zero.  (The
+ * exact 1080p x 4 frame 1395 -> 1225 us with the counts out of registers.) */
+template <>
+__device__ __forceinline__ void nystromStep(float a, const RayConst<float>& c, const RayState<float>& s,
+                                            StepOut<float>& o) {
+    const StepTerms<float> t = stepTerms(c.step);
+    const float a2 = a * a, twoA2 = 2.f * a2;
+    const F2 h = both(c.step), half = both(t.half), eighth = both(t.eighth), halfSq = both(t.halfSquare);
+    const F2 sixthSq = both(t.sixthSquare), sixth = both(t.sixth), two = both(2.f), four = both(4.f), zero = both(0.f);
+    const F2 n = pack(s.n[0], s.n[1]), v = pack(s.v[0], s.v[1]), q = pack(s.u, s.n[2]), w = pack(s.w, s.v[2]);
+    const float k1 = bendAt(c, s.u);
+    const float c1 = c.big + twoA2 * (s.n[2] * s.n[2]);
+    const float a1z = a2 * s.n[2] - c1 * s.n[2];
+    const F2 a1 = fma2(both(-c1), n, zero), r1 = pack(k1, a1z);
+    const F2 midN = add2(add2(n, times2(half, v)), times2(eighth, a1));
+    const F2 midQ = add2(add2(q, times2(half, w)), times2(eighth, r1));
+    float midU, midZ;
+    unpack(midQ, midU, midZ);
+    const float k2 = bendAt(c, midU);
+    const float c2 = c.big + twoA2 * (midZ * midZ);
+    const F2 a2s = fma2(both(-c2), midN, zero), r2 = pack(k2, a2 * midZ - c2 * midZ);
+    const F2 nv = add2(n, times2(h, v)), qw = add2(q, times2(h, w));
+    const F2 endN = add2(nv, times2(halfSq, a2s)), endQ = add2(qw, times2(halfSq, r2));
+    float endU, endZ;
+    unpack(endQ, endU, endZ);
+    const float c3 = c.big + twoA2 * (endZ * endZ);
+    const F2 a13 = add2(a1, fma2(both(-c3), endN, zero));
+    const F2 r13 = add2(r1, pack(bendAt(c, endU), a2 * endZ - c3 * endZ));
+    const F2 nextN = add2(nv, times2(sixthSq, fma2(two, a2s, a1))), nextQ = add2(qw, times2(sixthSq, fma2(two, r2, r1)));
+    const F2 nextV = add2(v, times2(sixth, fma2(four, a2s, a13))), nextW = add2(w, times2(sixth, fma2(four, r2, r13)));
+    unpack(nextN, o.next.n[0], o.next.n[1]);
+    unpack(nextQ, o.next.u, o.next.n[2]);
+    unpack(nextV, o.next.v[0], o.next.v[1]);
+    unpack(nextW, o.next.w, o.next.v[2]);
+    unpack(a1, o.a1[0], o.a1[1]);
+    o.k1 = k1, o.a1[2] = a1z;
+    o.next.drag = o.next.psi = 0.f;
+    if (a != 0.f) {
+        const F2 x = pack(midU, o.next.u);
+        const F2 num = times2(times2(both(-a), x), fma2(both(-1.f), times2(both(c.xiA), x), two));
+        float d0, d1, m0, m1;
+        unpack(num, m0, m1);
+        unpack(add2(fma2(both(-2.f), x, both(1.f)), times2(times2(both(a2), x), x)), d0, d1);
+        const float dragMid = m0 / fmaxf(d0, 1e-3f);
+        o.next.drag = m1 / fmaxf(d1, 1e-3f);
+        o.next.psi = s.psi + t.sixth * (s.drag + o.next.drag + 4.f * dragMid);
     }
 }
 #endif

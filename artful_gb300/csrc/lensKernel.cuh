@@ -58,10 +58,42 @@ __device__ __forceinline__ unsigned classBits(unsigned kind) {
     return bits;
 }
 
+/* What a thread counts over its rays, in shared memory: touched once a ray, it would hold registers
+ * through the stepping loop. */
+enum { kTallyRays, kTallySteps, kTallyCrossings, kTallyEscapes, kTallyCount };
+typedef unsigned Tallies[kTallyCount][256];
+
+__device__ __forceinline__ void clearTallies(Tallies& t) {
+    for (int k = 0; k < kTallyCount; ++k) t[k][threadIdx.x] = 0;
+}
+/* A warp's tallies to the launch's counters; the whole warp calls it. */
+__device__ __forceinline__ void flushTallies(const Tallies& t, unsigned long long* counters) {
+    __syncwarp();
+    const int to[kTallyCount] = {CRays, CSteps, CCrossings, CEscapes};
+    for (int k = 0; k < kTallyCount; ++k) {
+        const unsigned n = __reduce_add_sync(0xFFFFFFFFu, t[k][threadIdx.x]);
+        if ((threadIdx.x & 31) == 0 && n) atomicAdd(counters + to[k], (unsigned long long)n);
+    }
+}
+
+/* A finished ray's tallies and the rest of its end record. */
+__device__ __forceinline__ void finishRay(int steps, unsigned crossings, unsigned kind, int wide, ArtfCudaRayEnd* end,
+                                          Tallies& t) {
+    const unsigned add[kTallyCount] = {1u, (unsigned)steps, crossings, (kind & 15u) == ARTF_CUDA_END_SKY ? 1u : 0u};
+    for (int k = 0; k < kTallyCount; ++k) t[k][threadIdx.x] += add[k];
+    if (end) {
+        end->steps = (uint16_t)steps;
+        end->crossings = (uint8_t)(crossings > 255u ? 255u : crossings);
+        end->kind = (uint8_t)kind;
+        end->fp64Steps = (uint16_t)wide;
+        end->reserved = 0;
+    }
+}
+
 /* One ray, from its image position to its end (lens.inc:99-351).  Adds its light to sum (3). */
 template <typename R>
 __device__ __forceinline__ unsigned traceRay(const KernelParams<R>& p, R nx, R ny, R time, R* sum,
-                                             ArtfCudaRayEnd* end, Tally& t) {
+                                             ArtfCudaRayEnd* end, Tallies& t) {
     const Frame<R>& f = p.f;
     RayConst<R> c;
     RayState<R> s;
@@ -72,64 +104,58 @@ __device__ __forceinline__ unsigned traceRay(const KernelParams<R>& p, R nx, R n
 
     R raySum[3] = {R(0), R(0), R(0)}, through = R(1);
     unsigned kind = ARTF_CUDA_END_CAP, crossings = 0;
-    bool lit = false;
-    R hitR = R(NAN), hitPhi = R(NAN), mino = R(p.maxSteps) * c.step, dir[3] = {R(0), R(0), R(0)};
+    if (end) {
+        end->hitR = end->hitPhi = NAN;
+        for (int k = 0; k < 3; ++k) end->dir[k] = 0.f;
+        end->mino = (float)(R(p.maxSteps) * c.step);
+    }
     int i = 0;
-    for (; i < p.maxSteps; ++i) {
+    while (i < p.maxSteps) {
         StepOut<R> o;
         nystromStep(a, c, s, o);
+        ++i;
         Crossing<R> x;
+        bool opaque = false;
         if (crossingOf(f, rhoScale, c, s, o, x)) {
             ++crossings;
             R turn;
             const R light = shadeCrossing(f, rhoScale, p.map, p.fluid, c, x, through, raySum, &turn);
-            if (light > R(0) && !lit) {
-                lit = true;
-                hitR = recipR(x.uc);
-                hitPhi = turn - floorR(turn);
+            if (light > R(0) && !(kind & ARTF_CUDA_END_LIT)) {
+                kind |= ARTF_CUDA_END_LIT;
+                if (end) end->hitR = (float)recipR(x.uc), end->hitPhi = (float)(turn - floorR(turn));
             }
+            opaque = !(through > KF(.004)); /* (the transmission only changes here) */
         }
         if (R(0) > o.next.u) {
             const R part = divR(s.u, s.u - o.next.u);
-            R away[3];
+            R away[3], dir[3];
             for (int k = 0; k < 3; ++k) away[k] = s.n[k] + part * (o.next.n[k] - s.n[k]);
             const R awayPsi = s.psi + part * (o.next.psi - s.psi);
             skyDirection(away, awayPsi, dir);
             if (f.stars > R(0)) shadeSky(f, p.map, c, dir, through, raySum);
-            kind = ARTF_CUDA_END_SKY;
-            mino = (R(i) + part) * c.step;
-            ++i;
+            kind ^= ARTF_CUDA_END_CAP ^ ARTF_CUDA_END_SKY;
+            if (end) {
+                for (int k = 0; k < 3; ++k) end->dir[k] = (float)dir[k];
+                end->mino = (float)((R(i - 1) + part) * c.step);
+            }
             break;
         }
-        if (o.next.u > f.uHorizon) { kind = ARTF_CUDA_END_HORIZON; mino = R(i + 1) * c.step; ++i; break; }
-        if (!(through > KF(.004))) { kind = ARTF_CUDA_END_OPAQUE; mino = R(i + 1) * c.step; ++i; break; }
+        const bool fell = o.next.u > f.uHorizon;
+        if (fell || opaque) {
+            kind ^= ARTF_CUDA_END_CAP ^ (fell ? ARTF_CUDA_END_HORIZON : ARTF_CUDA_END_OPAQUE);
+            if (end) end->mino = (float)(R(i) * c.step);
+            break;
+        }
         s = o.next;
     }
     for (int k = 0; k < 3; ++k) sum[k] = sum[k] + raySum[k];
-    if (lit) kind |= ARTF_CUDA_END_LIT;
-    t.rays += 1;
-    t.steps += (unsigned)i;
-    t.crossings += crossings;
-    t.escapes += (kind & 15u) == ARTF_CUDA_END_SKY;
-    if (end) {
-        ArtfCudaRayEnd e;
-        e.hitR = (float)hitR;
-        e.hitPhi = (float)hitPhi;
-        for (int k = 0; k < 3; ++k) e.dir[k] = (float)dir[k];
-        e.mino = (float)mino;
-        e.steps = (uint16_t)i;
-        e.crossings = (uint8_t)(crossings > 255u ? 255u : crossings);
-        e.kind = (uint8_t)kind;
-        e.fp64Steps = (uint16_t)(sizeof(R) == 8 ? i : 0);
-        e.reserved = 0;
-        *end = e;
-    }
+    finishRay(i, crossings, kind, sizeof(R) == 8 ? i : 0, end, t);
     return kind;
 }
 
 /* All rays of one pixel, summed in the reference's order and scaled by 1 / rays (lens.inc:364-380). */
 template <typename R> __device__ __forceinline__ void tracePixel(const KernelParams<R>& p, int32_t x, int32_t y,
-                                                                  Tally& t) {
+                                                                  Tallies& t) {
     const size_t pixel = (size_t)y * (size_t)p.f.width + (size_t)x;
     R sum[3] = {R(0), R(0), R(0)};
     unsigned bits = 0;
@@ -150,7 +176,7 @@ template <typename R> __device__ __forceinline__ void tracePixel(const KernelPar
 }
 
 /* A warp's part of this launch's tiles: pixels row by row, a thread each, 8 x 4 of them or fewer. */
-template <typename R> __device__ __forceinline__ void tracePart(const KernelParams<R>& p, unsigned part, Tally& t) {
+template <typename R> __device__ __forceinline__ void tracePart(const KernelParams<R>& p, unsigned part, Tallies& t) {
     const int lane = threadIdx.x & 31;
     const unsigned first = part << p.lanesLog2, within = (first & 31u) + (unsigned)lane;
     const int tile = p.tileBegin + (int)(first >> 5);
@@ -158,18 +184,26 @@ template <typename R> __device__ __forceinline__ void tracePart(const KernelPara
     if (lane >> p.lanesLog2 == 0 && x < p.f.width && y < p.f.height) tracePixel(p, x, y, t);
 }
 
+/* Blocks of 256 a SM the registers are cut for: 128 registers a thread in float (what the compiler takes by
+ * itself, 80 in the exact trace, leaves a ray's stages too little in flight: 58.7 against 54.0 us for the
+ * exact 320 x 180 frame, 1267 against 1225 for 1080p x 4; 168 and 96 are slower too); in double none (186:
+ * 2381 against 2803 us at 128, 960 x 540). */
+template <typename R> constexpr int kBlocks = sizeof(R) == 4 ? 2 : 1;
+
 /* One warp per part, one thread per pixel. */
-template <typename R> __global__ void __launch_bounds__(256) traceTiles(const KernelParams<R> p) {
+template <typename R> __global__ void __launch_bounds__(256, kBlocks<R>) traceTiles(const KernelParams<R> p) {
     const unsigned part = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    Tally t;
+    __shared__ Tallies t;
+    clearTallies(t);
     if (part < (unsigned)p.tiles << 5 >> p.lanesLog2) tracePart(p, part, t);
-    flushTally(t, p.counters);
+    flushTallies(t, p.counters);
 }
 
 /* Persistent: a grid of resident warps that pull parts from the queue counter until none is left. */
-template <typename R> __global__ void __launch_bounds__(256) traceQueue(const KernelParams<R> p) {
+template <typename R> __global__ void __launch_bounds__(256, kBlocks<R>) traceQueue(const KernelParams<R> p) {
     const unsigned parts = (unsigned)p.tiles << 5 >> p.lanesLog2;
-    Tally t;
+    __shared__ Tallies t;
+    clearTallies(t);
     for (;;) {
         unsigned part = 0;
         if ((threadIdx.x & 31) == 0) part = (unsigned)atomicAdd(p.counters + CQueue, 1ull);
@@ -178,7 +212,7 @@ template <typename R> __global__ void __launch_bounds__(256) traceQueue(const Ke
         tracePart(p, part, t);
         __syncwarp();
     }
-    flushTally(t, p.counters);
+    flushTallies(t, p.counters);
 }
 
 /* A list of rays at given image positions, one a thread (the per-ray entry point). */
@@ -192,13 +226,14 @@ struct RayList {
 
 template <typename R> __global__ void __launch_bounds__(128) traceList(const KernelParams<R> p, const RayList l) {
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    Tally t;
+    __shared__ Tallies t;
+    clearTallies(t);
     if (i < l.n) {
         R sum[3] = {R(0), R(0), R(0)};
         traceRay(p, R(l.nx[i]), R(l.ny[i]), R(l.time[i]), sum, p.ends ? p.ends + i : nullptr, t);
         for (int k = 0; k < 3; ++k) l.rgb[3 * i + k] = (float)sum[k];
     }
-    flushTally(t, p.counters);
+    flushTallies(t, p.counters);
 }
 
 template <typename R> cudaError_t launchUniform(const TraceLaunch& l, const void* frameSource) {
@@ -238,8 +273,10 @@ template <typename R> cudaError_t launchUniform(const TraceLaunch& l, const void
          * its warps take half a tile each, and so on down to two pixels, and have fewer rays that part ways
          * (exact, 61 x 40: 76 -> 44 us; 200 x 112: 61 -> 54; FP32 160 x 90 x 4: 116 -> 89; parts for more
          * warps than there are cost more: 200 x 112 66 us).  In double a warp holds the FP64 pipe as long for
-         * two lanes as for 32, so there it keeps them. */
-        while (sizeof(R) == 4 && p.lanesLog2 > 1 && ((long long)p.tiles << 5 >> p.lanesLog2) * 2 <= warps) --p.lanesLog2;
+         * two lanes as for 32, so there parts are made up to eight warps a SM (61 x 40: 497 -> 325 us, 160 x
+         * 90 547 -> 489). */
+        const long long most = sizeof(R) == 4 ? warps : 8ll * l.smCount;
+        while (p.lanesLog2 > 1 && ((long long)p.tiles << 5 >> p.lanesLog2) * 2 <= most) --p.lanesLog2;
         const long long blocks = (((long long)p.tiles << 5 >> p.lanesLog2) * 32 + block - 1) / block;
         if (l.persistent) traceQueue<R><<<(unsigned)(blocks < slots ? blocks : slots), block, 0, l.stream>>>(p);
         else traceTiles<R><<<(unsigned)blocks, block, 0, l.stream>>>(p);

@@ -391,7 +391,7 @@ __device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t 
 
 /* What a thread counts over its rays, in shared memory: touched once a ray, it would hold ten registers
  * through the stepping loop. */
-enum { kTallyRays, kTallySteps, kTallyCrossings, kTallyEscapes, kTallyWide, kTallyBand, kTallyRadial, kTallyPolar, kTallyCount };
+enum { kMixedRays, kMixedSteps, kMixedCrossings, kMixedEscapes, kMixedWide, kMixedBand, kMixedRadial, kMixedPolar, kMixedCount };
 
 /* The end record of a finished ray, and its tallies. */
 __device__ __forceinline__ unsigned mixedFinish(const MixedRay& r, unsigned ended, ArtfCudaRayEnd* end,
@@ -400,9 +400,9 @@ __device__ __forceinline__ unsigned mixedFinish(const MixedRay& r, unsigned ende
     if (r.crossings & kLit) kind |= ARTF_CUDA_END_LIT;
     const unsigned crossings = r.crossings & ~kLit;
     const bool sky = (kind & 15u) == ARTF_CUDA_END_SKY;
-    const unsigned add[kTallyCount] = {1u, (unsigned)r.i, crossings, sky ? 1u : 0u, r.wide & 0xFFFFu, r.wide >> 16,
+    const unsigned add[kMixedCount] = {1u, (unsigned)r.i, crossings, sky ? 1u : 0u, r.wide & 0xFFFFu, r.wide >> 16,
                                        r.turns & 0xFFFFu, r.turns >> 16};
-    for (int k = 0; k < kTallyCount; ++k) tally[k][threadIdx.x] += add[k];
+    for (int k = 0; k < kMixedCount; ++k) tally[k][threadIdx.x] += add[k];
     if (end) {
         const double step = ffWide(Ff{r.c.step, r.stepLo});
         for (int k = 0; k < 3; ++k) end->dir[k] = sky ? r.s.n[k] : 0.f;
@@ -437,15 +437,15 @@ __device__ __forceinline__ unsigned traceRayMixed(const MixedParams& p, const Mi
     return mixedFinish(r, ended, end, tally);
 }
 
-__device__ __forceinline__ void clearTallies(unsigned (*tally)[256]) {
-    for (int k = 0; k < kTallyCount; ++k) tally[k][threadIdx.x] = 0;
+__device__ __forceinline__ void clearMixed(unsigned (*tally)[256]) {
+    for (int k = 0; k < kMixedCount; ++k) tally[k][threadIdx.x] = 0;
 }
 
 /* A warp's tallies to the launch's counters; the whole warp calls it. */
-__device__ __forceinline__ void flushTallies(unsigned (*tally)[256], unsigned rounds, unsigned long long* counters) {
-    const int to[kTallyCount] = {CRays, CSteps, CCrossings, CEscapes, CFp64Steps, CFp64Horizon, CFp64Radial, CFp64Polar};
+__device__ __forceinline__ void flushMixed(unsigned (*tally)[256], unsigned rounds, unsigned long long* counters) {
+    const int to[kMixedCount] = {CRays, CSteps, CCrossings, CEscapes, CFp64Steps, CFp64Horizon, CFp64Radial, CFp64Polar};
     const bool first = (threadIdx.x & 31) == 0;
-    for (int k = 0; k < kTallyCount; ++k) {
+    for (int k = 0; k < kMixedCount; ++k) {
         const unsigned n = __reduce_add_sync(0xFFFFFFFFu, tally[k][threadIdx.x]);
         if (first && n) atomicAdd(counters + to[k], (unsigned long long)n);
     }
@@ -581,10 +581,10 @@ __global__ void __launch_bounds__(128) placeOne(const MixedParams p, const __gri
  * rather than from the view table. */
 template <bool kOne, bool kAll>
 __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView* one) {
-    __shared__ unsigned tally[kTallyCount][256];
+    __shared__ unsigned tally[kMixedCount][256];
     const int lane = threadIdx.x & 31;
     unsigned rounds = 0;
-    clearTallies(tally);
+    clearMixed(tally);
     const unsigned parts = (unsigned)(p.totalUnits >> p.lanesLog2); /* 2^lanesLog2 rays each */
     for (;;) {
         unsigned part = 0;
@@ -640,7 +640,7 @@ __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView
         }
         __syncwarp();
     }
-    flushTallies(tally, rounds, p.counters);
+    flushMixed(tally, rounds, p.counters);
 }
 
 /* The views from the table (a batch).  The kernels come in pairs: the guards chosen at run time, and all
@@ -685,16 +685,16 @@ __global__ void __launch_bounds__(128) traceMixedList(const MixedParams p,
                                                       const __grid_constant__ MixedView view, const int count,
                                                       const float* nx, const float* ny, const float* time, float* rgb) {
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    __shared__ unsigned tally[kTallyCount][256];
+    __shared__ unsigned tally[kMixedCount][256];
     unsigned rounds = 0;
-    clearTallies(tally);
+    clearMixed(tally);
     if (i < count) {
         float sum[3] = {0.f, 0.f, 0.f};
         traceRayMixed<false>(p, view, nx[i], ny[i], time[i], sum, view.ends ? view.ends + i : nullptr, tally, rounds);
         for (int k = 0; k < 3; ++k) rgb[3 * i + k] = sum[k];
     }
     __syncwarp();
-    flushTallies(tally, rounds, p.counters);
+    flushMixed(tally, rounds, p.counters);
 }
 
 MixedParams paramsOf(const TraceLaunch& l, const void* deviceTable, int viewCount, int totalUnits) {

@@ -16,7 +16,8 @@ using D5 = Dual<5>;
 
 __global__ void __launch_bounds__(64) traceTangents(const KernelParams<D5> p, double* out) {
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    Tally t;
+    __shared__ Tallies t;
+    clearTallies(t);
     const int pixels = p.f.width * p.f.height;
     if (i < pixels) {
         const int x = i % p.f.width, y = i / p.f.width;
@@ -30,7 +31,7 @@ __global__ void __launch_bounds__(64) traceTangents(const KernelParams<D5> p, do
             for (int k = 0; k < 5; ++k) o[1 + k] = sum[c].d[k];
         }
     }
-    flushTally(t, p.counters);
+    flushTallies(t, p.counters);
 }
 
 }  // namespace
