@@ -33,11 +33,16 @@ static float fclampRef(float v, float lo, float hi) { return v < lo ? lo : v > h
 
 /* ---- orbits ------------------------------------------------------------------------------------- */
 
-/* x^(1/3) for x > 0 by Newton's iteration, 60 rounds from max(x, 1): converged to the last bit. */
+/* x^(1/3) for x > 0 by Newton's iteration, 60 rounds from max(x, 1): converged to the last bit, and left
+ * once a round changes nothing (no later one would: six to ten rounds instead of 60). */
 static double cubeRootNewton(double x) {
     if (x <= 0) return 0;
     double v = x > 1 ? x : 1;
-    for (int i = 0; i < 60; ++i) v = (2.0 * v + x / (v * v)) / 3.0;
+    for (int i = 0; i < 60; ++i) {
+        const double next = (2.0 * v + x / (v * v)) / 3.0;
+        if (next == v) break;
+        v = next;
+    }
     return v;
 }
 
@@ -355,7 +360,8 @@ static double iscoDouble(double a) {
     return 3.0 + z2 - (a < 0 ? -root : root);
 }
 
-static DScene paramsScene(const ArtfCudaHoleParams* p, const double* theta) {
+/* isco: iscoDouble of the spin, theta[0]. */
+static DScene paramsScene(const ArtfCudaHoleParams* p, const double* theta, double isco) {
     DScene s;
     memset(&s, 0, sizeof s);
     const double a = theta[0], i = theta[1], scale = theta[2], r = theta[4];
@@ -366,7 +372,7 @@ static DScene paramsScene(const ArtfCudaHoleParams* p, const double* theta) {
     s.holePosition = dvec(0, 0, 0);
     s.axis = dvec(0, 1, 0);
     s.velocity = dvec(0, 0, 0);
-    s.mass = 1.0, s.spin = a, s.inner = scale * iscoDouble(a), s.outer = p->outer, s.height = p->height;
+    s.mass = 1.0, s.spin = a, s.inner = scale * isco, s.outer = p->outer, s.height = p->height;
     s.shutter = 0.0, s.time = p->time, s.thickness = p->thickness, s.gain = p->gain, s.doppler = p->doppler;
     s.stars = p->stars, s.bloom = 0.0, s.exposure = 1.0, s.samples = 1;
     return s;
@@ -395,7 +401,7 @@ int artfCudaHoleParamsScene(const ArtfCudaHoleParams* p, ArtfCudaCamera* camera,
     if (!p || !camera || !desc || !paramsValid(p)) return ARTF_CUDA_EINVAL;
     double theta[5];
     thetaOf(p, theta);
-    const DScene s = paramsScene(p, theta);
+    const DScene s = paramsScene(p, theta, iscoDouble(theta[0]));
     memset(camera, 0, sizeof *camera);
     camera->position = vec((float)s.position.x, (float)s.position.y, (float)s.position.z);
     camera->up = vec(0, 1, 0);
@@ -445,11 +451,12 @@ int artfCudaHoleParamsFrames(const ArtfCudaHoleParams* p, int width, int height,
         if (!artfCudaHoleFrame(&camera, &desc, desc.time, width, height, f32)) return ARTF_CUDA_EINVAL;
     }
     if (f64) {
-        const DScene s = paramsScene(p, theta);
+        const DScene s = paramsScene(p, theta, iscoDouble(theta[0]));
         frame64Of(&s, s.time, width, height, f64);
     }
     if (jacobian) {
         /* central differences of the double frame, step 1e-6 of each parameter's scale */
+        const double isco = iscoDouble(theta[0]);
         for (int q = 0; q < 5; ++q) {
             double up[5], down[5];
             memcpy(up, theta, sizeof up);
@@ -458,7 +465,8 @@ int artfCudaHoleParamsFrames(const ArtfCudaHoleParams* p, int width, int height,
             up[q] += h;
             down[q] -= h;
             ArtfCudaHoleFrame64 fu, fd;
-            const DScene su = paramsScene(p, up), sd = paramsScene(p, down);
+            const DScene su = paramsScene(p, up, q == 0 ? iscoDouble(up[0]) : isco);
+            const DScene sd = paramsScene(p, down, q == 0 ? iscoDouble(down[0]) : isco);
             frame64Of(&su, su.time, width, height, &fu);
             frame64Of(&sd, sd.time, width, height, &fd);
             double gu[ARTF_CUDA_GRAD_FIELDS], gd[ARTF_CUDA_GRAD_FIELDS];

@@ -45,6 +45,18 @@ def theta_of(p: capi.HoleParams) -> np.ndarray:
     return np.array([getattr(p, n) for n in PARAM_NAMES], np.float64)
 
 
+def packed(params) -> C.Array:
+    """The parameter records of several views, side by side as the C ABI takes them."""
+    return params if isinstance(params, C.Array) else (capi.HoleParams * len(params))(*params)
+
+
+def packed_with_theta(base: C.Array, theta: np.ndarray) -> C.Array:
+    """base's records with their five parameters (the records' first doubles) replaced: (n, 5)."""
+    out = type(base).from_buffer_copy(base)
+    np.frombuffer(out, np.float64).reshape(len(base), -1)[:, :5] = theta
+    return out
+
+
 def with_theta(p: capi.HoleParams, theta) -> capi.HoleParams:
     q = capi.HoleParams()
     C.memmove(C.byref(q), C.byref(p), C.sizeof(capi.HoleParams))
@@ -117,7 +129,7 @@ class Adjoint:
 
     def __call__(self, params, targets, hdr=None, checkpoint: int | None = None, pixel_grads=None):
         n = len(params)
-        arr = (capi.HoleParams * n)(*params)
+        arr = packed(params)
         res = (capi.AdjointResult * n)()
         stats = capi.TraceStats()
         capi.check(self.lib.artfCudaHoleAdjoint(
@@ -125,9 +137,8 @@ class Adjoint:
             checkpoint or self.checkpoint, hdr.data_ptr() if hdr is not None else None,
             pixel_grads.data_ptr() if pixel_grads is not None else None, res, C.byref(stats)))
         self.last_stats = stats
-        loss = np.array([r.loss for r in res], np.float64)
-        grad = np.array([list(r.grad) for r in res], np.float64)
-        return loss, grad, stats
+        out = np.frombuffer(res, np.float64).reshape(n, 6)
+        return out[:, 0].copy(), out[:, 1:].copy(), stats
 
     def render(self, params):
         """The adjoint's own forward radiance for each view (its loss against a zero target)."""
@@ -146,7 +157,7 @@ def hole_loss():
     class HoleLoss(torch.autograd.Function):
         @staticmethod
         def forward(fctx, theta, adjoint, base, targets):
-            params = [with_theta(b, t) for b, t in zip(base, theta.detach().cpu().numpy())]
+            params = packed_with_theta(packed(base), theta.detach().cpu().numpy())
             loss, grad, _ = adjoint(params, targets)
             fctx.save_for_backward(torch.from_numpy(grad))
             return torch.from_numpy(loss)
