@@ -15,16 +15,17 @@
  * up.  The random draws that place the eddies (a xorshift sequence) are made on the host, in the
  * reference's order, and travel with the launches as kernel parameters.
  *
- * Work layout: 7 fields of 256 x 1024 floats (7 MB, L2-resident), one allocation.  A step is two launches
- * on the context's stream: `velocities`, a thread a cell; and `ringStep`, a block a ring, which does all
- * that follows within the ring: its new densities, its shift along itself, its mean drawn to 1, the next
- * step's eddies, and after the last step the field.  What bounds a step is latency: the sum in cell order
- * (1024 dependent additions, 2.1 us) and the two launches; the fields are read and written once.  One
- * block working through the eddies, and a launch a pass, took 62 us a step; this takes 11 (24 steps
- * of a 1024 x 256 gas, a call: 1486 -> 265 us; of that the launches as dependent ones 387 -> 265). */
+ * Work layout: 7 fields of 256 x 1024 floats (7 MB, L2-resident), one allocation.  A step is one launch on
+ * the context's stream, `gasStep`: a block a ring, in clusters of eight rings that exchange what a ring
+ * needs of its neighbours through shared memory.  What bounds a step is latency: the sum in cell order (1024
+ * dependent additions, 1.9 us), three reads in turn of fields that other SMs have just written, and one
+ * launch waiting for the last.  One block working through the eddies, and a launch a pass, took 62 us a
+ * step; a launch for the velocities and one for the rest of each ring 10.8, this takes 9.7 (24 steps a call:
+ * 1486 -> 265 -> 241 us; of that the launches as dependent ones 387 -> 265). */
 #include "nvtxRange.h"
 #include "artful_cuda.h"
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdlib.h>
@@ -48,6 +49,7 @@ constexpr int EDDIES_A_STEP = 16;          /* fluid.c:232-234: two large, fourte
 constexpr int START_EDDIES = 200;          /* fluid.c:312 */
 constexpr int EDDIES_A_LAUNCH = 128;       /* a launch's room for them */
 constexpr int RING_THREADS = 512;          /* a ring's block: two cells a thread */
+constexpr int RINGS = 8;                   /* a cluster's rings */
 constexpr int FIELD = FW * FH;
 
 /* What a cell's passes take from its ring alone (fluid.c:98-106, 128-135, 155-165, 270-287), formed once on
@@ -175,8 +177,8 @@ __device__ __forceinline__ void stirDensity(const Eddy& q, float r, int i, float
     if (eddyAt(q, r, i, shape, dr, dx)) s = clampF(s * (1.f + q.clump * shape), .03f, 8.f);
 }
 
-/* Eddies on their own (those of a gas's start, and of a run's first step): a block a ring, so that an eddy
- * out of the ring's reach costs the block one uniform test. */
+/* Eddies on their own (a gas's start, and its first step's): a block a ring, so that an eddy out of the
+ * ring's reach costs the block one uniform test. */
 __global__ void __launch_bounds__(RING_THREADS) stir(float* s, float* vr, float* w, const Ring* __restrict__ rings,
                                                      const __grid_constant__ Eddies<EDDIES_A_LAUNCH> eddies) {
     const int j = (int)blockIdx.x;
@@ -194,15 +196,10 @@ __global__ void __launch_bounds__(RING_THREADS) stir(float* s, float* vr, float*
     }
 }
 
-/* fluid.c:96-124 */
-__global__ void __launch_bounds__(256) velocities(const float* s, const float* vr, const float* w, float* outR,
-                                                  float* outW, const Ring* __restrict__ rings) {
-    const int cell = (int)(blockIdx.x * 256 + threadIdx.x); /* (256 divides the field) */
-    const int j = (int)(blockIdx.x * 256) / FW, i = cell - j * FW; /* (a block's cells are of one ring) */
-    const Ring g = rings[j];
-    startNext();
-    waitBefore();
-    const int up = atMost(j + 1, FH - 1), down = atLeast(j - 1, 0);
+/* fluid.c:96-124: a cell's new velocities */
+__device__ __forceinline__ void velocitiesAt(const float* s, const float* vr, const float* w, const Ring& g, int j, int i,
+                                             float& outR, float& outW) {
+    const int cell = j * FW + i, up = atMost(j + 1, FH - 1), down = atLeast(j - 1, 0);
     const float x = (float)i - w[cell] * g.toCells, y = (float)j - vr[cell] * g.toRows;
     const float v0 = bilinear(vr, x, y), w0 = bilinear(w, x, y);
     const float inv = 1.f / s[cell];
@@ -211,19 +208,19 @@ __global__ void __launch_bounds__(256) velocities(const float* s, const float* v
                           g.invArc * inv;
     const float w1 = w0 + DT * (-g.epicyclic * v0 - v0 * w0 * g.invR - g.sound2 * gradPhi);
     const float v1 = v0 + DT * (2.f * g.angular * w1 + w1 * w1 * g.invR - g.sound2 * gradR);
-    outW[cell] = clampF(w1 * g.keep, -.4f, .4f);
-    outR[cell] = clampF(v1 * g.keep, -.4f, .4f);
+    outW = clampF(w1 * g.keep, -.4f, .4f);
+    outR = clampF(v1 * g.keep, -.4f, .4f);
 }
 
-/* fluid.c:126-151: a cell's new density */
-__device__ __forceinline__ float densityAt(const float* s, const float* vr, const float* w, const Ring& g, int j, int i) {
-    const int cell = j * FW + i;
-    const int up = atMost(j + 1, FH - 1), down = atLeast(j - 1, 0);
+/* fluid.c:126-151: a cell's new density, from the old ones and the new velocities: its ring's (vr, w), and
+ * the radial ones of the rings above and below at its column. */
+__device__ __forceinline__ float densityAt(const float* s, const float* vr, const float* w, float vrUp, float vrDown,
+                                           const Ring& g, int j, int i) {
     const float drift = -.004f;
-    const float x = (float)i - w[cell] * g.toCells, y = (float)j - (vr[cell] + drift) * g.toRows;
+    const float x = (float)i - w[i] * g.toCells, y = (float)j - (vr[i] + drift) * g.toRows;
     const float moved = bilinear(s, x, y);
-    const float spread = (g.up * vr[(size_t)up * FW + i] - g.down * vr[(size_t)down * FW + i]) * g.invSpan * g.invR +
-                         (w[(size_t)j * FW + ((i + 1) & (FW - 1))] - w[(size_t)j * FW + ((i - 1) & (FW - 1))]) * g.invArc;
+    const float spread = (g.up * vrUp - g.down * vrDown) * g.invSpan * g.invR +
+                         (w[(i + 1) & (FW - 1)] - w[(i - 1) & (FW - 1)]) * g.invArc;
     const float next = moved * (1.f - DT * clampF(spread, -2.f, 2.f));
     return clampF(next + (1.f - next) * g.refill, .03f, 8.f);
 }
@@ -237,25 +234,28 @@ __device__ __forceinline__ float slideCell(const float* in, int i, const Ring& g
     return clampF(g.k0 * p0 + g.k1 * p1 + g.k2 * p2 + g.k3 * p3, lesser(p1, p2), greater(p1, p2));
 }
 
-/* The rest of a step, within a ring: the new densities from the old (s) and the new velocities (vr, w),
- * the shift of the three fields along the ring, the mean drawn to 1 (fluid.c:221-229: a sum in cell order,
- * by one thread, while the others stir the velocities), the next step's eddies, and, when `field` is
- * given, what shows of the ring (fluid.c:175-186).  Rings read their neighbours' old density and new
- * velocities and write neither. */
-__global__ void __launch_bounds__(RING_THREADS) ringStep(const float* s, const float* vr, const float* w, float* outS,
-                                                         float* outR, float* outW, const Ring* __restrict__ rings,
-                                                         float* field,
-                                                         const __grid_constant__ Eddies<EDDIES_A_STEP> eddies) {
-    constexpr int CELLS = FW / RING_THREADS;
+/* A step: a block a ring, clusters of RINGS neighbouring rings.  Each block finds its ring's new velocities
+ * from the old fields; the new densities take the neighbours' radial ones, which the cluster's blocks read
+ * from one another's shared memory (the rings the cluster borders on are found by all its blocks, a share
+ * each); the rest stays within the ring: the shift of the three fields along it, the mean drawn to 1
+ * (fluid.c:221-229: a sum in cell order, by one thread of a warp of its own, while the others stir the
+ * velocities), the next step's eddies, and, when `field` is given, what shows of the ring
+ * (fluid.c:175-186).  The fields are read from one copy and written to the other. */
+__global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 32)
+    gasStep(const float* s, const float* vr, const float* w, float* outS, float* outR, float* outW,
+            const Ring* __restrict__ rings, float* field, const __grid_constant__ Eddies<EDDIES_A_STEP> eddies) {
+    constexpr int CELLS = FW / RING_THREADS, SHARE = FW / RINGS;
     __shared__ __align__(16) float ringS[FW];
-    __shared__ float ringR[FW], ringW[FW];
+    __shared__ float ringR[FW], ringW[FW], outer[FW]; /* outer: of the ring beyond, in the first and last block */
     __shared__ uint32_t reaching; /* the eddies that reach the ring at all, a bit each */
     __shared__ float scale;
-    const int j = (int)blockIdx.x;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int tid = (int)threadIdx.x, j = (int)blockIdx.x, rank = j % RINGS;
+    const bool helper = tid >= RING_THREADS;
     const Ring g = rings[j];
     const size_t row = (size_t)j * FW;
-    if (threadIdx.x < 32) {
-        const int e = (int)threadIdx.x;
+    if (helper) {
+        const int e = tid - RING_THREADS;
         const float dr = e < eddies.count ? g.radius - eddies.e[e & (EDDIES_A_STEP - 1)].r0 : 0.f;
         const float size = eddies.e[e & (EDDIES_A_STEP - 1)].size;
         const uint32_t bits = __ballot_sync(0xFFFFFFFFu, e < eddies.count && !(dr * dr > 6.25f * size * size));
@@ -263,45 +263,76 @@ __global__ void __launch_bounds__(RING_THREADS) ringStep(const float* s, const f
     }
     startNext();
     waitBefore();
+    if (!helper) {
 #pragma unroll
-    for (int c = 0; c < CELLS; ++c) {
-        const int i = (int)threadIdx.x + c * RING_THREADS;
-        ringS[i] = densityAt(s, vr, w, g, j, i);
-        ringR[i] = vr[row + i], ringW[i] = w[row + i];
+        for (int c = 0; c < CELLS; ++c) {
+            const int i = tid + c * RING_THREADS;
+            velocitiesAt(s, vr, w, g, j, i, ringR[i], ringW[i]);
+        }
+        /* this block's share of the rings below and above the cluster, where there are any (found whole by the
+         * outer blocks they cost 1.3 us a step) */
+        if (tid < 2 * SHARE) {
+            const bool below = tid < SHARE;
+            const int beyond = j - rank + (below ? -1 : RINGS), i = rank * SHARE + (below ? tid : tid - SHARE);
+            if (beyond >= 0 && beyond < FH) {
+                float unused;
+                velocitiesAt(s, vr, w, rings[beyond], beyond, i, cluster.map_shared_rank(outer, below ? 0 : RINGS - 1)[i],
+                             unused);
+            }
+        }
     }
+    cluster.sync();
+    if (!helper) {
+        /* (the first and last ring border on themselves) */
+        const float* below = rank > 0 ? cluster.map_shared_rank(ringR, rank - 1) : j > 0 ? outer : ringR;
+        const float* above = rank < RINGS - 1 ? cluster.map_shared_rank(ringR, rank + 1) : j < FH - 1 ? outer : ringR;
+#pragma unroll
+        for (int c = 0; c < CELLS; ++c) {
+            const int i = tid + c * RING_THREADS;
+            ringS[i] = densityAt(s, ringR, ringW, above[i], below[i], g, j, i);
+        }
+    }
+    /* (no block leaves while a neighbour may read its ring: waited for at the end) */
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     __syncthreads();
     float slidS[CELLS], slidR[CELLS], slidW[CELLS];
+    if (!helper) {
 #pragma unroll
-    for (int c = 0; c < CELLS; ++c) {
-        const int i = (int)threadIdx.x + c * RING_THREADS;
-        slidS[c] = slideCell(ringS, i, g);
-        slidR[c] = slideCell(ringR, i, g);
-        slidW[c] = slideCell(ringW, i, g);
+        for (int c = 0; c < CELLS; ++c) slidS[c] = slideCell(ringS, tid + c * RING_THREADS, g);
     }
     __syncthreads();
+    if (!helper) {
 #pragma unroll
-    for (int c = 0; c < CELLS; ++c) ringS[threadIdx.x + c * RING_THREADS] = slidS[c];
+        for (int c = 0; c < CELLS; ++c) ringS[tid + c * RING_THREADS] = slidS[c];
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float sum = 0;
-        const float4* four = reinterpret_cast<const float4*>(ringS);
+    if (helper) {
+        if (tid == RING_THREADS) {
+            float sum = 0;
+            const float4* four = reinterpret_cast<const float4*>(ringS);
 #pragma unroll 16
-        for (int i = 0; i < FW / 4; ++i) {
-            const float4 q = four[i];
-            sum += q.x;
-            sum += q.y;
-            sum += q.z;
-            sum += q.w;
+            for (int i = 0; i < FW / 4; ++i) {
+                const float4 q = four[i];
+                sum += q.x;
+                sum += q.y;
+                sum += q.z;
+                sum += q.w;
+            }
+            const float mean = sum * (1.f / (float)FW);
+            scale = 1.f + .03f * (1.f / mean - 1.f);
         }
-        const float mean = sum * (1.f / (float)FW);
-        scale = 1.f + .03f * (1.f / mean - 1.f);
+        __syncthreads();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return;
     }
     /* The eddies near each cell: of the 16 some four reach a ring, and each a few dozen of its 1024 columns,
      * so most cells are done with a test of columns an eddy. */
     uint32_t near[CELLS];
 #pragma unroll
     for (int c = 0; c < CELLS; ++c) {
-        const int i = (int)threadIdx.x + c * RING_THREADS;
+        const int i = tid + c * RING_THREADS;
+        slidR[c] = slideCell(ringR, i, g);
+        slidW[c] = slideCell(ringW, i, g);
         near[c] = 0;
         for (uint32_t bits = reaching; bits; bits &= bits - 1) {
             const Eddy& q = eddies.e[__ffs((int)bits) - 1];
@@ -314,7 +345,7 @@ __global__ void __launch_bounds__(RING_THREADS) ringStep(const float* s, const f
     __syncthreads();
 #pragma unroll
     for (int c = 0; c < CELLS; ++c) {
-        const int i = (int)threadIdx.x + c * RING_THREADS;
+        const int i = tid + c * RING_THREADS;
         float v = clampF(slidS[c] * scale, .03f, 8.f);
         if (field) {
             const float shown = v * g.envelope;
@@ -324,6 +355,7 @@ __global__ void __launch_bounds__(RING_THREADS) ringStep(const float* s, const f
             stirDensity(eddies.e[__ffs((int)bits) - 1], g.radius, i, v);
         outS[row + i] = v;
     }
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 }  // namespace
@@ -337,7 +369,7 @@ struct ArtfCudaFluid {
     float* radial[2];
     float* orbital[2];
     float* field;
-    int cur;               /* which density copy is the current one (the velocities' is always 0) */
+    int cur;               /* which copy of the three fields is the current one */
     Ring* rings;           /* device copy */
     Ring host[FH];
     uint32_t state;        /* fluid.c:49 xorshift32 */
@@ -381,9 +413,8 @@ Eddy placeEddy(ArtfCudaFluid* f, bool small) {
     return q;
 }
 
-/* The next `large` large and `small` small eddies, drawn in that order. */
+/* The next `large` large and `small` small eddies, drawn in that order, after those q holds. */
 template <int N> void drawEddies(ArtfCudaFluid* f, Eddies<N>& q, int large, int small) {
-    q.count = 0;
     for (int e = 0; e < large; ++e) q.e[q.count++] = placeEddy(f, false);
     for (int e = 0; e < small; ++e) q.e[q.count++] = placeEddy(f, true);
 }
@@ -399,30 +430,35 @@ cudaError_t follow(ArtfCudaFluid* f, void (*kernel)(P...), unsigned blocks, unsi
     return cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
-/* `steps` steps, one at least (fluid.c:231-241), after `extra` eddies of the start, and the field after them. */
-int advanceSteps(ArtfCudaFluid* f, int extra, int64_t steps) {
-    Eddies<EDDIES_A_LAUNCH> first;
+static_assert(START_EDDIES % EDDIES_A_LAUNCH + EDDIES_A_STEP <= EDDIES_A_LAUNCH, "the last launch holds both");
+
+/* A gas's start: its eddies (fluid.c:309-313), and its first step's. */
+int stirStart(ArtfCudaFluid* f) {
+    Eddies<EDDIES_A_LAUNCH> q;
+    cudaError_t e = cudaSuccess;
+    for (int left = START_EDDIES; left >= 0 && e == cudaSuccess; left -= EDDIES_A_LAUNCH) {
+        q.count = 0;
+        drawEddies(f, q, atMost(left, EDDIES_A_LAUNCH), 0);
+        if (left < EDDIES_A_LAUNCH) drawEddies(f, q, 2, EDDIES_A_STEP - 2);
+        e = follow(f, stir, FH, RING_THREADS, f->dens[f->cur], f->radial[f->cur], f->orbital[f->cur], f->rings, q);
+    }
+    if (e != cudaSuccess) return artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
+    return ARTF_CUDA_OK;
+}
+
+/* `steps` steps, one at least (fluid.c:231-241), and the field after them.  Between calls the fields stand
+ * stirred for the step to come: each step's launch ends with the next one's eddies, which reach nothing that
+ * shows. */
+int advanceSteps(ArtfCudaFluid* f, int64_t steps) {
     Eddies<EDDIES_A_STEP> q;
     cudaError_t e = cudaSuccess;
-    for (int left = extra; left > 0 && e == cudaSuccess; left -= EDDIES_A_LAUNCH) {
-        drawEddies(f, first, atMost(left, EDDIES_A_LAUNCH), 0);
-        e = follow(f, stir, FH, RING_THREADS, f->dens[f->cur], f->radial[0], f->orbital[0], f->rings, first);
-    }
-    if (e == cudaSuccess) {
-        drawEddies(f, first, 2, EDDIES_A_STEP - 2);
-        e = follow(f, stir, FH, RING_THREADS, f->dens[f->cur], f->radial[0], f->orbital[0], f->rings, first);
-    }
     for (int64_t k = 0; k < steps && e == cudaSuccess; ++k) {
-        const bool last = k == steps - 1;
-        if (last) q.count = 0;
-        else drawEddies(f, q, 2, EDDIES_A_STEP - 2);
-        float *old = f->dens[f->cur], *next = f->dens[f->cur ^ 1];
-        e = follow(f, velocities, FIELD / 256, 256, old, f->radial[0], f->orbital[0], f->radial[1], f->orbital[1],
-                   f->rings);
-        if (e == cudaSuccess)
-            e = follow(f, ringStep, FH, RING_THREADS, old, f->radial[1], f->orbital[1], next, f->radial[0], f->orbital[0],
-                       f->rings, last ? f->field : (float*)nullptr, q);
-        f->cur ^= 1;
+        const int from = f->cur, to = f->cur ^ 1;
+        q.count = 0;
+        drawEddies(f, q, 2, EDDIES_A_STEP - 2);
+        e = follow(f, gasStep, FH, RING_THREADS + 32, f->dens[from], f->radial[from], f->orbital[from], f->dens[to],
+                   f->radial[to], f->orbital[to], f->rings, k == steps - 1 ? f->field : (float*)nullptr, q);
+        f->cur = to;
     }
     if (e != cudaSuccess) return artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
     return ARTF_CUDA_OK;
@@ -494,8 +530,8 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream); /* (the rings' staging is on this frame) */
-    int status = e == cudaSuccess ? advanceSteps(f, START_EDDIES, WARM_STEPS)
-                                  : artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
+    int status = e == cudaSuccess ? stirStart(f) : artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
+    if (!status) status = advanceSteps(f, WARM_STEPS);
     if (status) {
         artfCudaFluidFree(f);
         return status;
@@ -514,7 +550,7 @@ extern "C" int artfCudaFluidAdvance(ArtfCudaFluid* f, double time, int* stepped)
     double clock = f->time;
     const int steps = artfCudaFluidClock(&clock, time);
     if (steps > 0)
-        if (int s = advanceSteps(f, 0, steps)) return s;
+        if (int s = advanceSteps(f, steps)) return s;
     f->time = clock;
     if (stepped) *stepped = steps > 0;
     return ARTF_CUDA_OK;
@@ -526,7 +562,7 @@ extern "C" int artfCudaFluidStep(ArtfCudaFluid* f, int64_t steps, double time) {
     cudaStream_t stream = nullptr;
     if (int s = artf::contextStream(f->ctx, &stream)) return s;
     if (steps > 0)
-        if (int s = advanceSteps(f, 0, steps)) return s;
+        if (int s = advanceSteps(f, steps)) return s;
     f->time = time;
     return ARTF_CUDA_OK;
 }
