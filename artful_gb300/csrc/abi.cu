@@ -13,6 +13,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <unistd.h>
 
 static thread_local char lastError[256];
 
@@ -35,6 +36,7 @@ extern "C" const char* artfCudaLastError(void) { return lastError; }
 struct ArtfCuda {
     int device;
     int smCount;
+    bool hostPages; /* the device addresses any host memory, through the host's page tables */
     cudaStream_t stream;
     cudaEvent_t start, stop;
     float* map;
@@ -146,6 +148,7 @@ extern "C" int artfCudaCreate(int device, ArtfCuda** out) {
     if (!ctx) return fail(ARTF_CUDA_ENOMEM, "host allocation");
     ctx->device = device;
     ctx->smCount = prop.multiProcessorCount;
+    ctx->hostPages = prop.pageableMemoryAccess && prop.pageableMemoryAccessUsesHostPageTables;
     ctx->launchesLeft = -1;
     ctx->allocsLeft = -1;
     int status = ARTF_CUDA_OK;
@@ -567,6 +570,15 @@ extern "C" int artfCudaHoleTrace(ArtfCuda* ctx, const ArtfCudaHoleFrame* frame, 
     return runTrace(ctx, l, options->precision, options->bandRays, stats);
 }
 
+/* Every page of a host buffer written by the host first, so that none is new to its page tables when the
+ * device writes there. */
+static void touchPages(void* buffer, size_t bytes) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* p = (volatile char*)buffer;
+    for (size_t at = 0; at < bytes; at += page) p[at] = p[at];
+    p[bytes - 1] = p[bytes - 1];
+}
+
 extern "C" int artfCudaHoleRender(ArtfCuda* ctx, const ArtfCudaHoleFrame* frame, const ArtfCudaHoleFrame64* frame64,
                                   const float* hostMap, uint64_t mapVersion, const float* hostFluid,
                                   uint64_t fluidVersion, const ArtfCudaTraceOptions* options, float* hostHdr,
@@ -579,13 +591,23 @@ extern "C" int artfCudaHoleRender(ArtfCuda* ctx, const ArtfCudaHoleFrame* frame,
     ctx->drawnPixels = 0; /* (the light buffer is this path's from here on) */
     if ((status = hostInputs(ctx, hostMap, mapVersion, hostFluid, fluidVersion))) return status;
     const size_t pixels = (size_t)frame->size[0] * frame->size[1];
-    /* A page-locked host buffer, which the device addresses, takes the frame straight from the trace's
-     * kernels, over the link as they write it; any other buffer gets a copy of the device's frame. */
+    /* A host buffer that the device addresses takes the frame straight from the trace's kernels, over the
+     * link as they write it: a page-locked one, or, where the device goes through the host's page tables
+     * (Grace), any one whose pixels are aligned as the kernels store them (1080p, a ray a pixel: 678 us with a
+     * copy after the trace, 500 so, the trace alone 462).  Any other buffer gets a copy of the device's
+     * frame. */
     cudaPointerAttributes where;
-    if (cudaPointerGetAttributes(&where, hostHdr) == cudaSuccess && where.type == cudaMemoryTypeHost &&
-        where.devicePointer) {
-        if ((status = artfCudaHoleTrace(ctx, frame, frame64, nullptr, nullptr, options, (float*)where.devicePointer,
-                                        nullptr, stats)))
+    float* direct = nullptr;
+    if (cudaPointerGetAttributes(&where, hostHdr) == cudaSuccess) {
+        if (where.type == cudaMemoryTypeHost) {
+            direct = (float*)where.devicePointer;
+        } else if (where.type == cudaMemoryTypeUnregistered && ctx->hostPages && (uintptr_t)hostHdr % sizeof(float4) == 0) {
+            touchPages(hostHdr, sizeof(float4) * pixels);
+            direct = hostHdr;
+        }
+    }
+    if (direct) {
+        if ((status = artfCudaHoleTrace(ctx, frame, frame64, nullptr, nullptr, options, direct, nullptr, stats)))
             return status;
         CUDA_OR(ARTF_CUDA_ELAUNCH, cudaStreamSynchronize(ctx->stream));
         return ARTF_CUDA_OK;

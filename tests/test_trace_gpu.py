@@ -7,6 +7,8 @@
 """
 import hashlib
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -302,3 +304,22 @@ def test_small_frames_are_their_rays(lib, ctx, precision, width, height):
         np.testing.assert_allclose(images[0][..., :3].reshape(-1, 3), rgb, rtol=2e-7, atol=1e-12)
     else:
         assert np.array_equal(images[0][..., :3].reshape(-1, 3), rgb)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 4])
+@pytest.mark.parametrize("jitter", [0, 3])
+def test_host_path_at_any_alignment(lib, ctx, offset, jitter):
+    """Into plain host memory, aligned as the kernels store pixels or not, new or written before: the device
+    path's bits, and nothing beside the frame written."""
+    scene, frame, frame64, m, fluid = _scene_inputs(lib, "odd_101x67")
+    opts = capi.TraceOptions(capi.MIXED, jitter, 9, 1.0, 0.0, 0, 0, 1)
+    floats = scene.width * scene.height * 4
+    raw = np.empty(floats + 64, np.float32)
+    base = offset + (-(raw.ctypes.data // 4) % 4) + 8
+    raw[:base], raw[base + floats:] = 7.0, 7.0
+    capi.check(lib.artfCudaHoleRender(ctx, C.byref(frame), C.byref(frame64), m.ctypes.data, 0, fluid.ctypes.data, 0,
+                                      C.byref(opts), raw.ctypes.data + 4 * base, None))
+    g.set_inputs(lib, ctx, m, fluid)
+    hdr, _ = g.trace(lib, ctx, frame, frame64, capi.MIXED, jitter=jitter, seed=9, persistent=1)
+    assert np.array_equal(raw[base:base + floats].view(np.uint32), hdr.ravel().view(np.uint32))
+    assert np.all(raw[:base] == 7.0) and np.all(raw[base + floats:] == 7.0)
