@@ -114,37 +114,40 @@ __device__ __forceinline__ unsigned traceRay(const KernelParams<R>& p, R nx, R n
         StepOut<R> o;
         nystromStep(a, c, s, o);
         ++i;
-        Crossing<R> x;
-        bool opaque = false;
-        if (crossingOf(f, rhoScale, c, s, o, x)) {
-            ++crossings;
-            R turn;
-            const R light = shadeCrossing(f, rhoScale, p.map, p.fluid, c, x, through, raySum, &turn);
-            if (light > R(0) && !(kind & ARTF_CUDA_END_LIT)) {
-                kind |= ARTF_CUDA_END_LIT;
-                if (end) end->hitR = (float)recipR(x.uc), end->hitPhi = (float)(turn - floorR(turn));
+        /* (most steps meet nothing, which one branch decides) */
+        if ((s.n[2] * o.next.n[2] < R(0)) | (R(0) > o.next.u) | (o.next.u > f.uHorizon)) {
+            Crossing<R> x;
+            bool opaque = false;
+            if (crossingOf(f, rhoScale, c, s, o, x)) {
+                ++crossings;
+                R turn;
+                const R light = shadeCrossing(f, rhoScale, p.map, p.fluid, c, x, through, raySum, &turn);
+                if (light > R(0) && !(kind & ARTF_CUDA_END_LIT)) {
+                    kind |= ARTF_CUDA_END_LIT;
+                    if (end) end->hitR = (float)recipR(x.uc), end->hitPhi = (float)(turn - floorR(turn));
+                }
+                opaque = !(through > KF(.004)); /* (the transmission only changes here) */
             }
-            opaque = !(through > KF(.004)); /* (the transmission only changes here) */
-        }
-        if (R(0) > o.next.u) {
-            const R part = divR(s.u, s.u - o.next.u);
-            R away[3], dir[3];
-            for (int k = 0; k < 3; ++k) away[k] = s.n[k] + part * (o.next.n[k] - s.n[k]);
-            const R awayPsi = s.psi + part * (o.next.psi - s.psi);
-            skyDirection(away, awayPsi, dir);
-            if (f.stars > R(0)) shadeSky(f, p.map, c, dir, through, raySum);
-            kind ^= ARTF_CUDA_END_CAP ^ ARTF_CUDA_END_SKY;
-            if (end) {
-                for (int k = 0; k < 3; ++k) end->dir[k] = (float)dir[k];
-                end->mino = (float)((R(i - 1) + part) * c.step);
+            if (R(0) > o.next.u) {
+                const R part = divR(s.u, s.u - o.next.u);
+                R away[3], dir[3];
+                for (int k = 0; k < 3; ++k) away[k] = s.n[k] + part * (o.next.n[k] - s.n[k]);
+                const R awayPsi = s.psi + part * (o.next.psi - s.psi);
+                skyDirection(away, awayPsi, dir);
+                if (f.stars > R(0)) shadeSky(f, p.map, c, dir, through, raySum);
+                kind ^= ARTF_CUDA_END_CAP ^ ARTF_CUDA_END_SKY;
+                if (end) {
+                    for (int k = 0; k < 3; ++k) end->dir[k] = (float)dir[k];
+                    end->mino = (float)((R(i - 1) + part) * c.step);
+                }
+                break;
             }
-            break;
-        }
-        const bool fell = o.next.u > f.uHorizon;
-        if (fell || opaque) {
-            kind ^= ARTF_CUDA_END_CAP ^ (fell ? ARTF_CUDA_END_HORIZON : ARTF_CUDA_END_OPAQUE);
-            if (end) end->mino = (float)(R(i) * c.step);
-            break;
+            const bool fell = o.next.u > f.uHorizon;
+            if (fell || opaque) {
+                kind ^= ARTF_CUDA_END_CAP ^ (fell ? ARTF_CUDA_END_HORIZON : ARTF_CUDA_END_OPAQUE);
+                if (end) end->mino = (float)(R(i) * c.step);
+                break;
+            }
         }
         s = o.next;
     }

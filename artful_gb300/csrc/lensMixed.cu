@@ -320,12 +320,10 @@ __device__ __forceinline__ void mixedStart(const MixedParams& p, uint32_t guards
  * whole sub-step in FP64 (the frame-drag rate's Delta / r^2 cancels there, and it divides).  At a turning
  * point, of u or of n_z, that coordinate's motion in double-float: psi and its rate, and the components
  * about the axis, smooth there, stay the FP32 step's.  A step that turns both runs the motion twice. */
-__device__ __forceinline__ void mixedGuards(uint32_t guards, const MixedView& v, MixedRay& r, StepOut<float>& o,
-                                            unsigned& rounds) {
-    const bool band = (guards & ARTF_CUDA_GUARD_HORIZON) && r.s.u > v.uGuard;
-    bool turnR = (guards & ARTF_CUDA_GUARD_RADIAL) && ((r.s.w > 0.f) != (o.next.w > 0.f)) && !band;
-    bool turnP = (guards & ARTF_CUDA_GUARD_POLAR) && ((r.s.v[2] > 0.f) != (o.next.v[2] > 0.f));
+__device__ __forceinline__ void mixedGuards(const MixedView& v, MixedRay& r, bool band, bool turnR, bool turnP,
+                                            StepOut<float>& o, unsigned& rounds) {
     if (!(band || turnR || turnP)) return;
+    turnR = turnR && !band;
     r.wide += 1u | (band ? 0x10000u : 0u);
     r.turns += (turnR ? 1u : 0u) | (turnP ? 0x10000u : 0u);
     const unsigned first = (threadIdx.x & 31) == __ffs((int)__activemask()) - 1;
@@ -359,12 +357,11 @@ __device__ __forceinline__ void mixedGuards(uint32_t guards, const MixedView& v,
     }
 }
 
-/* After a step: the disc crossing, escape, horizon, opacity and the step cap.  Returns the end's kind
+/* What a step meets: the disc crossing, escape, horizon and opacity.  Returns the end's kind
  * (ARTF_CUDA_END_*) + 1, or 0 when the ray goes on. */
-__device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t guards, const MixedView& v,
-                                                 MixedRay& r, const StepOut<float>& o, ArtfCudaRayEnd* end) {
+__device__ __forceinline__ unsigned mixedMeets(bool compensated, const MixedView& v, MixedRay& r,
+                                               const StepOut<float>& o, ArtfCudaRayEnd* end) {
     const Frame<float>& f = v.f;
-    const bool compensated = guards & ARTF_CUDA_GUARD_PSI;
     const float increment = o.next.psi;
     Crossing<float> x;
     bool opaque = false;
@@ -380,7 +377,6 @@ __device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t 
         /* (the transmission only changes here) */
         opaque = !(r.through > .004f);
     }
-    ++r.i;
     if (0.f > o.next.u) {
         const float part = divR(r.s.u, r.s.u - o.next.u);
         float away[3], dir[3];
@@ -395,16 +391,7 @@ __device__ __forceinline__ unsigned mixedAdvance(const MixedParams& p, uint32_t 
     }
     if (o.next.u > f.uHorizon) return ARTF_CUDA_END_HORIZON + 1;
     if (opaque) return ARTF_CUDA_END_OPAQUE + 1;
-    if (compensated) {
-        const float sumHi = r.psiHi + increment, back = sumHi - r.psiHi;
-        r.psiLo += (r.psiHi - (sumHi - back)) + (increment - back);
-        r.psiHi = sumHi;
-    } else {
-        r.psiHi += increment;
-    }
-    r.s = o.next;
-    r.s.psi = 0.f;
-    return r.i >= p.maxSteps ? ARTF_CUDA_END_CAP + 1 : 0u;
+    return 0;
 }
 
 /* What a thread counts over its rays, in shared memory: touched once a ray, it would hold ten registers
@@ -444,12 +431,35 @@ __device__ __forceinline__ unsigned traceRayMixed(const MixedParams& p, const Mi
     MixedRay r;
     mixedStart(p, guards, v, nx, ny, time, r);
     if (end) end->hitR = end->hitPhi = NAN;
-    unsigned ended = 0;
-    while (!ended) {
+    const bool compensated = guards & ARTF_CUDA_GUARD_PSI;
+    unsigned ended = ARTF_CUDA_END_CAP + 1;
+    for (;;) {
         StepOut<float> o;
         nystromStep(v.f.a, r.c, r.s, o);
-        mixedGuards(guards, v, r, o, rounds);
-        ended = mixedAdvance(p, guards, v, r, o, end);
+        ++r.i;
+        /* Most steps need no guard and meet nothing, which one branch decides (all its tests made: 1464 us with
+         * a branch for each, 1372 with the tests in turn, 1331 so, at 1080p x 4). */
+        const bool band = (guards & ARTF_CUDA_GUARD_HORIZON) && r.s.u > v.uGuard;
+        const bool turnR = (guards & ARTF_CUDA_GUARD_RADIAL) && ((r.s.w > 0.f) != (o.next.w > 0.f));
+        const bool turnP = (guards & ARTF_CUDA_GUARD_POLAR) && ((r.s.v[2] > 0.f) != (o.next.v[2] > 0.f));
+        if (band | turnR | turnP | (r.s.n[2] * o.next.n[2] < 0.f) | (0.f > o.next.u) | (o.next.u > v.f.uHorizon)) {
+            mixedGuards(v, r, band, turnR, turnP, o, rounds);
+            if (const unsigned met = mixedMeets(compensated, v, r, o, end)) {
+                ended = met;
+                break;
+            }
+        }
+        const float increment = o.next.psi;
+        if (compensated) {
+            const float sumHi = r.psiHi + increment, back = sumHi - r.psiHi;
+            r.psiLo += (r.psiHi - (sumHi - back)) + (increment - back);
+            r.psiHi = sumHi;
+        } else {
+            r.psiHi += increment;
+        }
+        r.s = o.next;
+        r.s.psi = 0.f;
+        if (r.i >= p.maxSteps) break;
     }
     for (int k = 0; k < 3; ++k) sum[k] = sum[k] + r.sum[k];
     return mixedFinish(r, ended, end, tally);
