@@ -12,7 +12,7 @@
  * of each segment of K steps in a trail in device memory (field by field across rays), and leaves the
  * ray's loss adjoint and end there.  The reverse one walks each ray back from its last step that added
  * radiance, a segment at a time, each segment recomputed from its checkpoint into a ring of K kept
- * states in the thread's local memory; or, with K = 1 (every state kept, 48 bytes a step), a warp's rays
+ * states in the thread's local memory; or, with K = 1 (every state kept, 32 bytes written a step), a warp's rays
  * together from the warp's highest step, their states read back through shared memory with nothing
  * recomputed.  At each step, in reverse order, it
  * applies the transposed derivatives of the sky (at the escape), of the disc crossing (its three slices,
@@ -85,33 +85,6 @@ __device__ __forceinline__ void dragBack(float a, float xiA, float x, float dBar
     g.xiA += numBar * a * x * x;
 }
 
-/* The drag rate at x with the pieces its adjoint takes: the numerator, the reciprocal of the denominator
- * and whether the denominator was held at its floor.  One reciprocal serves the rate and its adjoint
- * (four reciprocals a step fewer than dragAt and dragBack apart: 1.314 -> 1.293 ms for 8 views). */
-struct DragTerms {
-    float rate, num, inv;
-    bool held;
-};
-
-__device__ __forceinline__ DragTerms dragTerms(float a, float a2, float xiA, float x) {
-    DragTerms d;
-    d.num = -a * x * (2.f - xiA * x);
-    const float raw = 1.f - (x + x) + a2 * x * x;
-    d.held = !(raw > 1e-3f);
-    d.inv = 1.f / (d.held ? 1e-3f : raw);
-    d.rate = d.num * d.inv;
-    return d;
-}
-
-/* dragBack with the rate's pieces already at hand. */
-__device__ __forceinline__ void dragBackWith(float a, float xiA, float x, const DragTerms& d, float dBar, float& xBar,
-                                             ConstBar& g) {
-    const float numBar = dBar * d.inv, denBar = d.held ? 0.f : -numBar * d.rate;
-    xBar += numBar * (-a * (2.f - 2.f * xiA * x)) + denBar * (2.f * a * a * x - 2.f);
-    g.a += numBar * (-x * (2.f - xiA * x)) + denBar * 2.f * a * x * x;
-    g.xiA += numBar * a * x * x;
-}
-
 /* lens.inc:30-41's polynomial arctangent (in turns): its slopes in y and x. */
 __device__ __forceinline__ void turnsSlope(float y, float x, float& dy, float& dx) {
     const float ax = fabsf(x), ay = fabsf(y);
@@ -160,126 +133,152 @@ __device__ __forceinline__ void speedSlopes(const Frame<float>& f, int32_t row, 
 
 /* ---- the Nystrom step taken back (lens.inc:165-192) ------------------------------------------------ */
 
-/* What every step of a ray taken back takes from the ray alone, formed once a ray: the step's products
- * (as stepTerms forms them) and the spin's. */
-struct BackTerms {
-    float h, half, eighth, halfSq, sixthSq, sixth, a, a2, twoA2, fourA2, fourA, twoA;
-};
-
-__device__ __forceinline__ BackTerms backTerms(float a, float step) {
-    BackTerms t;
-    const StepTerms<float> st = stepTerms(step);
-    t.h = step, t.half = st.half, t.eighth = st.eighth, t.halfSq = st.halfSquare, t.sixthSq = st.sixthSquare;
-    t.sixth = st.sixth;
-    t.a = a, t.a2 = a * a, t.twoA2 = 2.f * t.a2, t.fourA2 = 4.f * t.a2, t.fourA = 4.f * a, t.twoA = 2.f * a;
-    return t;
-}
-
-/* A(x) = (-c x0, -c x1, a^2 x2 - c x2), c = K + 2 a^2 x2^2 as the forward step forms it; returns c. */
-__device__ __forceinline__ float accelWith(const BackTerms& t, float big, const float* x, float* out) {
-    const float cc = big + t.twoA2 * (x[2] * x[2]);
-    out[0] = 0.f - cc * x[0], out[1] = 0.f - cc * x[1], out[2] = t.a2 * x[2] - cc * x[2];
-    return cc;
-}
-
-/* A(x) taken back from its adjoint y, with its c. */
-__device__ __forceinline__ void accelBackWith(const BackTerms& t, float cc, const float* x, const float* y, float* xBar,
-                                              ConstBar& g) {
-    const float cBar = -(x[0] * y[0] + x[1] * y[1] + x[2] * y[2]);
-    xBar[0] += -cc * y[0];
-    xBar[1] += -cc * y[1];
-    xBar[2] += (t.a2 - cc) * y[2] + cBar * t.fourA2 * x[2];
-    g.a += x[2] * (t.twoA * y[2] + cBar * t.fourA * x[2]);
-    g.big += cBar;
-}
-
-/* The polar part: from the adjoints of (n', v') and of the first stage's a1 (which a crossing reads), adds
- * to those of (n, v) and the constants. */
-__device__ __forceinline__ void polarBack(const BackTerms& t, float big, const float* n, const float* v,
-                                          const float* nNextBar, const float* vNextBar, const float* a1Extra,
-                                          bool extra, float* nBar, float* vBar, ConstBar& g, ConstBar& gs) {
-    const float h = t.h, half = t.half, eighth = t.eighth, halfSq = t.halfSq, sixthSq = t.sixthSq, sixth = t.sixth;
-    float a1[3], midN[3], a2s[3], endN[3], a3[3];
-    const float c1 = accelWith(t, big, n, a1);
-    for (int k = 0; k < 3; ++k) midN[k] = n[k] + half * v[k] + eighth * a1[k];
-    const float c2 = accelWith(t, big, midN, a2s);
-    for (int k = 0; k < 3; ++k) endN[k] = n[k] + h * v[k] + halfSq * a2s[k];
-    const float c3 = accelWith(t, big, endN, a3);
-    (void)a3;
-    float a1Bar[3], a2Bar[3], a3Bar[3], midBar[3] = {0.f, 0.f, 0.f}, endBar[3] = {0.f, 0.f, 0.f};
-    for (int k = 0; k < 3; ++k) {
-        /* n' = n + h v + h^2/6 (a1 + 2 a2);  v' = v + h/6 (a1 + a3 + 4 a2) */
-        nBar[k] += nNextBar[k];
-        vBar[k] += h * nNextBar[k] + vNextBar[k];
-        a1Bar[k] = sixthSq * nNextBar[k] + sixth * vNextBar[k];
-        a2Bar[k] = 2.f * sixthSq * nNextBar[k] + 4.f * sixth * vNextBar[k];
-        a3Bar[k] = sixth * vNextBar[k];
-    }
-    accelBackWith(t, c3, endN, a3Bar, endBar, gs);
-    for (int k = 0; k < 3; ++k) { /* endN = n + h v + h^2/2 a2 */
-        nBar[k] += endBar[k];
-        vBar[k] += h * endBar[k];
-        a2Bar[k] += halfSq * endBar[k];
-    }
-    accelBackWith(t, c2, midN, a2Bar, midBar, gs);
-    for (int k = 0; k < 3; ++k) { /* midN = n + h/2 v + h^2/8 a1 */
-        nBar[k] += midBar[k];
-        vBar[k] += half * midBar[k];
-        a1Bar[k] += eighth * midBar[k];
-    }
-    accelBackWith(t, c1, n, a1Bar, nBar, gs);
-    if (extra) accelBackWith(t, c1, n, a1Extra, nBar, g); /* (what a crossing read of a1: not the step's) */
-}
-
-/* The radial part: from the adjoints of (u', w', psi', drag') and of k1, adds to those of (u, w, psi,
- * drag) and the constants. */
-__device__ __forceinline__ void radialBack(const BackTerms& t, const RayConst<float>& c, float u, float w, float drag,
-                                           float uNextBar, float wNextBar, float psiNextBar, float dragNextBar,
-                                           float k1Extra, bool extra, float& uBar, float& wBar, float& psiBar,
-                                           float& dragBar, ConstBar& g, ConstBar& gs) {
-    const float h = t.h, half = t.half, eighth = t.eighth, halfSq = t.halfSq, sixthSq = t.sixthSq, sixth = t.sixth;
-    const float k1 = bendAt(c, u);
-    const float midU = u + half * w + eighth * k1;
-    const float k2 = bendAt(c, midU);
-    const float endU = u + h * w + halfSq * k2;
-    float midBar = 0.f;
-    if (t.a != 0.f) {
-        /* drag' = drag(u');  psi' = psi + h/6 (drag + drag' + 4 drag(midU)): the step length's explicit
-         * share here; its share through u' and midU is the motion's, taken over the whole ray */
-        const float uNext = u + h * w + sixthSq * (k1 + (k2 + k2));
-        const DragTerms dNext = dragTerms(t.a, t.a2, c.xiA, uNext), dMid = dragTerms(t.a, t.a2, c.xiA, midU);
-        const float s6 = psiNextBar * sixth;
-        psiBar += psiNextBar;
-        dragBar += s6;
-        g.step += psiNextBar * (drag + dNext.rate + 4.f * dMid.rate) * (1.f / 6.f);
-        dragBackWith(t.a, c.xiA, midU, dMid, 4.f * s6, midBar, g);
-        dragBackWith(t.a, c.xiA, uNext, dNext, dragNextBar + s6, uNextBar, g);
-    }
-    /* u' = u + h w + h^2/6 (k1 + 2 k2);  w' = w + h/6 (k1 + k3 + 4 k2) */
-    uBar += uNextBar;
-    wBar += h * uNextBar + wNextBar;
-    float k1Bar = sixthSq * uNextBar + sixth * wNextBar;
-    float k2Bar = 2.f * sixthSq * uNextBar + 4.f * sixth * wNextBar;
-    const float k3Bar = sixth * wNextBar;
-    float endBar = 0.f; /* endU = u + h w + h^2/2 k2 */
-    bendBack(c, endU, k3Bar, endBar, gs);
-    uBar += endBar;
-    wBar += h * endBar;
-    k2Bar += halfSq * endBar;
-    bendBack(c, midU, k2Bar, midBar, gs); /* midU = u + h/2 w + h^2/8 k1 */
-    uBar += midBar;
-    wBar += half * midBar;
-    k1Bar += eighth * midBar;
-    bendBack(c, u, k1Bar, uBar, gs);
-    if (extra) bendBack(c, u, k1Extra, uBar, g); /* (what a crossing read of k1: not the step's) */
-}
-
 /* The adjoints of one step's start state and of what the crossing and the sky read of its end. */
 struct StepBar {
     float u, w, n[3], v[3], psi, drag;
     float k1, a1[3];
     float nextU, nextN[3], nextPsi, nextDrag;
 };
+
+/* What the steps of a ray give the adjoints of its constants, in sums that the ray's end scales: of the
+ * coefficients that the step length scales (uA, uB, uC, K, and a through the axis), and of the drag rate's
+ * two evaluations a step, side by side. */
+struct StepSums {
+    float uA, uB, uC, big, axis;
+    F2 one, two, den; /* of numBar x, numBar x^2 and denBar x^2 */
+};
+
+/* A stage's acceleration of u and n_z, x (..) each, taken back from its adjoint y at (x.u, x.z): onto x, and
+ * into the sums.  dot: -(n . y), the adjoint of the stage's c = K + 2 a^2 n_z^2. */
+__device__ __forceinline__ F2 stageBack(const RayConst<float>& c, float a2, float fourA2, float stageC, float dot, F2 x,
+                                        F2 y, StepSums& sums) {
+    float u, z, yu, yz;
+    unpack(x, u, z);
+    unpack(y, yu, yz);
+    const float t = yu * u, t2 = t * u, m = dot * z;
+    sums.uA += t;
+    sums.uB += t2;
+    sums.uC = fmaf(t2, u, sums.uC);
+    sums.big += dot;
+    sums.axis = fmaf(z, fmaf(2.f, m, yz), sums.axis);
+    return pack(yu * fmaf(u, fmaf(3.f * c.uC, u, 2.f * c.uB), c.uA), fmaf(fourA2, m, (a2 - stageC) * yz));
+}
+
+/* -(n . y) over the three components. */
+__device__ __forceinline__ float minusDot(F2 n, F2 y, float z, float yz) {
+    float p0, p1;
+    unpack(mul2(n, y), p0, p1);
+    return -fmaf(z, yz, p0 + p1);
+}
+
+/* The drag rate at x, num / den with num = -a x (2 - xiA x) and den = max(1 - 2x + a^2 x^2, 1e-3): the rate,
+ * 1 / den, and whether den stands above its floor. */
+struct DragTerms {
+    float rate, inv;
+    bool free;
+};
+
+__device__ __forceinline__ DragTerms dragTerms(float a, float xiA, float x) {
+    const float raw = fmaf(x, fmaf(a * a, x, -2.f), 1.f), inv = recipR(fmaxf(raw, 1e-3f));
+    return DragTerms{x * fmaf(a * xiA, x, -2.f * a) * inv, inv, raw > 1e-3f};
+}
+
+/* One step taken back: from the state it started from, the u it ended at and the drag rate there (`drag`,
+ * left as that at the start), and the adjoints of its end, to those of its start, added to `to` (which holds
+ * what the step's events gave them).  As the step itself it runs in pairs, (n_x, n_y) and (u, n_z) and the two
+ * drag rates, and each step evaluates the drag rate at its start and middle, the end's being the start's of
+ * the step before it (32 fits of 256 x 144: the reverse kernel 697 -> 649 us). */
+__device__ __forceinline__ void stepBack(float a, const RayConst<float>& c, const RayState<float>& s, float nextU,
+                                         DragTerms& drag, const StepBar& from, StepBar& to, ConstBar& g, StepSums& sums) {
+    const StepTerms<float> t = stepTerms(c.step);
+    const float a2 = a * a, twoA2 = 2.f * a2, fourA2 = 4.f * a2;
+    const F2 h = both(c.step), half = both(t.half), eighth = both(t.eighth), halfSq = both(t.halfSquare);
+    const F2 sixthSq = both(t.sixthSquare), sixth = both(t.sixth);
+    /* the stages again */
+    const F2 n = pack(s.n[0], s.n[1]), v = pack(s.v[0], s.v[1]), q = pack(s.u, s.n[2]), w = pack(s.w, s.v[2]);
+    const float c1 = fmaf(twoA2, s.n[2] * s.n[2], c.big);
+    const F2 midN = fma2(mul2(eighth, both(-c1)), n, fma2(half, v, n));
+    const F2 midQ = fma2(eighth, pack(s.u * bendPoly(c, s.u), axisAccel(a2, c1, s.n[2])), fma2(half, w, q));
+    float midU, midZ;
+    unpack(midQ, midU, midZ);
+    const float c2 = fmaf(twoA2, midZ * midZ, c.big);
+    const F2 endN = fma2(mul2(halfSq, both(-c2)), midN, fma2(h, v, n));
+    const F2 endQ = fma2(halfSq, pack(midU * bendPoly(c, midU), axisAccel(a2, c2, midZ)), fma2(h, w, q));
+    float endU, endZ;
+    unpack(endQ, endU, endZ);
+    const float c3 = fmaf(twoA2, endZ * endZ, c.big);
+    (void)endU;
+    float uNextBar = from.nextU, midBarU = 0.f;
+    if (a != 0.f) {
+        /* drag' = drag(u');  psi' = psi + h/6 (drag + drag' + 4 drag(mid u)); the step length's explicit share
+         * here, its share through u' and mid u with the motion's, taken over the whole ray */
+        const DragTerms mid = dragTerms(a, c.xiA, midU), start = dragTerms(a, c.xiA, s.u);
+        const F2 x = pack(midU, nextU);
+        const float s6 = from.nextPsi * t.sixth;
+        to.psi += from.nextPsi;
+        to.drag += s6;
+        g.step = fmaf(from.nextPsi * (1.f / 6.f), start.rate + drag.rate + 4.f * mid.rate, g.step);
+        const F2 numBar = mul2(pack(4.f * s6, from.nextDrag + s6), pack(mid.inv, drag.inv));
+        float d0, d1;
+        unpack(mul2(numBar, pack(mid.rate, drag.rate)), d0, d1);
+        const F2 denBar = pack(mid.free ? -d0 : 0.f, drag.free ? -d1 : 0.f);
+        const F2 one = mul2(numBar, x);
+        sums.one = fma2(numBar, x, sums.one);
+        sums.two = fma2(one, x, sums.two);
+        sums.den = fma2(mul2(denBar, x), x, sums.den);
+        const F2 xBar = fma2(denBar, fma2(both(2.f * a2), x, both(-2.f)),
+                             mul2(numBar, fma2(both(2.f * a * c.xiA), x, both(-2.f * a))));
+        float x1;
+        unpack(xBar, midBarU, x1);
+        uNextBar += x1;
+        drag = start;
+    }
+    /* x' = x + h v + h^2/6 (a1 + 2 a2);  v' = v + h/6 (a1 + a3 + 4 a2) */
+    const F2 barN = pack(from.nextN[0], from.nextN[1]), barV = pack(from.v[0], from.v[1]);
+    const F2 barQ = pack(uNextBar, from.nextN[2]), barW = pack(from.w, from.v[2]);
+    const F2 three = mul2(sixth, barV), threeQ = mul2(sixth, barW); /* a3's adjoint */
+    F2 oneN = fma2(sixthSq, barN, three), oneQ = fma2(sixthSq, barQ, threeQ);
+    F2 twoN = fma2(mul2(sixthSq, both(2.f)), barN, mul2(three, both(4.f)));
+    F2 twoQ = fma2(mul2(sixthSq, both(2.f)), barQ, mul2(threeQ, both(4.f)));
+    F2 toN = add2(pack(to.n[0], to.n[1]), barN), toQ = add2(pack(to.u, to.n[2]), barQ);
+    F2 toV = fma2(h, barN, add2(pack(to.v[0], to.v[1]), barV)), toW = fma2(h, barQ, add2(pack(to.w, to.v[2]), barW));
+    float yu, yz;
+    /* the end: x + h v + h^2/2 a2 */
+    unpack(threeQ, yu, yz);
+    const F2 endBarN = mul2(both(-c3), three);
+    const F2 endBarQ = stageBack(c, a2, fourA2, c3, minusDot(endN, three, endZ, yz), endQ, threeQ, sums);
+    toN = fma2(both(-c3), three, toN), toQ = add2(toQ, endBarQ);
+    toV = fma2(h, endBarN, toV), toW = fma2(h, endBarQ, toW);
+    twoN = fma2(halfSq, endBarN, twoN), twoQ = fma2(halfSq, endBarQ, twoQ);
+    /* the middle: x + h/2 v + h^2/8 a1 */
+    unpack(twoQ, yu, yz);
+    const F2 midBarN = mul2(both(-c2), twoN);
+    const F2 midBarQ = add2(stageBack(c, a2, fourA2, c2, minusDot(midN, twoN, midZ, yz), midQ, twoQ, sums), pack(midBarU, 0.f));
+    toN = fma2(both(-c2), twoN, toN), toQ = add2(toQ, midBarQ);
+    toV = fma2(half, midBarN, toV), toW = fma2(half, midBarQ, toW);
+    oneN = fma2(eighth, midBarN, oneN), oneQ = fma2(eighth, midBarQ, oneQ);
+    /* the start */
+    unpack(oneQ, yu, yz);
+    toN = fma2(both(-c1), oneN, toN);
+    toQ = add2(toQ, stageBack(c, a2, fourA2, c1, minusDot(n, oneN, s.n[2], yz), q, oneQ, sums));
+    unpack(toN, to.n[0], to.n[1]);
+    unpack(toQ, to.u, to.n[2]);
+    unpack(toV, to.v[0], to.v[1]);
+    unpack(toW, to.w, to.v[2]);
+}
+
+/* What a crossing read of the first stage (k1, a1), taken back onto the start and the constants. */
+__device__ __forceinline__ void firstStageBack(float a, const RayConst<float>& c, const RayState<float>& s, StepBar& b,
+                                               ConstBar& g) {
+    bendBack(c, s.u, b.k1, b.u, g);
+    const float cc = c.big + 2.f * a * a * (s.n[2] * s.n[2]);
+    const float cBar = -(s.n[0] * b.a1[0] + s.n[1] * b.a1[1] + s.n[2] * b.a1[2]);
+    b.n[0] += -cc * b.a1[0];
+    b.n[1] += -cc * b.a1[1];
+    b.n[2] += (a * a - cc) * b.a1[2] + cBar * (4.f * a * a) * s.n[2];
+    g.a += s.n[2] * (2.f * a * b.a1[2] + cBar * (4.f * a) * s.n[2]);
+    g.big += cBar;
+}
 
 /* ---- a disc crossing taken back (lens.inc:195-289) ------------------------------------------------- */
 
@@ -717,18 +716,16 @@ __device__ void startBack(const AdjointView& v, float nx, float ny, const RayCon
 
 /* ---- the kernels -------------------------------------------------------------------------------- */
 
-struct alignas(16) Kept {
-    RayState<float> s;
-    float through; /* the disc's transmission before this step's crossing */
-};
-
 /* Each ray's trail from the forward kernel to the reverse one, in device memory, field by field across
  * rays (a warp's 32 rays are adjacent in every field: its loads and stores coalesce):
  *   head  (steps, top, escaped, 0) as ints: steps taken, and steps 0 .. top - 1 go back
  *   bar   (dL/dR, dL/dG, dL/dB, the transmission at the end)
  *   end   the state after the last step (three float4)
  *   saved the state at the start of each segment of K steps (three float4 a segment)
- * A state is (u, w, n0, n1), (n2, v0, v1, v2), (psi, drag, through, 0). */
+ * A state is (u, w, n0, n1), (n2, v0, v1, v2), (psi, drag, through, 0).  With every state kept (K = 1) the
+ * third is written only where a step back reads it, at the steps that cross the disc's plane or end the ray,
+ * and is then what its crossing takes: (psi, the transmission before it, the next psi, 0); the drag rate
+ * follows from u. */
 struct Trail {
     int4* head;
     float4* bar;
@@ -739,17 +736,14 @@ struct Trail {
 
 /* (streaming stores: the trail, larger than L2, is marked to leave it first, so that the map the forward
  * kernel shades from stays; 0.182 -> 0.180 ms at 512x288) */
-__device__ __forceinline__ void storeState(float4* at, size_t stride, const RayState<float>& s, float through) {
+__device__ __forceinline__ void storeMotion(float4* at, size_t stride, const RayState<float>& s) {
     __stcs(at, make_float4(s.u, s.w, s.n[0], s.n[1]));
     __stcs(at + stride, make_float4(s.n[2], s.v[0], s.v[1], s.v[2]));
-    __stcs(at + 2 * stride, make_float4(s.psi, s.drag, through, 0.f));
 }
 
-__device__ __forceinline__ void loadState(const float4* at, size_t stride, RayState<float>& s, float& through) {
-    const float4 a = at[0], b = at[stride], c = at[2 * stride];
+__device__ __forceinline__ void setMotion(RayState<float>& s, float4 a, float4 b) {
     s.u = a.x, s.w = a.y, s.n[0] = a.z, s.n[1] = a.w;
     s.n[2] = b.x, s.v[0] = b.y, s.v[1] = b.z, s.v[2] = b.w;
-    s.psi = c.x, s.drag = c.y, through = c.z;
 }
 
 struct AdjointLaunch {
@@ -762,19 +756,6 @@ struct AdjointLaunch {
     Trail trail;
     int tilesX, tilesPerView, totalTiles, K;
 };
-
-/* One step from s, with its crossing's shading. */
-__device__ __forceinline__ void stepOnce(const AdjointView& v, float rhoScale, const RayConst<float>& c,
-                                         const RayState<float>& s, StepOut<float>& o, float& through, float* sum,
-                                         unsigned& crossings) {
-    nystromStep(v.f.a, c, s, o);
-    Crossing<float> x;
-    if (crossingOf(v.f, rhoScale, c, s, o, x)) {
-        float turn;
-        shadeCrossing(v.f, rhoScale, v.map, v.fluid, c, x, through, sum, &turn);
-        ++crossings;
-    }
-}
 
 /* The ray of pixel (px, py) at its centre: its image position, constants of motion and first state. */
 __device__ __forceinline__ void adjointStart(const AdjointView& v, int px, int py, float& nx, float& ny,
@@ -838,26 +819,40 @@ template <int kK> __global__ void __launch_bounds__(kThreads, 6) adjointForward(
         int steps = 0, lastCrossing = -1;
         unsigned crossings = 0;
         bool escaped = false;
-        RayState<float> end = s;
         for (int step = 0; step < kMaxSteps; ++step) {
-            if (step % K == 0) storeState(tr.saved + (size_t)(3 * (step / K)) * tr.rays + t.ray, tr.rays, s, through);
-            StepOut<float> o;
-            const unsigned crossed = crossings;
-            stepOnce(v, rhoScale, c, s, o, through, sum, crossings);
-            if (crossings != crossed) lastCrossing = step;
-            ++steps;
-            end = o.next;
-            if (0.f > o.next.u) {
-                const float part = s.u / (s.u - o.next.u);
-                float away[3], dir[3];
-                for (int k = 0; k < 3; ++k) away[k] = s.n[k] + part * (o.next.n[k] - s.n[k]);
-                skyDirection(away, s.psi + part * (o.next.psi - s.psi), dir);
-                if (f.stars > 0.f) shadeSky(f, v.map, c, dir, through, sum);
-                escaped = true;
-                break;
+            if (step % K == 0) {
+                float4* const at = tr.saved + (size_t)(3 * (step / K)) * tr.rays + t.ray;
+                storeMotion(at, tr.rays, s);
+                if (kK != 1) __stcs(at + 2 * tr.rays, make_float4(s.psi, s.drag, through, 0.f));
             }
-            if (o.next.u > f.uHorizon || !(through > .004f)) break;
+            StepOut<float> o;
+            nystromStep(f.a, c, s, o);
+            ++steps;
+            bool ended = false;
+            /* (most steps meet nothing, which one branch decides) */
+            if ((s.n[2] * o.next.n[2] < 0.f) | (0.f > o.next.u) | (o.next.u > f.uHorizon) | (step == kMaxSteps - 1)) {
+                if (kK == 1)
+                    __stcs(tr.saved + (size_t)(3 * step + 2) * tr.rays + t.ray,
+                           make_float4(s.psi, through, o.next.psi, 0.f));
+                Crossing<float> x;
+                if (crossingOf(f, rhoScale, c, s, o, x)) {
+                    float turn;
+                    shadeCrossing(f, rhoScale, v.map, v.fluid, c, x, through, sum, &turn);
+                    ++crossings;
+                    lastCrossing = step;
+                }
+                if (0.f > o.next.u) {
+                    const float part = divR(s.u, s.u - o.next.u);
+                    float away[3], dir[3];
+                    for (int k = 0; k < 3; ++k) away[k] = s.n[k] + part * (o.next.n[k] - s.n[k]);
+                    skyDirection(away, s.psi + part * (o.next.psi - s.psi), dir);
+                    if (f.stars > 0.f) shadeSky(f, v.map, c, dir, through, sum);
+                    escaped = true;
+                }
+                ended = escaped || o.next.u > f.uHorizon || !(through > .004f);
+            }
             s = o.next;
+            if (ended) break;
         }
         const float4 want = v.target[t.py * f.width + t.px];
         const float diff[3] = {sum[0] - want.x, sum[1] - want.y, sum[2] - want.z};
@@ -871,7 +866,8 @@ template <int kK> __global__ void __launch_bounds__(kThreads, 6) adjointForward(
         tr.head[t.ray] = make_int4(steps, top, escaped ? 1 : 0, 0);
         tr.bar[t.ray] = make_float4(2.f * diff[0] * v.lossScale, 2.f * diff[1] * v.lossScale,
                                     2.f * diff[2] * v.lossScale, through);
-        storeState(tr.end + t.ray, tr.rays, end, through);
+        storeMotion(tr.end + t.ray, tr.rays, s);
+        __stcs(tr.end + 2 * tr.rays + t.ray, make_float4(s.psi, s.drag, through, 0.f));
         tally.rays += 1;
         tally.steps += (unsigned)steps;
         tally.crossings += crossings;
@@ -918,57 +914,67 @@ template <int kK> __global__ void __launch_bounds__(kThreads, 3) adjointReverse(
         const float rhoScale = recipR(1.f - divR(f.inner, f.outer));
         const float4 bar = tr.bar[t.ray];
         const float sumBar[3] = {bar.x, bar.y, bar.z}, throughEnd = bar.w;
-        const BackTerms bt = backTerms(a, c.step);
         StepBar next;
         memset(&next, 0, sizeof next);
-        ConstBar g, gs; /* gs: what the steps' own maps give the constants the step length scales */
+        ConstBar g;
+        StepSums sums; /* what the steps' own maps give */
         memset(&g, 0, sizeof g);
-        memset(&gs, 0, sizeof gs);
+        memset(&sums, 0, sizeof sums);
         float throughBar = 0.f, direct = 0.f; /* direct: velocities against what crossings add to their adjoints */
-        RayState<float> after; /* the state after the step being taken back */
-        /* One step taken back: k, the state it started from; after, the state it ended in. */
-        auto back = [&](const Kept& k, int step) {
-            StepOut<float> o;
-            o.next = after;
-            o.k1 = bendAt(c, k.s.u);
-            accelWith(bt, c.big, k.s.n, o.a1);
+        RayState<float> after = start; /* the state after the step being taken back: its u and n */
+        DragTerms drag = {0.f, 0.f, false}; /* and the drag rate there */
+        /* One step taken back: s, the state it started from (u, w, n, v); after, the one it ended in; met():
+         * what its crossing takes (Trail), read only at a step that may have one. */
+        auto back = [&](RayState<float>& from, int step, auto met) {
             StepBar b;
             memset(&b, 0, sizeof b);
-            b.nextU = next.u;
-            for (int j = 0; j < 3; ++j) b.nextN[j] = next.n[j];
-            b.nextPsi = next.psi;
-            b.nextDrag = next.drag;
-            if (escaped && step == steps - 1 && f.stars > 0.f)
-                skyBack(v, c, k.s, o.next, throughEnd, sumBar, throughBar, b, g);
-            Crossing<float> x;
-            const bool crossed = crossingOf(f, rhoScale, c, k.s, o, x);
-            if (crossed) {
-                crossingBack(v, rhoScale, c, k.s, o, x, k.through, sumBar, throughBar, b, g);
-                direct += k.s.w * b.w + k.s.v[0] * b.v[0] + k.s.v[1] * b.v[1] + k.s.v[2] * b.v[2];
+            next.nextU = next.u, next.nextPsi = next.psi, next.nextDrag = next.drag;
+            for (int j = 0; j < 3; ++j) next.nextN[j] = next.n[j];
+            /* (most steps met nothing) */
+            if ((step == steps - 1) | (from.n[2] * after.n[2] < 0.f)) {
+                b.nextU = next.nextU, b.nextPsi = next.nextPsi, b.nextDrag = next.nextDrag;
+                for (int j = 0; j < 3; ++j) b.nextN[j] = next.nextN[j];
+                const float4 taken = met();
+                StepOut<float> o;
+                o.next = after;
+                o.next.psi = taken.z, o.next.drag = drag.rate;
+                from.psi = taken.x, from.drag = a != 0.f ? dragTerms(a, c.xiA, from.u).rate : 0.f;
+                o.k1 = bendAt(c, from.u);
+                const float c1 = c.big + 2.f * a * a * (from.n[2] * from.n[2]);
+                o.a1[0] = -c1 * from.n[0], o.a1[1] = -c1 * from.n[1], o.a1[2] = a * a * from.n[2] - c1 * from.n[2];
+                if (escaped && step == steps - 1 && f.stars > 0.f)
+                    skyBack(v, c, from, o.next, throughEnd, sumBar, throughBar, b, g);
+                Crossing<float> x;
+                if (crossingOf(f, rhoScale, c, from, o, x)) {
+                    crossingBack(v, rhoScale, c, from, o, x, taken.y, sumBar, throughBar, b, g);
+                    direct += from.w * b.w + from.v[0] * b.v[0] + from.v[1] * b.v[1] + from.v[2] * b.v[2];
+                    firstStageBack(a, c, from, b, g);
+                }
+                next.nextU = b.nextU, next.nextPsi = b.nextPsi, next.nextDrag = b.nextDrag;
+                for (int j = 0; j < 3; ++j) next.nextN[j] = b.nextN[j];
             }
-            radialBack(bt, c, k.s.u, k.s.w, k.s.drag, b.nextU, next.w, b.nextPsi, b.nextDrag, b.k1, crossed, b.u, b.w,
-                       b.psi, b.drag, g, gs);
-            polarBack(bt, c.big, k.s.n, k.s.v, b.nextN, next.v, b.a1, crossed, b.n, b.v, g, gs);
+            stepBack(a, c, from, after.u, drag, next, b, g, sums);
             next = b;
-            after = k.s;
+            after = from;
         };
-        float unused;
+        auto dragHere = [&]() { return a != 0.f ? dragTerms(a, c.xiA, after.u) : DragTerms{0.f, 0.f, false}; };
         if constexpr (kK == 1) {
             /* the state after the last step taken back: the ray's end when that step was its last, else kept */
-            loadState(top == steps ? tr.end + t.ray : tr.saved + (size_t)(3 * top) * tr.rays + t.ray, tr.rays, after,
-                      unused);
+            const float4* const last = top == steps ? tr.end + t.ray : tr.saved + (size_t)(3 * top) * tr.rays + t.ray;
+            setMotion(after, last[0], last[tr.rays]);
+            drag = dragHere();
             /* The warp walks back together from its highest step, each lane taking back only its own steps
              * (below its top): at each step the active lanes' kept states are one run of 512 bytes in each
-             * of the trail's three planes. */
+             * of the trail's planes. */
             const int warpTop = __reduce_max_sync(__activemask(), top);
             const float4* lane = tr.saved + t.ray;
-            __shared__ float4 stage[kThreads / 32][kStage][3][32];
-            float4(*mine)[3][32] = stage[threadIdx.x >> 5];
+            __shared__ float4 stage[kThreads / 32][kStage][2][32];
+            float4(*mine)[2][32] = stage[threadIdx.x >> 5];
             const int me = (int)(threadIdx.x & 31);
             auto fetch = [&](int s) {
                 if (s >= 0 && s < top) {
                     const float4* from = lane + (size_t)(3 * s) * tr.rays;
-                    for (int q = 0; q < 3; ++q) {
+                    for (int q = 0; q < 2; ++q) {
                         const unsigned to = (unsigned)__cvta_generic_to_shared(&mine[s % kStage][q][me]);
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to), "l"(from + q * tr.rays)
                                      : "memory");
@@ -982,35 +988,50 @@ template <int kK> __global__ void __launch_bounds__(kThreads, 3) adjointReverse(
                 asm volatile("cp.async.wait_group %0;\n" ::"n"(kStage - 1) : "memory");
                 if (step < top) {
                     const float4(*at)[32] = mine[step % kStage];
-                    const float4 p0 = at[0][me], p1 = at[1][me], p2 = at[2][me];
-                    Kept k;
-                    k.s.u = p0.x, k.s.w = p0.y, k.s.n[0] = p0.z, k.s.n[1] = p0.w;
-                    k.s.n[2] = p1.x, k.s.v[0] = p1.y, k.s.v[1] = p1.z, k.s.v[2] = p1.w;
-                    k.s.psi = p2.x, k.s.drag = p2.y, k.through = p2.z;
-                    back(k, step);
+                    RayState<float> s;
+                    setMotion(s, at[0][me], at[1][me]);
+                    back(s, step, [&]() { return lane[(size_t)(3 * step + 2) * tr.rays]; });
                 }
             }
         } else {
-            Kept ring[kK ? kK : kMaxK];
+            float4 ring[kK ? kK : kMaxK][2], met[kK ? kK : kMaxK];
             for (int first = ((top - 1) / K) * K; first >= 0; first -= K) {
                 const int last = min(first + K, top); /* steps first .. last - 1 */
                 /* the segment's states from its kept start; the state after its last step is the ray's end
                  * when that step was the ray's last, else one more step on */
+                const float4* const kept = tr.saved + (size_t)(3 * (first / K)) * tr.rays + t.ray;
                 RayState<float> r;
-                float through;
-                loadState(tr.saved + (size_t)(3 * (first / K)) * tr.rays + t.ray, tr.rays, r, through);
-                float junk[3] = {0.f, 0.f, 0.f};
-                unsigned n = 0;
+                setMotion(r, kept[0], kept[tr.rays]);
+                const float4 rest = kept[2 * tr.rays];
+                r.psi = rest.x, r.drag = rest.y;
+                float through = rest.z;
                 for (int step = first; step < last; ++step) {
-                    ring[step - first] = Kept{r, through};
-                    if (step == steps - 1) break;
+                    ring[step - first][0] = make_float4(r.u, r.w, r.n[0], r.n[1]);
+                    ring[step - first][1] = make_float4(r.n[2], r.v[0], r.v[1], r.v[2]);
+                    if (step == steps - 1) {
+                        met[step - first] = make_float4(r.psi, through, tr.end[2 * tr.rays + t.ray].x, 0.f);
+                        break;
+                    }
                     StepOut<float> o;
-                    stepOnce(v, rhoScale, c, r, o, through, junk, n);
+                    nystromStep(a, c, r, o);
+                    if (r.n[2] * o.next.n[2] < 0.f) {
+                        met[step - first] = make_float4(r.psi, through, o.next.psi, 0.f);
+                        Crossing<float> x;
+                        if (crossingOf(f, rhoScale, c, r, o, x)) {
+                            float turn, junk[3] = {0.f, 0.f, 0.f};
+                            shadeCrossing(f, rhoScale, v.map, v.fluid, c, x, through, junk, &turn);
+                        }
+                    }
                     r = o.next;
                 }
                 after = r;
-                if (last == steps) loadState(tr.end + t.ray, tr.rays, after, unused);
-                for (int step = last - 1; step >= first; --step) back(ring[step - first], step);
+                if (last == steps) setMotion(after, tr.end[t.ray], tr.end[tr.rays + t.ray]);
+                drag = dragHere();
+                for (int step = last - 1; step >= first; --step) {
+                    RayState<float> s;
+                    setMotion(s, ring[step - first][0], ring[step - first][1]);
+                    back(s, step, [&]() { return met[step - first]; });
+                }
             }
         }
         /* The step length's adjoint from the motion, over the whole ray at once.  A Nystrom step of length h
@@ -1019,10 +1040,17 @@ template <int kK> __global__ void __launch_bounds__(kThreads, 3) adjointReverse(
          * summed over the ray the terms telescope to the first state's velocities against their adjoints,
          * less the velocities against what crossings added to their adjoints, and the scaled coefficients
          * against what the steps gave their adjoints (for a: 2 a^2 d/d(a^2) = a d/da). */
+        const float axis = 2.f * a * sums.axis;
         g.step += (start.w * next.w + start.v[0] * next.v[0] + start.v[1] * next.v[1] + start.v[2] * next.v[2] -
-                   direct + 2.f * (c.uA * gs.uA + c.uB * gs.uB + c.uC * gs.uC + c.big * gs.big) + a * gs.a) /
+                   direct + 2.f * (c.uA * sums.uA + c.uB * sums.uB + c.uC * sums.uC + c.big * sums.big) + a * axis) /
                   c.step;
-        g.a += gs.a, g.big += gs.big, g.uA += gs.uA, g.uB += gs.uB, g.uC += gs.uC;
+        float one0, one1, two0, two1, den0, den1;
+        unpack(sums.one, one0, one1);
+        unpack(sums.two, two0, two1);
+        unpack(sums.den, den0, den1);
+        g.a += axis - 2.f * (one0 + one1) + c.xiA * (two0 + two1) + 2.f * a * (den0 + den1);
+        g.xiA += a * (two0 + two1);
+        g.big += sums.big, g.uA += sums.uA, g.uB += sums.uB, g.uC += sums.uC;
         startBack(v, nx, ny, c, next, g, grad);
     }
     if (t.inside && v.pixelGrads)

@@ -481,7 +481,7 @@ template <typename R> ARTF_HD void nystromStep(R a, const RayConst<R>& c, const 
 }
 
 /* Blackwell's packed instructions do two float operations in one issue slot, each rounded as by itself. */
-#if defined(__CUDA_ARCH__) && (defined(ARTF_PINNED_FMA) || defined(ARTF_EXACT_FLOAT))
+#if defined(__CUDACC__) && (defined(ARTF_PINNED_FMA) || defined(ARTF_EXACT_FLOAT))
 #if defined(ARTF_EXACT_FLOAT)
 #define ARTF_FTZ "" /* (subnormals kept, as the reference keeps them) */
 #else
@@ -511,16 +511,17 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b) {
 }
 __device__ __forceinline__ F2 both(float a) { return pack(a, a); }
 #endif
+#if defined(__CUDACC__) && defined(ARTF_PINNED_FMA)
+__device__ __forceinline__ float bendPoly(const RayConst<float>& c, float x) {
+    return __fmaf_rn(x, __fmaf_rn(x, c.uC, c.uB), c.uA);
+}
+__device__ __forceinline__ float axisAccel(float a2, float c, float z) { return __fmaf_rn(a2, z, -__fmul_rn(c, z)); }
+#endif
 
 #if defined(__CUDA_ARCH__) && defined(ARTF_PINNED_FMA)
 /* The FP32 step, packed.  Its four coordinates, u and n, go through the same Nystrom stages with the same
  * factors, so they ride in two pairs, (n_x, n_y) and (u, n_z), and the two drag rates in one: 27 of some
  * 115 instructions a step fewer (the mixed 1080p x 4 frame 1.86 -> 1.76 ms). */
-__device__ __forceinline__ float bendPoly(const RayConst<float>& c, float x) {
-    return __fmaf_rn(x, __fmaf_rn(x, c.uC, c.uB), c.uA);
-}
-__device__ __forceinline__ float axisAccel(float a2, float c, float z) { return __fmaf_rn(a2, z, -__fmul_rn(c, z)); }
-
 /* Each rounding is written out as the scalar code's compiles: x + (y + y) is fma(2, y, x), which rounds
  * the same. */
 template <>
