@@ -15,6 +15,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 namespace {
 
@@ -42,8 +43,27 @@ struct Planes {
     float* c[3];
 };
 
+/* The pass is a chain of short kernels, so each may start while the one before it drains (programmatic
+ * dependent launch) and waits here, before its first read, until that one has finished and its writes are
+ * visible.  Since a kernel of the chain finishes only after the one before it, so has all before them. */
+__device__ __forceinline__ void chained() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t follow(cudaStream_t stream, void (*kernel)(P...), dim3 grid, int block, const A&... args) {
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid, c.blockDim = dim3((unsigned)block), c.stream = stream, c.attrs = &early, c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 /* software.c:334-351: level 0 from the frame's light. */
 __global__ void bloomFirst(const float4* hdr, int width, int height, Planes bloom, uint32_t at, int toW, int toH) {
+    chained();
     const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), y = (int)blockIdx.y;
     if (x >= toW || y >= toH) return;
     const int lastX = width - 1, lastY = height - 1;
@@ -55,31 +75,76 @@ __global__ void bloomFirst(const float4* hdr, int width, int height, Planes bloo
         bloom.c[c][at + (size_t)y * toW + x] = (bright(s[c][0]) + bright(s[c][1]) + bright(s[c][2]) + bright(s[c][3])) * .25f;
 }
 
-/* software.c:353-365: level L from level L - 1, four taps. */
+/* software.c:353-365: a texel of level L from level L - 1, four taps. */
+__device__ __forceinline__ float downTexel(const float* from, int fromW, int fromH, int x, int y) {
+    const float cy = (float)y * 2.f + .5f, cx = (float)x * 2.f + .5f;
+    float sum = 0;
+    for (int k = 0; k < 4; ++k) sum += tap(from, fromW, fromH, cx + (k & 1 ? 1.f : -1.f), cy + (k & 2 ? 1.f : -1.f));
+    return sum * .25f;
+}
+
+/* software.c:368-386: what a texel of level L gains, four taps of level L + 1. */
+__device__ __forceinline__ float upTexel(const float* from, int fromW, int fromH, int x, int y) {
+    const float sy = ((float)y + .5f) * .5f - .5f, sx = ((float)x + .5f) * .5f - .5f;
+    float sum = 0;
+    for (int k = 0; k < 4; ++k) sum += tap(from, fromW, fromH, sx + (k & 1 ? .5f : -.5f), sy + (k & 2 ? .5f : -.5f));
+    return sum * (.25f * kFade);
+}
+
 __global__ void bloomDown(Planes bloom, uint32_t fromAt, int fromW, int fromH, uint32_t toAt, int toW, int toH) {
+    chained();
     const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), y = (int)blockIdx.y;
     if (x >= toW || y >= toH) return;
-    const float cy = (float)y * 2.f + .5f, cx = (float)x * 2.f + .5f;
+    for (int c = 0; c < 3; ++c)
+        bloom.c[c][toAt + (size_t)y * toW + x] = downTexel(bloom.c[c] + fromAt, fromW, fromH, x, y);
+}
+
+__global__ void bloomUp(Planes bloom, uint32_t fromAt, int fromW, int fromH, uint32_t toAt, int toW, int toH) {
+    chained();
+    const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), y = (int)blockIdx.y;
+    if (x >= toW || y >= toH) return;
     for (int c = 0; c < 3; ++c) {
-        const float* level = bloom.c[c] + fromAt;
-        float sum = 0;
-        for (int k = 0; k < 4; ++k) sum += tap(level, fromW, fromH, cx + (k & 1 ? 1.f : -1.f), cy + (k & 2 ? 1.f : -1.f));
-        bloom.c[c][toAt + (size_t)y * toW + x] = sum * .25f;
+        float* out = bloom.c[c] + toAt + (size_t)y * toW + x;
+        *out += upTexel(bloom.c[c] + fromAt, fromW, fromH, x, y);
     }
 }
 
-/* software.c:368-386: level L gains four taps of level L + 1. */
-__global__ void bloomUp(Planes bloom, uint32_t fromAt, int fromW, int fromH, uint32_t toAt, int toW, int toH) {
-    const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), y = (int)blockIdx.y;
-    if (x >= toW || y >= toH) return;
-    const float sy = ((float)y + .5f) * .5f - .5f, sx = ((float)x + .5f) * .5f - .5f;
-    for (int c = 0; c < 3; ++c) {
-        const float* level = bloom.c[c] + fromAt;
-        float sum = 0;
-        for (int k = 0; k < 4; ++k) sum += tap(level, fromW, fromH, sx + (k & 1 ? .5f : -.5f), sy + (k & 2 ? .5f : -.5f));
-        float* out = bloom.c[c] + toAt + (size_t)y * toW + x;
-        *out += sum * (.25f * kFade);
+/* The pyramid's small levels, `first` to the last, down and up again in one block's shared memory: a launch
+ * each is some 3 us, most of it waiting for the one before.  Up to 1024 texels in all (a 1080p frame's last
+ * three levels: the frame 535 -> 525 us); 4096 keep the one block longer than their launches take (21 us by
+ * itself; the frame 532). */
+constexpr int kTailThreads = 1024;
+constexpr size_t kTailTexels = 1024;
+struct TailLevels {
+    uint32_t level[ARTF_CUDA_BLOOM_LEVELS][4];
+    int first, count;
+};
+
+__global__ void __launch_bounds__(kTailThreads) bloomTail(Planes bloom, const __grid_constant__ TailLevels t) {
+    __shared__ float held[3 * kTailTexels];
+    chained();
+    const uint32_t base = t.level[t.first][0], texels = t.level[t.count - 1][0] - base +
+                                                        t.level[t.count - 1][1] * t.level[t.count - 1][2];
+    for (int i = t.first; i < t.count; ++i) {
+        const int w = (int)t.level[i][1], h = (int)t.level[i][2], fw = (int)t.level[i - 1][1], fh = (int)t.level[i - 1][2];
+        for (int k = (int)threadIdx.x; k < 3 * w * h; k += kTailThreads) {
+            const int c = k / (w * h), at = k - c * w * h, y = at / w, x = at - y * w;
+            const float* from = i == t.first ? bloom.c[c] + t.level[i - 1][0]
+                                             : held + c * texels + (t.level[i - 1][0] - base);
+            held[c * texels + (t.level[i][0] - base) + at] = downTexel(from, fw, fh, x, y);
+        }
+        __syncthreads();
     }
+    for (int i = t.count - 1; i-- > t.first;) {
+        const int w = (int)t.level[i][1], h = (int)t.level[i][2], fw = (int)t.level[i + 1][1], fh = (int)t.level[i + 1][2];
+        for (int k = (int)threadIdx.x; k < 3 * w * h; k += kTailThreads) {
+            const int c = k / (w * h), at = k - c * w * h, y = at / w, x = at - y * w;
+            held[c * texels + (t.level[i][0] - base) + at] +=
+                upTexel(held + c * texels + (t.level[i + 1][0] - base), fw, fh, x, y);
+        }
+        __syncthreads();
+    }
+    for (uint32_t k = threadIdx.x; k < 3 * texels; k += kTailThreads) bloom.c[k / texels][base + k % texels] = held[k];
 }
 
 /* lens.inc:56-61: the dither's hash (the star lattice's). */
@@ -100,6 +165,7 @@ __device__ __forceinline__ float toneCurve(float x) {
 /* lens.inc:395-440: light plus glow, exposed, tone mapped and dithered to premultiplied BGRA. */
 __global__ void toneMap(const float4* hdr, int width, int height, Planes bloom, uint32_t at, int bw, int bh,
                         float exposure, float spread, uint32_t* bgra) {
+    chained();
     const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), y = (int)blockIdx.y;
     if (x >= width || y >= height) return;
     const float sy = ((float)y + .5f) * .5f - .5f, baseY = floorf(sy), partY = sy - baseY;
@@ -142,21 +208,38 @@ extern "C" int artfCudaPostLaunch(const ArtfCudaHoleFrame* frame, const float* h
     Planes planes = {{bloomPlanes[0], bloomPlanes[1], bloomPlanes[2]}};
     const int block = 128;
     const uint32_t(*table)[4] = frame->bloom;
-    for (int i = 0; i < levels; ++i) {
-        const dim3 grid((table[i][1] + block - 1) / block, table[i][2]);
-        if (i == 0) bloomFirst<<<grid, block, 0, s>>>((const float4*)hdr, width, height, planes, table[0][0],
-                                                      (int)table[0][1], (int)table[0][2]);
-        else bloomDown<<<grid, block, 0, s>>>(planes, table[i - 1][0], (int)table[i - 1][1], (int)table[i - 1][2],
-                                              table[i][0], (int)table[i][1], (int)table[i][2]);
+    cudaError_t e = cudaSuccess;
+    /* the levels from `tail` on in one launch: from the second at the earliest, where they lie one after another
+     * and fit the block, and there are two or more */
+    int tail = levels;
+    size_t texels = 0;
+    for (int i = levels - 1; i > 0; --i) {
+        texels += (size_t)table[i][1] * table[i][2];
+        if (texels > kTailTexels || (i + 1 < levels && table[i][0] + table[i][1] * table[i][2] != table[i + 1][0])) break;
+        tail = i;
     }
-    for (int i = levels - 1; i-- > 0;) {
+    if (levels - tail < 2) tail = levels;
+    for (int i = 0; i < tail && e == cudaSuccess; ++i) {
         const dim3 grid((table[i][1] + block - 1) / block, table[i][2]);
-        bloomUp<<<grid, block, 0, s>>>(planes, table[i + 1][0], (int)table[i + 1][1], (int)table[i + 1][2], table[i][0],
-                                       (int)table[i][1], (int)table[i][2]);
+        if (i == 0) e = follow(s, bloomFirst, grid, block, (const float4*)hdr, width, height, planes, table[0][0],
+                               (int)table[0][1], (int)table[0][2]);
+        else e = follow(s, bloomDown, grid, block, planes, table[i - 1][0], (int)table[i - 1][1], (int)table[i - 1][2],
+                        table[i][0], (int)table[i][1], (int)table[i][2]);
+    }
+    if (tail < levels && e == cudaSuccess) {
+        TailLevels t;
+        memcpy(t.level, table, sizeof t.level);
+        t.first = tail, t.count = levels;
+        e = follow(s, bloomTail, dim3(1), kTailThreads, planes, t);
+    }
+    for (int i = tail < levels ? tail : levels - 1; i-- > 0 && e == cudaSuccess;) {
+        const dim3 grid((table[i][1] + block - 1) / block, table[i][2]);
+        e = follow(s, bloomUp, grid, block, planes, table[i + 1][0], (int)table[i + 1][1], (int)table[i + 1][2],
+                   table[i][0], (int)table[i][1], (int)table[i][2]);
     }
     const float spread = frame->look[3] * (1.f - kFade);
-    toneMap<<<dim3((width + block - 1) / block, height), block, 0, s>>>(
-        (const float4*)hdr, width, height, planes, table[0][0], (int)table[0][1], (int)table[0][2], frame->image[0],
-        spread, bgra);
-    return cudaGetLastError() == cudaSuccess ? ARTF_CUDA_OK : ARTF_CUDA_ELAUNCH;
+    if (e == cudaSuccess)
+        e = follow(s, toneMap, dim3((width + block - 1) / block, height), block, (const float4*)hdr, width, height, planes,
+                   table[0][0], (int)table[0][1], (int)table[0][2], frame->image[0], spread, bgra);
+    return e == cudaSuccess ? ARTF_CUDA_OK : ARTF_CUDA_ELAUNCH;
 }

@@ -265,3 +265,64 @@ def test_frame_read_after_a_draw(lib, ctx, golden):
                                       C.byref(opts), light2.ctypes.data, None))
     assert lib.artfCudaFrameRead(ctx, None, only.ctypes.data) == -1
     assert b"no frame drawn" in lib.artfCudaLastError()
+
+
+@pytest.mark.parametrize("width,height", [(1, 1), (7, 9), (61, 40), (130, 65), (257, 511), (1920, 1080)])
+def test_bloom_pyramid_equals_its_levels_one_by_one(lib, ctx, width, height):
+    """The post pass over sizes whose pyramids have one level, levels in one launch and levels of their own:
+    every level and the BGRA frame against the pyramid and tone map in numpy, float for float."""
+    import torch
+    rng = np.random.default_rng(width * 31 + height)
+    view = scenes.Scene("post", scenes.hole_desc(0.5), scenes.camera(70.0, 30.0), width, height)
+    view.desc.bloom = 4.5
+    frame, _, _ = scenes.frame(view)
+    f = np.float32
+    hdr = np.zeros((height, width, 4), np.float32)
+    hdr[..., :3] = (rng.exponential(2.0, (height, width, 3)) ** 1.5).astype(np.float32)
+    levels = [tuple(int(v) for v in frame.bloom[i])[:3] for i in range(frame.size[3])]
+    total = sum(w * h for _, w, h in levels)
+
+    def tap(level, sx, sy):
+        h, w = level.shape
+        bx, by = np.floor(sx), np.floor(sy)
+        px, py = (sx - bx).astype(f), (sy - by).astype(f)
+        x0, x1 = np.clip(bx.astype(int), 0, w - 1), np.clip(bx.astype(int) + 1, 0, w - 1)
+        y0, y1 = np.clip(by.astype(int), 0, h - 1), np.clip(by.astype(int) + 1, 0, h - 1)
+        top = level[y0, x0] + (level[y0, x1] - level[y0, x0]) * px
+        bottom = level[y1, x0] + (level[y1, x1] - level[y1, x0]) * px
+        return top + (bottom - top) * py
+
+    want = []
+    for c in range(3):
+        bright = np.minimum(np.maximum(hdr[..., c] - f(2), f(0)), f(48))
+        pyramid = []
+        for i, (_, w, h) in enumerate(levels):
+            y, x = np.meshgrid(np.arange(h), np.arange(w), indexing="ij")
+            if i == 0:
+                y0, y1 = np.minimum(2 * y, height - 1), np.minimum(2 * y + 1, height - 1)
+                x0, x1 = np.minimum(2 * x, width - 1), np.minimum(2 * x + 1, width - 1)
+                pyramid.append((bright[y0, x0] + bright[y0, x1] + bright[y1, x0] + bright[y1, x1]) * f(.25))
+                continue
+            cx, cy, s = x.astype(f) * f(2) + f(.5), y.astype(f) * f(2) + f(.5), np.zeros((h, w), f)
+            for k in range(4):
+                s = s + tap(pyramid[-1], cx + f(1 if k & 1 else -1), cy + f(1 if k & 2 else -1))
+            pyramid.append(s * f(.25))
+        for i in range(len(levels) - 2, -1, -1):
+            _, w, h = levels[i]
+            y, x = np.meshgrid(np.arange(h), np.arange(w), indexing="ij")
+            sx, sy, s = (x.astype(f) + f(.5)) * f(.5) - f(.5), (y.astype(f) + f(.5)) * f(.5) - f(.5), np.zeros((h, w), f)
+            for k in range(4):
+                s = s + tap(pyramid[i + 1], sx + f(.5 if k & 1 else -.5), sy + f(.5 if k & 2 else -.5))
+            pyramid[i] = pyramid[i] + s * (f(.25) * f(.85))
+        want.append(np.concatenate([p.ravel() for p in pyramid]))
+    device = torch.from_numpy(hdr).cuda()
+    planes = [torch.zeros(total, dtype=torch.float32, device="cuda") for _ in range(3)]
+    bgra = torch.zeros((height, width), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    pointers = (C.c_void_p * 3)(*[p.data_ptr() for p in planes])
+    capi.check(lib.artfCudaPostLaunch(C.byref(frame), device.data_ptr(), pointers, bgra.data_ptr(),
+                                      lib.artfCudaStream(ctx)))
+    torch.cuda.synchronize()
+    for p, w in zip(planes, want):
+        np.testing.assert_array_equal(p.cpu().numpy().view(np.uint32), w.view(np.uint32))
+    assert bool((bgra != 0).all())
