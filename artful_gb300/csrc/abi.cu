@@ -15,6 +15,10 @@
 #include <string.h>
 #include <unistd.h>
 
+namespace artf {
+void trimGases(int device);
+}
+
 static thread_local char lastError[256];
 
 static int fail(int status, const char* format, ...) {
@@ -193,6 +197,7 @@ extern "C" void artfCudaDestroy(ArtfCuda* ctx) {
     if (ctx->stop) cudaEventDestroy(ctx->stop);
     if (ctx->staged) cudaEventDestroy(ctx->staged);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    artf::trimGases(ctx->device);
     free(ctx);
 }
 

@@ -31,6 +31,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <mutex>
+
 namespace artf {
 int contextStream(ArtfCuda* ctx, cudaStream_t* stream);
 int contextFluid(ArtfCuda* ctx, float** fluid);
@@ -362,9 +364,10 @@ __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 3
 
 struct ArtfCudaFluid {
     ArtfCuda* ctx;
+    int device;
     cudaStream_t stream;
     float inner, outer;
-    float* block;          /* the seven fields, one allocation */
+    float* block;          /* the seven fields and the rings' terms, one allocation */
     float* dens[2];
     float* radial[2];
     float* orbital[2];
@@ -377,6 +380,58 @@ struct ArtfCudaFluid {
 };
 
 namespace {
+
+/* Where gases' memory comes from: a pool a device, which keeps up to two gases' worth when they are freed, so
+ * that a disc that changes does not map and unmap its gas each time (0.2 ms of a new gas's 0.9), until a
+ * context is destroyed (trimGases).  NULL where the device has no pools. */
+constexpr size_t GAS_BYTES = sizeof(float) * FIELD * 7 + sizeof(Ring) * FH;
+constexpr int MOST_DEVICES = 64;
+std::mutex poolLock;
+cudaMemPool_t pools[MOST_DEVICES];
+
+cudaMemPool_t poolOf(int device) {
+    if (device < 0 || device >= MOST_DEVICES) return nullptr;
+    std::lock_guard<std::mutex> hold(poolLock);
+    if (!pools[device]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        uint64_t keep = 2 * (GAS_BYTES + ((size_t)2 << 20));
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        pools[device] = pool;
+    }
+    return pools[device];
+}
+
+/* A gas's memory, its use by the stream's work to come; and given back, once the device is done with it (work
+ * on other streams that reads the field among it). */
+cudaError_t takeGas(ArtfCudaFluid* f) {
+    const cudaMemPool_t pool = poolOf(f->device);
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync((void**)&f->block, GAS_BYTES, pool, f->stream)
+                               : cudaMalloc((void**)&f->block, GAS_BYTES);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError(); /* (or the next launch's check would report it) */
+        f->block = nullptr;
+    }
+    return e;
+}
+
+void giveGas(ArtfCudaFluid* f) {
+    if (!f->block) return;
+    int current = 0;
+    const bool known = cudaGetDevice(&current) == cudaSuccess;
+    cudaSetDevice(f->device);
+    cudaDeviceSynchronize();
+    if (poolOf(f->device)) cudaFreeAsync(f->block, cudaStreamLegacy); /* (its context may be gone) */
+    else cudaFree(f->block);
+    if (known) cudaSetDevice(current);
+}
 
 uint32_t draw(ArtfCudaFluid* f) {
     uint32_t x = f->state;
@@ -466,11 +521,17 @@ int advanceSteps(ArtfCudaFluid* f, int64_t steps) {
 
 }  // namespace
 
+namespace artf {
+/* The memory the device's pool holds beyond the gases that live, given back (a context was destroyed). */
+void trimGases(int device) {
+    std::lock_guard<std::mutex> hold(poolLock);
+    if (device >= 0 && device < MOST_DEVICES && pools[device]) cudaMemPoolTrimTo(pools[device], 0);
+}
+}  // namespace artf
+
 extern "C" void artfCudaFluidFree(ArtfCudaFluid* f) {
     if (!f) return;
-    cudaStreamSynchronize(f->stream);
-    cudaFree(f->block);
-    cudaFree(f->rings);
+    giveGas(f);
     free(f);
 }
 
@@ -487,8 +548,7 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
     if (!f) return artf::failWith(ARTF_CUDA_ENOMEM, "host allocation");
     f->ctx = ctx, f->stream = stream, f->inner = inner, f->outer = outer;
     f->state = 0x9E3779B9u, f->time = time;
-    if (cudaMalloc(&f->block, sizeof(float) * FIELD * 7) != cudaSuccess ||
-        cudaMalloc(&f->rings, sizeof f->host) != cudaSuccess) {
+    if (cudaGetDevice(&f->device) != cudaSuccess || takeGas(f) != cudaSuccess) {
         artfCudaFluidFree(f);
         return artf::failWith(ARTF_CUDA_ENOMEM, "fluid: device allocation");
     }
@@ -496,6 +556,7 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
         f->dens[k] = f->block + FIELD * (3 * k), f->radial[k] = f->block + FIELD * (3 * k + 1),
         f->orbital[k] = f->block + FIELD * (3 * k + 2);
     f->field = f->block + FIELD * 6;
+    f->rings = (Ring*)(f->block + FIELD * 7);
     /* the rings (fluid.c:270-290), on the host in float as the reference has them */
     const float k = 1.f - inner / outer;
     for (int j = 0; j < FH; ++j) {
@@ -524,12 +585,12 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
         g.toRows = DT / ((g.up - g.down) * (j == 0 || j == FH - 1 ? 1.f : .5f));
     }
     cudaError_t e = cudaMemcpyAsync(f->rings, f->host, sizeof f->host, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(f->block, 0, sizeof(float) * FIELD * 7, stream);
+    /* (at rest: the two velocities lie together; the rest is written before it is read) */
+    if (e == cudaSuccess) e = cudaMemsetAsync(f->radial[0], 0, sizeof(float) * FIELD * 2, stream);
     if (e == cudaSuccess) {
         seedDensity<<<(FIELD + 255) / 256, 256, 0, stream>>>(f->dens[0], f->rings);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream); /* (the rings' staging is on this frame) */
     int status = e == cudaSuccess ? stirStart(f) : artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
     if (!status) status = advanceSteps(f, WARM_STEPS);
     if (status) {

@@ -162,3 +162,32 @@ def test_each_run_of_steps_equals_the_oracle(lib, ctx, oracle_lib, inner, outer,
         np.testing.assert_array_equal(a.read()[0].view(np.uint32), b.read()[0].view(np.uint32))
     a.free()
     b.free()
+
+
+def test_gases_come_and_go(lib, ctx):
+    """Gases made and freed in turn and several at once, in two contexts one of which goes meanwhile: each the
+    bytes a gas of its disc has, in memory others have used."""
+    discs = [(6.0, 12.0, 0.0), (2.4, 20.0, 0.8), (1.9, 34.0, 0.95)]
+    want = {}
+    for d in discs:
+        a = GpuFluid(lib, ctx, *d, 0.0)
+        want[d] = a.read()[0]
+        a.free()
+    other = C.c_void_p()
+    capi.check(lib.artfCudaCreate(0, C.byref(other)))
+    try:
+        held = []
+        for k in range(9):
+            held.append((discs[k % 3], GpuFluid(lib, other if k % 2 else ctx, *discs[k % 3], 0.0)))
+            if k % 3 == 2:
+                d, a = held.pop(0)
+                assert np.array_equal(a.read()[0], want[d])
+                a.free()
+        for d, a in held:
+            assert np.array_equal(a.read()[0], want[d])
+            a.free()
+    finally:
+        lib.artfCudaDestroy(other)
+    a = GpuFluid(lib, ctx, *discs[1], 0.0)
+    assert np.array_equal(a.read()[0], want[discs[1]])
+    a.free()
