@@ -26,6 +26,7 @@
  * view heaviest first, each block copying its view's entry to shared memory, each warp tracing one tile.
  * Each tile's six sums go to the tile's own slot; a last kernel adds them in a fixed order, in double, so
  * the result does not depend on scheduling. */
+#define ARTF_CLAMP_ROWS 1 /* table rows read the plain way (lensCore.cuh: placeOf) */
 #define ARTF_PINNED_FMA 1 /* every float sum of two products rounds the same wherever it is compiled (lensCore.cuh) */
 #include "lensKernel.cuh"
 #include "lensTangent.h"

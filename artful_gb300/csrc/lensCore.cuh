@@ -14,8 +14,9 @@
  *
  * Layout in device memory: the map is one float block (ArtfCudaHoleFrame's companion, 11.5 MB: it stays
  * resident in the 126 MB L2 for a whole frame); the fluid 1 MB; the frame constants travel as a kernel
- * parameter (constant bank).  Every map read has its index clamped into the map: for the reference's
- * inputs the clamp never moves an index, and no input can make a thread read outside the buffers. */
+ * parameter (constant bank).  No input can make a thread read outside the buffers: every index is held to
+ * its table where it is formed, or clamped into the map where the reference lets it stray (the sky's rows,
+ * the colours), which for the reference's inputs never moves one. */
 #pragma once
 
 #include "artful_cuda.h"
@@ -212,6 +213,14 @@ ARTF_HD double expR(double x) { return exp(x); }
 ARTF_HD float logR(float x) { return logf(x); }
 ARTF_HD double logR(double x) { return log(x); }
 
+/* Whether an index that its table already holds is clamped all the same: see placeOf. */
+#ifdef ARTF_CLAMP_ROWS
+constexpr bool kClampRows = true;
+#else
+constexpr bool kClampRows = false;
+#endif
+ARTF_HD int32_t tableIndex(int32_t at) { return kClampRows ? clampI(at, 0, ARTF_CUDA_MAP_FLOATS - 1) : at; }
+
 /* The rings' orbit speed at a map row (hole.c:186-191 setRings, rows even in 1/r). */
 template <typename R> ARTF_HD R ringSpeedAt(const Frame<R>& f, const float* map, int32_t row) {
     if (f.analyticTables) {
@@ -219,7 +228,7 @@ template <typename R> ARTF_HD R ringSpeedAt(const Frame<R>& f, const float* map,
         const R r = divR(f.inner, R(1) - rho * (R(1) - divR(f.inner, f.outer)));
         return recipR(KF(6.2831853) * (r * rootR(r) + f.a));
     }
-    return R(fetch(map, clampI(ARTF_CUDA_ROWS_AT + row + row, 0, ARTF_CUDA_MAP_FLOATS - 1)));
+    return R(fetch(map, tableIndex(ARTF_CUDA_ROWS_AT + row + row)));
 }
 
 /* The rings' glow at a map row: (r / inner)^-q of the synthetic disc. */
@@ -229,7 +238,7 @@ template <typename R> ARTF_HD R ringGlowAt(const Frame<R>& f, const float* map, 
         const R span = R(1) - rho * (R(1) - divR(f.inner, f.outer)); /* inner / r */
         return expR(f.emissivity * logR(span));
     }
-    return R(fetch(map, clampI(ARTF_CUDA_GLOW_AT + row, 0, ARTF_CUDA_MAP_FLOATS - 1)));
+    return R(fetch(map, tableIndex(ARTF_CUDA_GLOW_AT + row)));
 }
 
 /* ---- per ray ------------------------------------------------------------------------------------ */
@@ -682,17 +691,48 @@ template <typename R> ARTF_HD R sineOf(R turns) {
     return p * x2 * x + x;
 }
 
+/* The floor of a place in a table, 0 <= x < 2^22, and as an integer; placeOf: at most `last`.  In float on
+ * the GPU by an addition of 2^23 rounded down, whose low bits are the floor: additions, where a floor and a
+ * conversion go through the slow conversion pipe (with the clamps it made needless, the exact 320 x 180 frame
+ * 53.7 -> 52.1 us, FP32 1280 x 720 x 4 457 -> 453).  Not in a unit that
+ * defines ARTF_CLAMP_ROWS: the adjoint keeps the floors and the clamps, with which its kernels' registers fall
+ * out better (a fit of 32 views 1253 us, 1290 with neither; one 512 x 288 view 430 and 448). */
+template <typename R> ARTF_HD R placeOf(R x, int32_t last, int32_t& index) {
+    const R whole = minX(floorR(x), R(last));
+    index = truncI(whole);
+    return whole;
+}
+template <typename R> ARTF_HD R placeOf(R x, int32_t& index) {
+    const R whole = floorR(x);
+    index = truncI(whole);
+    return whole;
+}
+#if defined(__CUDA_ARCH__) && !defined(ARTF_CLAMP_ROWS)
+template <> __device__ __forceinline__ float placeOf(float x, int32_t last, int32_t& index) {
+    const float t = fminf(__fadd_rd(x, 8388608.f), 8388608.f + (float)last);
+    index = __float_as_int(t) & 0x3FFFFF;
+    return __fadd_rn(t, -8388608.f);
+}
+template <> __device__ __forceinline__ float placeOf(float x, int32_t& index) {
+    const float t = __fadd_rd(x, 8388608.f);
+    index = __float_as_int(t) & 0x3FFFFF;
+    return __fadd_rn(t, -8388608.f);
+}
+#endif
+
 /* lens.inc:89-96: a row of a region of `width` (a power of two) columns starting `at` floats into a
- * buffer of `count` floats, read at a turn, linear in between.  The index is clamped to the buffer,
- * not the region: wherever the reference reads inside its buffer, this reads the same float. */
-template <typename R>
+ * buffer of `count` floats, read at a turn, linear in between.  kHeld: the row may lie outside the region,
+ * and the index is clamped to the buffer: wherever the reference reads inside its buffer, this reads the same
+ * float.  A row that placeOf found lies inside, and with the column's mask so does the index. */
+template <bool kHeld = true, typename R>
 ARTF_HD R rowAt(const float* buffer, int32_t count, int32_t at, int32_t width, int32_t row, R turn) {
-    const R pos = (turn - floorR(turn)) * R(width);
-    const R column = floorR(pos), part = pos - column;
-    const int32_t c0 = truncI(column) & (width - 1), c1 = (c0 + 1) & (width - 1);
-    const int32_t base = at + row * width;
-    const R lo = R(fetch(buffer, clampI(base + c0, 0, count - 1)));
-    const R hi = R(fetch(buffer, clampI(base + c1, 0, count - 1)));
+    const R pos = (turn - floorR(turn)) * R(width); /* 0 .. width, whole ones included */
+    int32_t c0;
+    const R column = placeOf(pos, c0), part = pos - column;
+    c0 &= width - 1;
+    const int32_t c1 = (c0 + 1) & (width - 1), base = at + row * width;
+    const R lo = R(fetch(buffer, kHeld ? clampI(base + c0, 0, count - 1) : base + c0));
+    const R hi = R(fetch(buffer, kHeld ? clampI(base + c1, 0, count - 1) : base + c1));
     return lo + (hi - lo) * part;
 }
 
@@ -748,30 +788,31 @@ template <typename R> ARTF_HD R shadeCrossing(const Frame<R>& f, R rhoScale, con
         const R rhoK = (R(1) - f.inner * uk) * rhoScale;
         const bool inside = rhoK > R(0) && rhoK < R(1);
         const R rowPos = apart(inside ? rhoK : R(0), R(ARTF_CUDA_MAP_HEIGHT - 1));
-        const R rowFloor = minX(floorR(rowPos), R(ARTF_CUDA_MAP_HEIGHT - 2));
-        const R rowPart = rowPos - rowFloor;
-        const int32_t row0 = truncI(rowFloor), row1 = row0 + 1;
+        int32_t row0;
+        const R rowFloor = placeOf(rowPos, ARTF_CUDA_MAP_HEIGHT - 2, row0), rowPart = rowPos - rowFloor;
+        const int32_t row1 = row0 + 1;
         inBounds(f.fault, kBoundsGasRow, row0, ARTF_CUDA_MAP_HEIGHT - 1); /* (row0 and row1) */
         const R speed0 = ringSpeedAt(f, map, row0), speed1 = ringSpeedAt(f, map, row1);
         const R turnK = turn + (inside ? apart(rate, ds) : R(0));
-        const R d0 = rowAt(map, mapCount, 0, ARTF_CUDA_MAP_WIDTH, row0, turnK - speed0 * c.time);
-        const R d1 = rowAt(map, mapCount, 0, ARTF_CUDA_MAP_WIDTH, row1, turnK - speed1 * c.time);
+        const R d0 = rowAt<kClampRows>(map, mapCount, 0, ARTF_CUDA_MAP_WIDTH, row0, turnK - speed0 * c.time);
+        const R d1 = rowAt<kClampRows>(map, mapCount, 0, ARTF_CUDA_MAP_WIDTH, row1, turnK - speed1 * c.time);
         R density = d0 + (d1 - d0) * rowPart;
         /* the fluid, each ring turned on since it was stepped */
         const R fluidPos = apart(inside ? rhoK : R(0), R(ARTF_CUDA_FLUID_HEIGHT - 1));
-        const R fluidFloor = minX(floorR(fluidPos), R(ARTF_CUDA_FLUID_HEIGHT - 2));
-        const int32_t fluidRow = truncI(fluidFloor);
+        int32_t fluidRow;
+        const R fluidFloor = placeOf(fluidPos, ARTF_CUDA_FLUID_HEIGHT - 2, fluidRow);
         inBounds(f.fault, kBoundsFluidRow, fluidRow, ARTF_CUDA_FLUID_HEIGHT - 1); /* (and the row after) */
         const R fluidTurn = turnK - speed0 * fluidTime;
-        const R g0 = rowAt(fluid, fluidCount, 0, ARTF_CUDA_FLUID_WIDTH, fluidRow, fluidTurn);
-        const R g1 = rowAt(fluid, fluidCount, 0, ARTF_CUDA_FLUID_WIDTH, fluidRow + 1, fluidTurn);
+        const R g0 = rowAt<kClampRows>(fluid, fluidCount, 0, ARTF_CUDA_FLUID_WIDTH, fluidRow, fluidTurn);
+        const R g1 = rowAt<kClampRows>(fluid, fluidCount, 0, ARTF_CUDA_FLUID_WIDTH, fluidRow + 1, fluidTurn);
         const R gas = g0 + (g1 - g0) * (fluidPos - fluidFloor);
         density = density * (R(1.f - .1f) + KF(.1) * gas);
         /* dust: less light, more opacity */
         const R dustPos = (inside ? rhoK : R(0)) * R(ARTF_CUDA_DUST_HEIGHT - 1);
-        const int32_t dustRow = truncI(minX(floorR(dustPos), R(ARTF_CUDA_DUST_HEIGHT - 1)));
+        int32_t dustRow;
+        placeOf(dustPos, ARTF_CUDA_DUST_HEIGHT - 1, dustRow);
         inBounds(f.fault, kBoundsDustRow, dustRow, ARTF_CUDA_DUST_HEIGHT);
-        const R dusty = rowAt(map, mapCount, ARTF_CUDA_DUST_AT, ARTF_CUDA_DUST_WIDTH, dustRow, turnK - speed0 * c.time);
+        const R dusty = rowAt<kClampRows>(map, mapCount, ARTF_CUDA_DUST_AT, ARTF_CUDA_DUST_WIDTH, dustRow, turnK - speed0 * c.time);
         const R lit = R(1) - KF(.97) * dusty;
         /* how far from the disc's middle plane, and what the slice stops and gives */
         const R height = t * divR(reach, f.discHeight);
@@ -788,7 +829,7 @@ template <typename R> ARTF_HD R shadeCrossing(const Frame<R>& f, R rhoScale, con
     const R rhoSafe = minX(maxX(rhoCenter, R(0)), R(1));
     const int32_t rowIndex = truncI(rhoSafe * R(ARTF_CUDA_MAP_HEIGHT - 1));
     inBounds(f.fault, kBoundsRingRow, rowIndex, ARTF_CUDA_MAP_HEIGHT);
-    R heat = R(fetch(map, clampI(ARTF_CUDA_ROWS_AT + rowIndex + rowIndex + 1, 0, mapCount - 1)));
+    R heat = R(fetch(map, tableIndex(ARTF_CUDA_ROWS_AT + rowIndex + rowIndex + 1)));
     const R gives = ringGlowAt(f, map, rowIndex);
     R light = f.gain * glow * gives;
     if (f.doppler != R(0)) {

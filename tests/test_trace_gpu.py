@@ -306,6 +306,20 @@ def test_small_frames_are_their_rays(lib, ctx, precision, width, height):
         assert np.array_equal(images[0][..., :3].reshape(-1, 3), rgb)
 
 
+@pytest.mark.parametrize("time", [-7.25, 0.0, 6.0e4, 1.5e30])
+@pytest.mark.parametrize("inner,outer", [(7.0, 7.1), (0.0, 20.0)])
+def test_exact_table_places_match_oracle(lib, ctx, time, inner, outer):
+    """Rings turned back, not at all, by thousands of turns and by so many that no fraction is left, of a narrow
+    disc and a wide one: the places in the tables are the oracle's, bit for bit."""
+    desc = scenes.hole_desc(0.7, inner=inner, outer=outer, time=time)
+    view = scenes.Scene("places", desc, scenes.camera(82.0, 26.0), 97, 53, seed=4)
+    frame, _, clamped = scenes.frame(view)
+    m, fluid = scenes.synth_map(lib, clamped, 4, 3.0), scenes.unit_fluid()
+    g.set_inputs(lib, ctx, m, fluid)
+    hdr, _ = g.trace(lib, ctx, frame, None, capi.EXACT)
+    assert np.array_equal(hdr.view(np.uint32), binding.render32(frame, m, fluid).view(np.uint32))
+
+
 @pytest.mark.parametrize("offset", [0, 1, 2, 4])
 @pytest.mark.parametrize("jitter", [0, 3])
 def test_host_path_at_any_alignment(lib, ctx, offset, jitter):
