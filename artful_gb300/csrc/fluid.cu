@@ -20,8 +20,10 @@
  * needs of its neighbours through shared memory.  What bounds a step is latency: the sum in cell order (1024
  * dependent additions, 1.9 us), three reads in turn of fields that other SMs have just written, and one
  * launch waiting for the last.  One block working through the eddies, and a launch a pass, took 62 us a
- * step; a launch for the velocities and one for the rest of each ring 10.8, this takes 9.7 (24 steps a call:
- * 1486 -> 265 -> 241 us; of that the launches as dependent ones 387 -> 265). */
+ * step; a launch for the velocities and one for the rest of each ring 10.8, one launch 9.7, and with a cell's
+ * two velocities side by side, read together, 9.1 (24 steps a call: 1486 -> 265 -> 241 -> 225 us; of that the
+ * launches as dependent ones 387 -> 265).  Two blocks a SM are as many as a step has: cut for three, the blocks
+ * crowd on fewer SMs and 24 steps take 284. */
 #include "nvtxRange.h"
 #include "artful_cuda.h"
 
@@ -100,17 +102,22 @@ __device__ __forceinline__ float noise(float x, float y, uint32_t period, uint32
     return (lo + (hi - lo) * sy) * (1.f / 16777216.f);
 }
 
-/* fluid.c:82-93 (an index never leaves the field: y0 <= FH - 2, columns wrap) */
-__device__ __forceinline__ float bilinear(const float* a, float x, float y) {
+/* fluid.c:82-93, where it reads: the cell's two columns and two rows, and how far between them (an index
+ * never leaves the field: y0 <= FH - 2, columns wrap). */
+struct Between {
+    uint32_t lo0, lo1; /* of the lower row; the upper's lie FW on */
+    float px, py;
+};
+__device__ __forceinline__ Between betweenOf(float x, float y) {
     const float fy = clampF(y, 0.f, (float)(FH - 1) - .001f);
     const int y0 = (int)fy;
-    const float py = fy - (float)y0;
-    const float fx = floorf(x), px = x - fx;
-    const int x0 = (int)fx & (FW - 1), x1 = (x0 + 1) & (FW - 1);
-    const float* lo = a + (size_t)y0 * FW;
-    const float* hi = lo + FW;
-    const float top = lo[x0] + (lo[x1] - lo[x0]) * px, bottom = hi[x0] + (hi[x1] - hi[x0]) * px;
-    return top + (bottom - top) * py;
+    const float fx = floorf(x);
+    const uint32_t x0 = (uint32_t)(int)fx & (FW - 1), row = (uint32_t)y0 * FW;
+    return {row + x0, row + ((x0 + 1) & (FW - 1)), x - fx, fy - (float)y0};
+}
+__device__ __forceinline__ float bilinear(const Between& b, float lo0, float lo1, float hi0, float hi1) {
+    const float top = lo0 + (lo1 - lo0) * b.px, bottom = hi0 + (hi1 - hi0) * b.px;
+    return top + (bottom - top) * b.py;
 }
 
 /* ---- kernels: one thread a cell, unless said otherwise ------------------------------------------ */
@@ -167,11 +174,11 @@ __device__ __forceinline__ bool eddyAt(const Eddy& q, float r, int i, float& sha
 }
 
 /* What an eddy does to a cell it reaches (fluid.c:215-217): to its velocities, and to its density. */
-__device__ __forceinline__ void stirFlow(const Eddy& q, float r, int i, float& vr, float& w) {
+__device__ __forceinline__ void stirFlow(const Eddy& q, float r, int i, float2& v) {
     float shape, dr, dx;
     if (!eddyAt(q, r, i, shape, dr, dx)) return;
-    vr -= q.strength * shape * dx / q.size;
-    w += q.strength * shape * dr / q.size;
+    v.x -= q.strength * shape * dx / q.size;
+    v.y += q.strength * shape * dr / q.size;
 }
 
 __device__ __forceinline__ void stirDensity(const Eddy& q, float r, int i, float& s) {
@@ -181,59 +188,67 @@ __device__ __forceinline__ void stirDensity(const Eddy& q, float r, int i, float
 
 /* Eddies on their own (a gas's start, and its first step's): a block a ring, so that an eddy out of the
  * ring's reach costs the block one uniform test. */
-__global__ void __launch_bounds__(RING_THREADS) stir(float* s, float* vr, float* w, const Ring* __restrict__ rings,
+__global__ void __launch_bounds__(RING_THREADS) stir(float* s, float2* flow, const Ring* __restrict__ rings,
                                                      const __grid_constant__ Eddies<EDDIES_A_LAUNCH> eddies) {
     const int j = (int)blockIdx.x;
     const float r = rings[j].radius;
     startNext();
     waitBefore();
     for (int i = (int)threadIdx.x; i < FW; i += RING_THREADS) {
-        const size_t at = (size_t)j * FW + (size_t)i;
-        float cellS = s[at], cellR = vr[at], cellW = w[at];
+        const uint32_t at = (uint32_t)(j * FW + i);
+        float cellS = s[at];
+        float2 v = flow[at];
         for (int e = 0; e < eddies.count; ++e) {
-            stirFlow(eddies.e[e], r, i, cellR, cellW);
+            stirFlow(eddies.e[e], r, i, v);
             stirDensity(eddies.e[e], r, i, cellS);
         }
-        s[at] = cellS, vr[at] = cellR, w[at] = cellW;
+        s[at] = cellS, flow[at] = v;
     }
 }
 
-/* fluid.c:96-124: a cell's new velocities */
-__device__ __forceinline__ void velocitiesAt(const float* s, const float* vr, const float* w, const Ring& g, int j, int i,
-                                             float& outR, float& outW) {
-    const int cell = j * FW + i, up = atMost(j + 1, FH - 1), down = atLeast(j - 1, 0);
-    const float x = (float)i - w[cell] * g.toCells, y = (float)j - vr[cell] * g.toRows;
-    const float v0 = bilinear(vr, x, y), w0 = bilinear(w, x, y);
+/* fluid.c:96-124: a cell's new velocities (along the radius, along the orbit) */
+__device__ __forceinline__ float2 velocitiesAt(const float* s, const float2* flow, const Ring& g, int j, int i) {
+    const uint32_t row = (uint32_t)(j * FW), cell = row + (uint32_t)i;
+    const uint32_t up = j < FH - 1 ? cell + FW : cell, down = j > 0 ? cell - FW : cell;
+    const float2 v = flow[cell];
+    const Between b = betweenOf((float)i - v.y * g.toCells, (float)j - v.x * g.toRows);
+    const float2 lo0 = flow[b.lo0], lo1 = flow[b.lo1], hi0 = flow[b.lo0 + FW], hi1 = flow[b.lo1 + FW];
+    const float v0 = bilinear(b, lo0.x, lo1.x, hi0.x, hi1.x), w0 = bilinear(b, lo0.y, lo1.y, hi0.y, hi1.y);
     const float inv = 1.f / s[cell];
-    const float gradR = (s[(size_t)up * FW + i] - s[(size_t)down * FW + i]) * g.invSpan * inv;
-    const float gradPhi = (s[(size_t)j * FW + ((i + 1) & (FW - 1))] - s[(size_t)j * FW + ((i - 1) & (FW - 1))]) *
-                          g.invArc * inv;
+    const float gradR = (s[up] - s[down]) * g.invSpan * inv;
+    const float gradPhi = (s[row + ((i + 1) & (FW - 1))] - s[row + ((i - 1) & (FW - 1))]) * g.invArc * inv;
     const float w1 = w0 + DT * (-g.epicyclic * v0 - v0 * w0 * g.invR - g.sound2 * gradPhi);
     const float v1 = v0 + DT * (2.f * g.angular * w1 + w1 * w1 * g.invR - g.sound2 * gradR);
-    outW = clampF(w1 * g.keep, -.4f, .4f);
-    outR = clampF(v1 * g.keep, -.4f, .4f);
+    return make_float2(clampF(v1 * g.keep, -.4f, .4f), clampF(w1 * g.keep, -.4f, .4f));
 }
 
-/* fluid.c:126-151: a cell's new density, from the old ones and the new velocities: its ring's (vr, w), and
- * the radial ones of the rings above and below at its column. */
-__device__ __forceinline__ float densityAt(const float* s, const float* vr, const float* w, float vrUp, float vrDown,
-                                           const Ring& g, int j, int i) {
+/* fluid.c:126-151: a cell's new density, from the old ones and the new velocities: its ring's, and the radial
+ * ones of the rings above and below at its column. */
+__device__ __forceinline__ float densityAt(const float* s, const float2* flow, float vrUp, float vrDown, const Ring& g, int j,
+                                           int i) {
     const float drift = -.004f;
-    const float x = (float)i - w[i] * g.toCells, y = (float)j - (vr[i] + drift) * g.toRows;
-    const float moved = bilinear(s, x, y);
+    const float2 v = flow[i];
+    const Between b = betweenOf((float)i - v.y * g.toCells, (float)j - (v.x + drift) * g.toRows);
+    const float moved = bilinear(b, s[b.lo0], s[b.lo1], s[b.lo0 + FW], s[b.lo1 + FW]);
     const float spread = (g.up * vrUp - g.down * vrDown) * g.invSpan * g.invR +
-                         (w[(i + 1) & (FW - 1)] - w[(i - 1) & (FW - 1)]) * g.invArc;
+                         (flow[(i + 1) & (FW - 1)].y - flow[(i - 1) & (FW - 1)].y) * g.invArc;
     const float next = moved * (1.f - DT * clampF(spread, -2.f, 2.f));
     return clampF(next + (1.f - next) * g.refill, .03f, 8.f);
 }
 
 /* fluid.c:153-173: a ring moved along itself by its orbit, a Catmull-Rom cubic held within its two middle
  * neighbours */
+__device__ __forceinline__ float slide(float p0, float p1, float p2, float p3, const Ring& g) {
+    return clampF(g.k0 * p0 + g.k1 * p1 + g.k2 * p2 + g.k3 * p3, lesser(p1, p2), greater(p1, p2));
+}
 __device__ __forceinline__ float slideCell(const float* in, int i, const Ring& g) {
     const int at = i + g.shift;
-    const float p0 = in[(at - 1) & (FW - 1)], p1 = in[at & (FW - 1)];
-    const float p2 = in[(at + 1) & (FW - 1)], p3 = in[(at + 2) & (FW - 1)];
-    return clampF(g.k0 * p0 + g.k1 * p1 + g.k2 * p2 + g.k3 * p3, lesser(p1, p2), greater(p1, p2));
+    return slide(in[(at - 1) & (FW - 1)], in[at & (FW - 1)], in[(at + 1) & (FW - 1)], in[(at + 2) & (FW - 1)], g);
+}
+__device__ __forceinline__ float2 slideCell(const float2* in, int i, const Ring& g) {
+    const int at = i + g.shift;
+    const float2 p0 = in[(at - 1) & (FW - 1)], p1 = in[at & (FW - 1)], p2 = in[(at + 1) & (FW - 1)], p3 = in[(at + 2) & (FW - 1)];
+    return make_float2(slide(p0.x, p1.x, p2.x, p3.x, g), slide(p0.y, p1.y, p2.y, p3.y, g));
 }
 
 /* A step: a block a ring, clusters of RINGS neighbouring rings.  Each block finds its ring's new velocities
@@ -244,18 +259,20 @@ __device__ __forceinline__ float slideCell(const float* in, int i, const Ring& g
  * velocities), the next step's eddies, and, when `field` is given, what shows of the ring
  * (fluid.c:175-186).  The fields are read from one copy and written to the other. */
 __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 32)
-    gasStep(const float* s, const float* vr, const float* w, float* outS, float* outR, float* outW,
-            const Ring* __restrict__ rings, float* field, const __grid_constant__ Eddies<EDDIES_A_STEP> eddies) {
+    gasStep(const float* s, const float2* flow, float* outS, float2* outFlow, const Ring* __restrict__ rings,
+            float* field, const __grid_constant__ Eddies<EDDIES_A_STEP> eddies) {
     constexpr int CELLS = FW / RING_THREADS, SHARE = FW / RINGS;
-    __shared__ __align__(16) float ringS[FW];
-    __shared__ float ringR[FW], ringW[FW], outer[FW]; /* outer: of the ring beyond, in the first and last block */
+    __shared__ __align__(16) float slidRing[FW];
+    __shared__ float ringS[FW];
+    __shared__ float2 ringFlow[FW];
+    __shared__ float outer[FW];   /* the radial velocities of the ring beyond, in the first and last block */
     __shared__ uint32_t reaching; /* the eddies that reach the ring at all, a bit each */
     __shared__ float scale;
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int tid = (int)threadIdx.x, j = (int)blockIdx.x, rank = j % RINGS;
     const bool helper = tid >= RING_THREADS;
     const Ring g = rings[j];
-    const size_t row = (size_t)j * FW;
+    const uint32_t row = (uint32_t)(j * FW);
     if (helper) {
         const int e = tid - RING_THREADS;
         const float dr = e < eddies.count ? g.radius - eddies.e[e & (EDDIES_A_STEP - 1)].r0 : 0.f;
@@ -269,50 +286,45 @@ __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 3
 #pragma unroll
         for (int c = 0; c < CELLS; ++c) {
             const int i = tid + c * RING_THREADS;
-            velocitiesAt(s, vr, w, g, j, i, ringR[i], ringW[i]);
+            ringFlow[i] = velocitiesAt(s, flow, g, j, i);
         }
         /* this block's share of the rings below and above the cluster, where there are any (found whole by the
          * outer blocks they cost 1.3 us a step) */
         if (tid < 2 * SHARE) {
             const bool below = tid < SHARE;
             const int beyond = j - rank + (below ? -1 : RINGS), i = rank * SHARE + (below ? tid : tid - SHARE);
-            if (beyond >= 0 && beyond < FH) {
-                float unused;
-                velocitiesAt(s, vr, w, rings[beyond], beyond, i, cluster.map_shared_rank(outer, below ? 0 : RINGS - 1)[i],
-                             unused);
-            }
+            if (beyond >= 0 && beyond < FH)
+                cluster.map_shared_rank(outer, below ? 0 : RINGS - 1)[i] = velocitiesAt(s, flow, rings[beyond], beyond, i).x;
         }
     }
     cluster.sync();
     if (!helper) {
         /* (the first and last ring border on themselves) */
-        const float* below = rank > 0 ? cluster.map_shared_rank(ringR, rank - 1) : j > 0 ? outer : ringR;
-        const float* above = rank < RINGS - 1 ? cluster.map_shared_rank(ringR, rank + 1) : j < FH - 1 ? outer : ringR;
+        const bool outBelow = rank == 0 && j > 0, outAbove = rank == RINGS - 1 && j < FH - 1;
+        const float* below = outBelow ? outer : &cluster.map_shared_rank(ringFlow, rank > 0 ? rank - 1 : rank)->x;
+        const float* above = outAbove ? outer : &cluster.map_shared_rank(ringFlow, rank < RINGS - 1 ? rank + 1 : rank)->x;
+        const int stepBelow = outBelow ? 1 : 2, stepAbove = outAbove ? 1 : 2;
 #pragma unroll
         for (int c = 0; c < CELLS; ++c) {
             const int i = tid + c * RING_THREADS;
-            ringS[i] = densityAt(s, ringR, ringW, above[i], below[i], g, j, i);
+            ringS[i] = densityAt(s, ringFlow, above[i * stepAbove], below[i * stepBelow], g, j, i);
         }
     }
-    /* (no block leaves while a neighbour may read its ring: waited for at the end) */
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     __syncthreads();
-    float slidS[CELLS], slidR[CELLS], slidW[CELLS];
+    /* (no block leaves while a neighbour may read its ring: waited for at the end; nothing is handed over) */
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    float slidS[CELLS];
     if (!helper) {
 #pragma unroll
-        for (int c = 0; c < CELLS; ++c) slidS[c] = slideCell(ringS, tid + c * RING_THREADS, g);
-    }
-    __syncthreads();
-    if (!helper) {
-#pragma unroll
-        for (int c = 0; c < CELLS; ++c) ringS[tid + c * RING_THREADS] = slidS[c];
+        for (int c = 0; c < CELLS; ++c)
+            slidRing[tid + c * RING_THREADS] = slidS[c] = slideCell(ringS, tid + c * RING_THREADS, g);
     }
     __syncthreads();
     if (helper) {
         if (tid == RING_THREADS) {
             float sum = 0;
-            const float4* four = reinterpret_cast<const float4*>(ringS);
-#pragma unroll 16
+            const float4* four = reinterpret_cast<const float4*>(slidRing);
+#pragma unroll 32
             for (int i = 0; i < FW / 4; ++i) {
                 const float4 q = four[i];
                 sum += q.x;
@@ -333,16 +345,15 @@ __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 3
 #pragma unroll
     for (int c = 0; c < CELLS; ++c) {
         const int i = tid + c * RING_THREADS;
-        slidR[c] = slideCell(ringR, i, g);
-        slidW[c] = slideCell(ringW, i, g);
+        float2 v = slideCell(ringFlow, i, g);
         near[c] = 0;
         for (uint32_t bits = reaching; bits; bits &= bits - 1) {
             const Eddy& q = eddies.e[__ffs((int)bits) - 1];
             if (((i - q.i0 + q.reach) & (FW - 1)) <= 2 * q.reach) near[c] |= bits & (0u - bits);
         }
         for (uint32_t bits = near[c]; bits; bits &= bits - 1)
-            stirFlow(eddies.e[__ffs((int)bits) - 1], g.radius, i, slidR[c], slidW[c]);
-        outR[row + i] = slidR[c], outW[row + i] = slidW[c];
+            stirFlow(eddies.e[__ffs((int)bits) - 1], g.radius, i, v);
+        outFlow[row + i] = v;
     }
     __syncthreads();
 #pragma unroll
@@ -369,8 +380,7 @@ struct ArtfCudaFluid {
     float inner, outer;
     float* block;          /* the seven fields and the rings' terms, one allocation */
     float* dens[2];
-    float* radial[2];
-    float* orbital[2];
+    float2* flow[2];       /* velocities along the radius and the orbit, side by side: read together */
     float* field;
     int cur;               /* which copy of the three fields is the current one */
     Ring* rings;           /* device copy */
@@ -495,7 +505,7 @@ int stirStart(ArtfCudaFluid* f) {
         q.count = 0;
         drawEddies(f, q, atMost(left, EDDIES_A_LAUNCH), 0);
         if (left < EDDIES_A_LAUNCH) drawEddies(f, q, 2, EDDIES_A_STEP - 2);
-        e = follow(f, stir, FH, RING_THREADS, f->dens[f->cur], f->radial[f->cur], f->orbital[f->cur], f->rings, q);
+        e = follow(f, stir, FH, RING_THREADS, f->dens[f->cur], f->flow[f->cur], f->rings, q);
     }
     if (e != cudaSuccess) return artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
     return ARTF_CUDA_OK;
@@ -511,8 +521,8 @@ int advanceSteps(ArtfCudaFluid* f, int64_t steps) {
         const int from = f->cur, to = f->cur ^ 1;
         q.count = 0;
         drawEddies(f, q, 2, EDDIES_A_STEP - 2);
-        e = follow(f, gasStep, FH, RING_THREADS + 32, f->dens[from], f->radial[from], f->orbital[from], f->dens[to],
-                   f->radial[to], f->orbital[to], f->rings, k == steps - 1 ? f->field : (float*)nullptr, q);
+        e = follow(f, gasStep, FH, RING_THREADS + 32, f->dens[from], f->flow[from], f->dens[to], f->flow[to],
+                   f->rings, k == steps - 1 ? f->field : (float*)nullptr, q);
         f->cur = to;
     }
     if (e != cudaSuccess) return artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
@@ -553,8 +563,7 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
         return artf::failWith(ARTF_CUDA_ENOMEM, "fluid: device allocation");
     }
     for (int k = 0; k < 2; ++k)
-        f->dens[k] = f->block + FIELD * (3 * k), f->radial[k] = f->block + FIELD * (3 * k + 1),
-        f->orbital[k] = f->block + FIELD * (3 * k + 2);
+        f->dens[k] = f->block + FIELD * (3 * k), f->flow[k] = (float2*)(f->block + FIELD * (3 * k + 1));
     f->field = f->block + FIELD * 6;
     f->rings = (Ring*)(f->block + FIELD * 7);
     /* the rings (fluid.c:270-290), on the host in float as the reference has them */
@@ -585,8 +594,8 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
         g.toRows = DT / ((g.up - g.down) * (j == 0 || j == FH - 1 ? 1.f : .5f));
     }
     cudaError_t e = cudaMemcpyAsync(f->rings, f->host, sizeof f->host, cudaMemcpyHostToDevice, stream);
-    /* (at rest: the two velocities lie together; the rest is written before it is read) */
-    if (e == cudaSuccess) e = cudaMemsetAsync(f->radial[0], 0, sizeof(float) * FIELD * 2, stream);
+    /* (at rest; the rest is written before it is read) */
+    if (e == cudaSuccess) e = cudaMemsetAsync(f->flow[0], 0, sizeof(float2) * FIELD, stream);
     if (e == cudaSuccess) {
         seedDensity<<<(FIELD + 255) / 256, 256, 0, stream>>>(f->dens[0], f->rings);
         e = cudaGetLastError();
