@@ -289,16 +289,12 @@ static artf::TraceLaunch launchOf(const ArtfCuda* ctx, const ArtfCudaTraceOption
     l.stepScale = o->stepScale > 0.f ? o->stepScale : 1.f;
     l.horizonBand = o->horizonBand;
     l.blockSize = o->blockSize;
-    l.compactEvery = o->compactEvery;
     l.persistent = o->persistent;
     l.guards = o->guards;
-    l.fp64Batch = o->fp64Batch;
     l.refillBatch = o->refillBatch;
     l.order = o->order;
     if (ctx->hasTuning && o->precision == ARTF_CUDA_MIXED) {
         if (!l.blockSize) l.blockSize = ctx->tuned.blockSize;
-        if (!l.compactEvery) l.compactEvery = ctx->tuned.compactEvery;
-        if (!l.fp64Batch) l.fp64Batch = ctx->tuned.fp64Batch;
         if (!l.refillBatch) l.refillBatch = ctx->tuned.refillBatch;
     }
     l.counters = ctx->counters;

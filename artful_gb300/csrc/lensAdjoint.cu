@@ -22,8 +22,8 @@
  * derivative (which texel or star cell, the 0.004 opacity cut-off, the step cap) contribute none: the
  * pathwise derivative.
  *
- * Work layout: a view table in device memory; grid (blocks of four 8 x 4 tiles, views), the tiles of a
- * view heaviest first, each block copying its view's entry to shared memory, each warp tracing one tile.
+ * Work layout: a view table in device memory; grid (blocks of four 8 x 4 tiles, views), in the reverse
+ * kernel the tiles of a view heaviest first, each block copying its view's entry to shared memory, each warp tracing one tile.
  * Each tile's six sums go to the tile's own slot; a last kernel adds them in a fixed order, in double, so
  * the result does not depend on scheduling. */
 #define ARTF_CLAMP_ROWS 1 /* table rows read the plain way (lensCore.cuh: placeOf) */

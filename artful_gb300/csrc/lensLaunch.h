@@ -29,10 +29,8 @@ struct TraceLaunch {
     float stepScale;
     float horizonBand;
     int blockSize;
-    int compactEvery;
     int persistent;
     uint32_t guards;
-    int fp64Batch;
     int refillBatch;
     int order;                    /* ARTF_CUDA_ORDER_* (the mixed trace's queue) */
     int smCount;

@@ -31,8 +31,8 @@
  * one another, so a wide step serves most of a warp at a time, and a ray's step costs nothing for the
  * schedule's sake.  (Lanes that waited for full rounds of wide steps and were refilled one by one, as an
  * FP64 wide step wanted, paid 80 thread instructions a step in votes and flags: 2.15 against 1.61 ms for the
- * 1080p x 4 frame, 7.63 against 5.51 for 64 views.)  What a step costs is issue slots (71 % of them used, FMA
- * pipe 50 % busy), so the FP32 step runs its coordinates in pairs with packed instructions (nystromStep: 1.86
+ * 1080p x 4 frame, 7.63 against 5.51 for 64 views.)  What a step costs is issue slots (76 % of them used, FMA
+ * pipe 55 % busy), so the FP32 step runs its coordinates in pairs with packed instructions (nystromStep: 1.86
  * -> 1.76 ms), the wide step is one code path (1.74 -> 1.61 with the counts out of registers) and each float
  * rounding is written out or pinned (ARTF_PINNED_FMA): whatever registers a kernel is given, its images are
  * the same bits.  A frame of fewer rays than the GPU's warps could take is bound by its longest ray's
@@ -47,7 +47,6 @@
 
 namespace artf {
 
-/* A view as the kernel reads it, from the device view table. */
 /* A value as the unevaluated sum hi + lo of two floats, |lo| at most half an ulp of hi: Dekker's
  * double-length arithmetic (1971), about 48 significant bits from FP32 instructions, which this GPU
  * issues 64 times as fast as FP64 ones. */
@@ -61,6 +60,7 @@ struct MotionTermsFf {
     Ff forward[3], right[3], up[3], metric[4], rho, a, a2, mu0Squared, minusTwoA2;
 };
 
+/* A view as the kernels read it, from the device view table or as a parameter. */
 struct MixedView {
     Frame<float> f;
     Frame<double> d;
@@ -70,7 +70,7 @@ struct MixedView {
     float4* hdr;
     ArtfCudaRayEnd* ends;
     /* Rays of the view's pixels, plane k for ray k (radiance, class bits), or NULL.  With planes, a work
-     * unit is one ray and mixedCombine sums each pixel's rays afterwards; without, a unit is a pixel
+     * unit is one ray and combinePlanes sums each pixel's rays afterwards; without, a unit is a pixel
      * whose rays one lane traces in turn. */
     float4* rayOut;
     double wideA2;            /* a^2 in double, for the horizon band's FP64 sub-step */

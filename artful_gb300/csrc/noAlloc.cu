@@ -108,9 +108,7 @@ extern "C" int artfCudaHoleBatchNoAlloc(const ArtfCudaView* views, int count, co
     l.stepScale = options->stepScale > 0.f ? options->stepScale : 1.f;
     l.horizonBand = options->horizonBand;
     l.blockSize = options->blockSize;
-    l.compactEvery = options->compactEvery;
     l.guards = options->guards;
-    l.fp64Batch = options->fp64Batch;
     l.refillBatch = options->refillBatch;
     l.counters = (unsigned long long*)scratch;
     l.smCount = sms;

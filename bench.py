@@ -44,9 +44,9 @@ WORKLOAD = "kerr-hole 1920x1080, 4 jittered rays/px, a=0.998, r_obs=50 M, i=85 d
 # Kernels one mixed frame launches: the tile probe, the heavy-first order, the trace, the ray-plane sum.
 LAUNCHES_PER_MIXED_FRAME = 4
 # DRAM bytes (read + write) of one launch of the mixed trace kernel at this workload, from one ncu
-# capture (dram__bytes_read.sum 17.23 MB + dram__bytes_write.sum 73.95 MB): the map read once, and the
+# capture (dram__bytes_read.sum 16.56 MB + dram__bytes_write.sum 73.54 MB): the map read once, and the
 # part of the 133 MB of ray planes that leaves L2 before the sum reads it back.
-TRACE_TRAFFIC_BYTES = 91_173_120
+TRACE_TRAFFIC_BYTES = 90_104_576
 TRACE_TRAFFIC_GEODESICS = 1920 * 1080 * 4
 FLOPS_WIDE_RADIAL = 61  # lensFlops.h: a whole radial sub-step in the horizon's band (spin != 0)
 # How busy the mixed trace keeps its pipes, from one ncu --set full capture of its kernel at 960x540 x 4
@@ -56,10 +56,10 @@ FLOPS_WIDE_RADIAL = 61  # lensFlops.h: a whole radial sub-step in the horizon's 
 MIXED_PIPES_BUSY = {"fp64": 0.035, "fp32_fma": 0.398, "alu": 0.370, "issue": 0.690,
                     "source": "ncu sm__inst_executed_pipe_fp64, sm__pipe_fma_cycles_active, sm__inst_executed_pipe_alu, "
                               "smsp__issue_active "
-                              "of traceMixedQueueOneAll at 960x540 x 4"}
+                              "of traceMixedOneAll at 960x540 x 4"}
 TRACE_TRAFFIC_SOURCE = "ncu dram__bytes of one launch of the mixed trace kernel at 1920x1080 x 4 jittered rays"
 # The adjoint's checkpoint interval: 32, a ray's state kept every 32 steps and each segment recomputed in
-# the reverse pass; 1, every state kept (48 bytes a step) and nothing recomputed.
+# the reverse pass; 1, every state kept (48 bytes a step, 32 of them written at most steps) and nothing recomputed.
 ADJOINT_CHECKPOINT = 1
 
 
@@ -268,9 +268,8 @@ def sweep(args):
         e = np.frombuffer(ends.cpu().numpy().tobytes(), END_DTYPE).copy() if with_ends else None
         return s, (statistics.median(times) if times else s.ms), e, hdr.cpu().numpy().copy()
 
-    def o(precision, scale=1.0, guards=0, band=0.0, batch=0, wait=0, refill=0, block=0):
-        return capi.TraceOptions(precision, rays, scene.jitter_seed, scale, band, block, wait, 1, guards, batch,
-                                 refill)
+    def o(precision, scale=1.0, guards=0, band=0.0, refill=0, block=0):
+        return capi.TraceOptions(precision, rays, scene.jitter_seed, scale, band, block, 0, 1, guards, 0, refill)
 
     _, ms64, e64, img64 = run(o(capi.FP64), True, 2)
     _, _, e64h, img64h = run(o(capi.FP64, 0.5), True, 0)
@@ -281,16 +280,11 @@ def sweep(args):
                       "vs_fp64_half": endpoint_error(e32, e64h, img32, img64h)}), flush=True)
     G = capi
     variants = [
-        ("defaults: all guards, band 0.95, batch 32, refill 32, wait 256, block 128", dict()),
+        ("defaults: all guards, band 0.95, up to 32 rays a warp, block 128", dict()),
         ("band 0.8", dict(band=0.8)),
         ("band 0.99", dict(band=0.99)),
-        ("batch 16", dict(batch=16)),
-        ("batch 24", dict(batch=24)),
-        ("refill 8", dict(refill=8)),
-        ("refill 24", dict(refill=24)),
-        ("refill 32", dict(refill=32)),
-        ("wait 16", dict(wait=16)),
-        ("wait 256", dict(wait=256)),
+        ("8 rays a warp", dict(refill=8)),
+        ("16 rays a warp", dict(refill=16)),
         ("block 64", dict(block=64)),
         ("block 256", dict(block=256)),
         ("motion + psi only", dict(guards=G.GUARD_MOTION | G.GUARD_PSI)),
