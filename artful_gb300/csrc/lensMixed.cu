@@ -99,6 +99,11 @@ struct MixedParams {
     float stepScale;
     int maxSteps;
     int lanesLog2;    /* a warp's rays at a time: 2^lanesLog2 of its lanes */
+    int cornersLog2;  /* the probe's rays a tile: 1, or one at each corner */
+    /* the order's slots a weight class; of the heavy classes' slots (its first), mostHeavy at most, a warp takes
+     * eight rays at a time (the kernels that split) */
+    const unsigned* classes;
+    int mostHeavy;
     uint32_t guards;  /* ARTF_CUDA_GUARD_* */
 };
 
@@ -499,10 +504,18 @@ __device__ __forceinline__ int viewOf(const MixedParams& p, int unit) {
  * step count of one FP32 ray through its middle, stepped without shading (the disc is thin: it seldom
  * ends a ray) up to 64 steps (a sky ray takes about 25; what goes on longer is heavy); tiles are
  * counting-sorted by weight class, heaviest first.  The order changes when a ray is traced, never what
- * it computes, so the frame is the same bits in any order. */
+ * it computes, so the frame is the same bits in any order.
+ *
+ * A frame of few slots a resident warp is bound by its heavy tiles alone: a warp of 32 rays that part ways
+ * runs all they need one after another, some 100 us of a 512 x 288 frame's 126.  There the heavy tiles come
+ * apart, eight rays a warp, and each tile's weight is the most steps of its four corners' rays: the photon
+ * ring is thinner than a tile, and one ray misses tiles whose long rays then start last.  Every heavy tile
+ * costs more warps so; with the frame's size it gains less, and at six slots a warp nothing (mixedGrid). */
 
 constexpr int kWeightClasses = 9; /* steps / 8 up to 64: the probe stops there (all heavier tiles, class 8) */
 constexpr int kProbeSteps = 64;
+constexpr int kHeavyClass = 5; /* 40 steps or more at a corner */
+constexpr int kHeavyRaysLog2 = 3, kCornersLog2 = 2;
 
 /* The view a batch-wide tile belongs to: the last whose first tile is at or below it. */
 __device__ __forceinline__ int tileView(const MixedParams& p, int tile) {
@@ -523,12 +536,16 @@ __device__ __forceinline__ void probeTiles(const MixedParams& p, const MixedView
     __shared__ unsigned counts[kWeightClasses];
     if (threadIdx.x < kWeightClasses) counts[threadIdx.x] = 0;
     __syncthreads();
-    const int g = (int)(blockIdx.x * 128 + threadIdx.x);
+    const int at = (int)(blockIdx.x * 128 + threadIdx.x), g = at >> p.cornersLog2;
+    const int corner = at & ((1 << p.cornersLog2) - 1);
+    int w = 0;
+    unsigned planes = 0;
     if (g < totalTiles) {
         const MixedView& v = kOne ? *one : p.views[tileView(p, g)];
         const int tile = g - v.tileBase;
-        const int x = min((tile % v.tilesX) * 8 + 4, (int)v.f.width - 1);
-        const int y = min(v.rowBegin + (tile / v.tilesX) * 4 + 2, v.rowBegin + v.rows - 1);
+        const int dx = p.cornersLog2 ? (corner & 1) * 7 : 4, dy = p.cornersLog2 ? (corner >> 1) * 3 : 2;
+        const int x = min((tile % v.tilesX) * 8 + dx, (int)v.f.width - 1);
+        const int y = min(v.rowBegin + (tile / v.tilesX) * 4 + dy, v.rowBegin + v.rows - 1);
         float nx, ny, moment;
         samplePosition(v.h, v.jitter, v.seed, x, y, 0, &nx, &ny, &moment);
         RayConst<float> c;
@@ -545,9 +562,13 @@ __device__ __forceinline__ void probeTiles(const MixedParams& p, const MixedView
             if (0.f > o.next.u || o.next.u > v.f.uHorizon) break;
             s = o.next;
         }
-        const int w = min(i >> 3, kWeightClasses - 1);
+        w = min(i >> 3, kWeightClasses - 1);
+        planes = v.rayOut ? (unsigned)v.rays : 1u;
+    }
+    for (int off = 1; off < 1 << p.cornersLog2; off <<= 1) w = max(w, __shfl_xor_sync(0xFFFFFFFFu, w, off));
+    if (g < totalTiles && corner == 0) {
         weights[g] = w;
-        atomicAdd(counts + w, v.rayOut ? (unsigned)v.rays : 1u);
+        atomicAdd(counts + w, planes);
     }
     __syncthreads();
     if (threadIdx.x < kWeightClasses && counts[threadIdx.x]) atomicAdd(classes + threadIdx.x, counts[threadIdx.x]);
@@ -606,21 +627,31 @@ __global__ void __launch_bounds__(128) placeOne(const MixedParams p, const __gri
 
 /* The persistent trace: each warp takes slots from the queue, one ray plane of one 8 x 4 tile of pixels a
  * slot, and traces a slot's 32 rays together.  kOne: a single view, read from `one` (a kernel parameter)
- * rather than from the view table. */
-template <bool kOne, bool kAll>
+ * rather than from the view table.  kSplit: the heavy slots in parts of eight rays (kernels of their own: the
+ * test in the loop costs a large frame 1 %). */
+template <bool kOne, bool kAll, bool kSplit = false>
 __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView* one) {
     __shared__ unsigned tally[kMixedCount][256];
     const int lane = threadIdx.x & 31;
     unsigned rounds = 0;
     clearMixed(tally);
-    const unsigned parts = (unsigned)(p.totalUnits >> p.lanesLog2); /* 2^lanesLog2 rays each */
+    unsigned heavy = 0; /* the rays in heavy slots */
+    if (kSplit) {
+        for (int c = kHeavyClass; c < kWeightClasses; ++c) heavy += __ldg(p.classes + c);
+        heavy = min(heavy, (unsigned)p.mostHeavy) << 5;
+    }
+    const unsigned heavyParts = heavy >> kHeavyRaysLog2;
+    const unsigned parts = heavyParts + (((unsigned)p.totalUnits - heavy) >> p.lanesLog2); /* 2^lanesLog2 rays each */
     for (;;) {
         unsigned part = 0;
         if (lane == 0) part = (unsigned)atomicAdd(p.counters + CQueue, 1ull);
         part = __shfl_sync(0xFFFFFFFFu, part, 0);
         if (part >= parts) break;
         /* (a tile's rays row by row: 8 x 4 pixels a part, 8 x 2, 8 x 1, 4 x 1 or 2 x 1) */
-        const unsigned first = part << p.lanesLog2, within = (first & 31u) + (unsigned)lane;
+        const bool split = kSplit && part < heavyParts;
+        const int lanesLog2 = split ? kHeavyRaysLog2 : p.lanesLog2;
+        const unsigned first = split ? part << lanesLog2 : heavy + ((part - heavyParts) << lanesLog2);
+        const unsigned within = (first & 31u) + (unsigned)lane;
         const int slot = (int)(first >> 5);
         const MixedView* v = kOne ? one : p.views;
         int plane, tile;
@@ -639,7 +670,7 @@ __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView
         }
         const int x = (tile % v->tilesX) * 8 + (int)(within & 7u);
         const int y = v->rowBegin + (tile / v->tilesX) * 4 + (int)(within >> 3);
-        if (lane >> p.lanesLog2 == 0 && x < v->f.width && y < v->rowBegin + v->rows) {
+        if (lane >> lanesLog2 == 0 && x < v->f.width && y < v->rowBegin + v->rows) {
             const size_t index = (size_t)y * (size_t)v->f.width + (size_t)x;
             const int64_t pixels = (int64_t)v->f.width * v->f.height;
             float sum[3] = {0.f, 0.f, 0.f};
@@ -676,6 +707,7 @@ __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView
  * their bits agree): its dead branches fold away and its code is smaller. */
 __global__ void __launch_bounds__(256, 2) traceMixedTable(const MixedParams p) { mixedTiles<false, false>(p, nullptr); }
 __global__ void __launch_bounds__(256, 2) traceMixedTableAll(const MixedParams p) { mixedTiles<false, true>(p, nullptr); }
+__global__ void __launch_bounds__(256, 2) traceMixedTableSplit(const MixedParams p) { mixedTiles<false, true, true>(p, nullptr); }
 
 /* A single view (a frame) as a kernel parameter: its fields are then read from the constant bank where
  * they are used, not loaded from the view table in global memory at every step. */
@@ -684,6 +716,9 @@ __global__ void __launch_bounds__(256, 2) traceMixedOne(const MixedParams p, con
 }
 __global__ void __launch_bounds__(256, 2) traceMixedOneAll(const MixedParams p, const __grid_constant__ MixedView view) {
     mixedTiles<true, true>(p, &view);
+}
+__global__ void __launch_bounds__(256, 2) traceMixedOneSplit(const MixedParams p, const __grid_constant__ MixedView view) {
+    mixedTiles<true, true, true>(p, &view);
 }
 
 /* Each pixel of the views with ray planes: its rays' radiance summed in ray order and scaled by
@@ -735,6 +770,8 @@ MixedParams paramsOf(const TraceLaunch& l, const void* deviceTable, int viewCoun
     p.maxSteps = l.stepScale < .75f ? 384 : 192;
     p.guards = l.guards ? l.guards : ARTF_CUDA_GUARD_ALL;
     p.order = nullptr;
+    p.classes = nullptr;
+    p.cornersLog2 = p.mostHeavy = 0;
     return p;
 }
 
@@ -862,10 +899,16 @@ size_t mixedOrderBytes(int totalTiles, int totalUnits) {
  * warps share the rays and each has fewer that part ways (a warp runs what any of its rays needs, and
  * rays of a small frame's neighbouring pixels part early: a 101 x 67 frame took 119 us by 32 rays, 84 by
  * 8, 80 by 4 or 2; at 1920 x 1080 a warp's 32 rays stay together, 30.2 of 32 lanes busy).  refillBatch
- * sets the most. */
+ * sets the most.
+ * Heavy slots are split where warps take whole slots of 32, the fewer the more slots there are: a quarter of
+ * the warps' number at three slots a warp, none from six on (us, whole slots against split: 320 x 180 99 and
+ * 79, 384 x 216 104 and 80, 512 x 288 126 and 101, 640 x 360 114 and 97, 320 x 180 x 4 rays 155 and 115, 768 x
+ * 432 180 and 156; at 960 x 540, 6.7 slots a warp, 143 and 150; at 1280 x 720, 11.8, splitting 304 slots 181
+ * and 188). */
 struct MixedGrid {
-    int blocks, lanesLog2;
+    int blocks, most, lanesLog2; /* the launch's blocks, and as many as are resident at once */
     bool resident; /* every part has a warp at once: the order they start in makes no difference */
+    int mostHeavy; /* the heavy slots that are split at most, for a trace that orders its slots */
 };
 
 static MixedGrid mixedGrid(const TraceLaunch& l, int totalUnits, const void* kernel) {
@@ -878,7 +921,10 @@ static MixedGrid mixedGrid(const TraceLaunch& l, int totalUnits, const void* ker
     while (l.refillBatch > 0 && 1 << g.lanesLog2 > l.refillBatch) --g.lanesLog2;
     while (g.lanesLog2 > 1 && (long long)(totalUnits >> g.lanesLog2) * 2 <= warps) --g.lanesLog2;
     const long long parts = totalUnits >> g.lanesLog2, needed = (parts * 32 + block - 1) / block;
+    const long long slots = totalUnits >> 5, room = (6 * warps - slots) / 12;
+    g.mostHeavy = room > 0 && g.lanesLog2 == 5 ? (int)room : 0;
     g.resident = parts <= warps;
+    g.most = (int)grid;
     g.blocks = (int)(grid > needed ? needed : grid);
     if (g.blocks < 1) g.blocks = 1;
     return g;
@@ -899,9 +945,11 @@ cudaError_t launchMixedTable(const TraceLaunch& l, const void* deviceTable, int 
     }
     const void* kernel = single ? (all ? (const void*)traceMixedOneAll : (const void*)traceMixedOne)
                                 : (all ? (const void*)traceMixedTableAll : (const void*)traceMixedTable);
-    const MixedGrid grid = mixedGrid(l, totalUnits, kernel);
+    MixedGrid grid = mixedGrid(l, totalUnits, kernel);
     p.lanesLog2 = grid.lanesLog2;
-    if (orderScratch && l.order == ARTF_CUDA_ORDER_HEAVY_FIRST && totalTiles > 0 && !grid.resident) {
+    const bool ordered = orderScratch && l.order == ARTF_CUDA_ORDER_HEAVY_FIRST && totalTiles > 0;
+    const bool split = ordered && all && grid.mostHeavy > 0;
+    if (ordered && (split || !grid.resident)) {
         unsigned* classes = (unsigned*)orderScratch;
         unsigned* cursors = classes + 32;
         int* weights = (int*)((char*)orderScratch + kOrderHead);
@@ -909,20 +957,29 @@ cudaError_t launchMixedTable(const TraceLaunch& l, const void* deviceTable, int 
         const cudaError_t e = cudaMemsetAsync(orderScratch, 0, kOrderHead, l.stream);
         if (e != cudaSuccess) return e;
         const unsigned tiles = (unsigned)((totalTiles + 127) / 128);
+        if (split) {
+            p.classes = classes;
+            p.mostHeavy = grid.mostHeavy;
+            p.cornersLog2 = kCornersLog2;
+            grid.blocks = grid.most;
+        }
+        const unsigned probes = (unsigned)((((long long)totalTiles << p.cornersLog2) + 127) / 128);
         if (single) {
-            probeOne<<<tiles, 128, 0, l.stream>>>(p, one, totalTiles, weights, classes);
+            probeOne<<<probes, 128, 0, l.stream>>>(p, one, totalTiles, weights, classes);
             placeOne<<<tiles, 128, 0, l.stream>>>(p, one, totalTiles, weights, classes, cursors, order);
         } else {
-            probeTable<<<tiles, 128, 0, l.stream>>>(p, totalTiles, weights, classes);
+            probeTable<<<probes, 128, 0, l.stream>>>(p, totalTiles, weights, classes);
             placeTable<<<tiles, 128, 0, l.stream>>>(p, totalTiles, weights, classes, cursors, order);
         }
         p.order = order;
     }
     if (single) {
-        if (all) traceMixedOneAll<<<grid.blocks, block, 0, l.stream>>>(p, one);
+        if (split) traceMixedOneSplit<<<grid.blocks, block, 0, l.stream>>>(p, one);
+        else if (all) traceMixedOneAll<<<grid.blocks, block, 0, l.stream>>>(p, one);
         else traceMixedOne<<<grid.blocks, block, 0, l.stream>>>(p, one);
     } else {
-        if (all) traceMixedTableAll<<<grid.blocks, block, 0, l.stream>>>(p);
+        if (split) traceMixedTableSplit<<<grid.blocks, block, 0, l.stream>>>(p);
+        else if (all) traceMixedTableAll<<<grid.blocks, block, 0, l.stream>>>(p);
         else traceMixedTable<<<grid.blocks, block, 0, l.stream>>>(p);
     }
     if (combinePixels > 0) {

@@ -222,6 +222,24 @@ def test_heavy_first_gives_the_same_bits(lib, ctx, jitter):
     assert lib.artfCudaHoleBatch(ctx, views, len(views), C.byref(_opts(order=2)), None) == -1  # ARTF_CUDA_EINVAL
 
 
+@pytest.mark.parametrize("count,scale,jitter", [(1, 0.3, 0), (1, 0.5, 3), (3, 0.25, 0), (7, 0.3, 0)])
+def test_split_heavy_tiles_give_the_same_bits(lib, ctx, count, scale, jitter):
+    """Frames and batches of few tiles a warp, whose heavy tiles come apart in the queue: the pixels, the ends and
+    the counts of the same rays in pixel order, none of them split, and of warps that take 16 rays at most."""
+    import torch
+    views, keep = _views(lib, count=count, scale=scale, rays=max(1, jitter))
+    seen = []
+    for kw in (dict(order=capi.ORDER_PIXELS), dict(), dict(refillBatch=16), dict(blockSize=64)):
+        for _, _, _, hdr, ends in keep:
+            hdr.zero_(), ends.zero_()
+        stats = capi.TraceStats()
+        capi.check(lib.artfCudaHoleBatch(ctx, views, count, C.byref(_opts(jitter=jitter, seed=5, **kw)), C.byref(stats)))
+        torch.cuda.synchronize()
+        seen.append(([hdr.cpu().numpy().tobytes() + ends.cpu().numpy().tobytes() for _, _, _, hdr, ends in keep],
+                     stats.rays, stats.steps, stats.crossings, stats.fp64Radial, stats.fp64Polar, stats.fp64Horizon))
+    assert all(s == seen[0] for s in seen[1:])
+
+
 @pytest.mark.parametrize("guards", [0, capi.GUARD_MOTION | capi.GUARD_RADIAL | capi.GUARD_PSI])
 def test_every_queue_kernel_gives_a_view_the_same_bits(lib, ctx, guards):
     """A frame runs the single-view queue kernel (its view a kernel parameter) and a graph of that one
