@@ -21,7 +21,7 @@
  * dependent additions, 1.9 us), three reads in turn of fields that other SMs have just written, and one
  * launch waiting for the last.  One block working through the eddies, and a launch a pass, took 62 us a
  * step; a launch for the velocities and one for the rest of each ring 10.8, one launch 9.7, and with a cell's
- * two velocities side by side, read together, 9.1 (24 steps a call: 1486 -> 265 -> 241 -> 225 us; of that the
+ * two velocities side by side, read together, 9.0 (24 steps a call: 1486 -> 265 -> 241 -> 222 us; of that the
  * launches as dependent ones 387 -> 265).  Two blocks a SM are as many as a step has: cut for three, the blocks
  * crowd on fewer SMs and 24 steps take 284. */
 #include "nvtxRange.h"
@@ -280,7 +280,6 @@ __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 3
         const uint32_t bits = __ballot_sync(0xFFFFFFFFu, e < eddies.count && !(dr * dr > 6.25f * size * size));
         if (e == 0) reaching = bits;
     }
-    startNext();
     waitBefore();
     if (!helper) {
 #pragma unroll
@@ -298,6 +297,7 @@ __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 3
         }
     }
     cluster.sync();
+    startNext(); /* (any later is alike; at the kernel's start its blocks are in the way of these: 225, not 222 us) */
     if (!helper) {
         /* (the first and last ring border on themselves) */
         const bool outBelow = rank == 0 && j > 0, outAbove = rank == RINGS - 1 && j < FH - 1;
