@@ -528,12 +528,22 @@ __device__ __forceinline__ int tileView(const MixedParams& p, int tile) {
     return lo;
 }
 
+/* The probe, the order, the trace and the sum of planes follow one another at once (programmatic dependent
+ * launch): each may start while the one before it drains, and waits here, before it reads or writes what others
+ * do, until that one has finished, and with it all before (1080p x 4 1321 -> 1308 us, one ray a pixel 374 -> 364,
+ * 512 x 288 102 -> 98). */
+__device__ __forceinline__ void chained() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 /* Each tile's weight class, and each class's count of queue slots (a tile has one a ray plane), counted
  * in the block first so that each class takes one global atomic a block. */
 template <bool kOne>
 __device__ __forceinline__ void probeTiles(const MixedParams& p, const MixedView* one, int totalTiles, int* weights,
                                            unsigned* classes) {
     __shared__ unsigned counts[kWeightClasses];
+    chained();
     if (threadIdx.x < kWeightClasses) counts[threadIdx.x] = 0;
     __syncthreads();
     const int at = (int)(blockIdx.x * 128 + threadIdx.x), g = at >> p.cornersLog2;
@@ -582,6 +592,7 @@ __device__ __forceinline__ void placeTiles(const MixedParams& p, const MixedView
                                            const int* weights, const unsigned* classes, unsigned* cursors,
                                            uint2* order) {
     __shared__ unsigned counts[kWeightClasses], runs[kWeightClasses];
+    chained();
     if (threadIdx.x < kWeightClasses) counts[threadIdx.x] = 0;
     __syncthreads();
     const int g = (int)(blockIdx.x * 128 + threadIdx.x);
@@ -635,9 +646,10 @@ __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView
     const int lane = threadIdx.x & 31;
     unsigned rounds = 0;
     clearMixed(tally);
+    chained();
     unsigned heavy = 0; /* the rays in heavy slots */
     if (kSplit) {
-        for (int c = kHeavyClass; c < kWeightClasses; ++c) heavy += __ldg(p.classes + c);
+        for (int c = kHeavyClass; c < kWeightClasses; ++c) heavy += __ldcg(p.classes + c); /* (not __ldg: a read-only load could move above the wait) */
         heavy = min(heavy, (unsigned)p.mostHeavy) << 5;
     }
     const unsigned heavyParts = heavy >> kHeavyRaysLog2;
@@ -656,7 +668,7 @@ __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView
         const MixedView* v = kOne ? one : p.views;
         int plane, tile;
         if (p.order) {
-            const uint2 s = __ldg(p.order + slot);
+            const uint2 s = __ldcg(p.order + slot);
             if (!kOne) v = p.views + (s.x & 4095u);
             plane = v->rayOut ? (int)(s.x >> 12) : 0;
             tile = (int)s.y;
@@ -724,6 +736,7 @@ __global__ void __launch_bounds__(256, 2) traceMixedOneSplit(const MixedParams p
 /* Each pixel of the views with ray planes: its rays' radiance summed in ray order and scaled by
  * 1 / rays, and their class bits; the same operations, in the same order, as the per-pixel path. */
 __device__ __forceinline__ void combinePlanes(const MixedView& v) {
+    chained();
     if (!v.rayOut) return;
     const size_t pixels = (size_t)v.f.width * (size_t)v.rows; /* the band's */
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
@@ -930,6 +943,17 @@ static MixedGrid mixedGrid(const TraceLaunch& l, int totalUnits, const void* ker
     return g;
 }
 
+/* A launch that may start while the stream's work before it drains: kernels that wait in chained(). */
+template <typename... P, typename... A>
+static cudaError_t follow(cudaStream_t stream, void (*kernel)(P...), dim3 grid, int block, const A&... args) {
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid, c.blockDim = dim3((unsigned)block), c.stream = stream, c.attrs = &early, c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 cudaError_t launchMixedTable(const TraceLaunch& l, const void* deviceTable, int viewCount, int totalUnits,
                              size_t combinePixels, int totalTiles, void* orderScratch, const void* hostView) {
     MixedParams p = paramsOf(l, deviceTable, viewCount, totalUnits);
@@ -949,12 +973,13 @@ cudaError_t launchMixedTable(const TraceLaunch& l, const void* deviceTable, int 
     p.lanesLog2 = grid.lanesLog2;
     const bool ordered = orderScratch && l.order == ARTF_CUDA_ORDER_HEAVY_FIRST && totalTiles > 0;
     const bool split = ordered && all && grid.mostHeavy > 0;
+    cudaError_t e = cudaSuccess;
     if (ordered && (split || !grid.resident)) {
         unsigned* classes = (unsigned*)orderScratch;
         unsigned* cursors = classes + 32;
         int* weights = (int*)((char*)orderScratch + kOrderHead);
         uint2* order = (uint2*)((char*)weights + (((size_t)totalTiles * sizeof(int) + 15) & ~(size_t)15));
-        const cudaError_t e = cudaMemsetAsync(orderScratch, 0, kOrderHead, l.stream);
+        e = cudaMemsetAsync(orderScratch, 0, kOrderHead, l.stream);
         if (e != cudaSuccess) return e;
         const unsigned tiles = (unsigned)((totalTiles + 127) / 128);
         if (split) {
@@ -966,27 +991,24 @@ cudaError_t launchMixedTable(const TraceLaunch& l, const void* deviceTable, int 
         const unsigned probes = (unsigned)((((long long)totalTiles << p.cornersLog2) + 127) / 128);
         if (single) {
             probeOne<<<probes, 128, 0, l.stream>>>(p, one, totalTiles, weights, classes);
-            placeOne<<<tiles, 128, 0, l.stream>>>(p, one, totalTiles, weights, classes, cursors, order);
+            e = follow(l.stream, placeOne, dim3(tiles), 128, p, one, totalTiles, weights, classes, cursors, order);
         } else {
             probeTable<<<probes, 128, 0, l.stream>>>(p, totalTiles, weights, classes);
-            placeTable<<<tiles, 128, 0, l.stream>>>(p, totalTiles, weights, classes, cursors, order);
+            e = follow(l.stream, placeTable, dim3(tiles), 128, p, totalTiles, weights, classes, cursors, order);
         }
         p.order = order;
     }
-    if (single) {
-        if (split) traceMixedOneSplit<<<grid.blocks, block, 0, l.stream>>>(p, one);
-        else if (all) traceMixedOneAll<<<grid.blocks, block, 0, l.stream>>>(p, one);
-        else traceMixedOne<<<grid.blocks, block, 0, l.stream>>>(p, one);
-    } else {
-        if (split) traceMixedTableSplit<<<grid.blocks, block, 0, l.stream>>>(p);
-        else if (all) traceMixedTableAll<<<grid.blocks, block, 0, l.stream>>>(p);
-        else traceMixedTable<<<grid.blocks, block, 0, l.stream>>>(p);
+    const dim3 blocks((unsigned)grid.blocks);
+    if (e == cudaSuccess && single)
+        e = follow(l.stream, split ? traceMixedOneSplit : all ? traceMixedOneAll : traceMixedOne, blocks, block, p, one);
+    else if (e == cudaSuccess)
+        e = follow(l.stream, split ? traceMixedTableSplit : all ? traceMixedTableAll : traceMixedTable, blocks, block, p);
+    if (e == cudaSuccess && combinePixels > 0) {
+        const unsigned sums = (unsigned)((combinePixels + 255) / 256);
+        if (single) e = follow(l.stream, combineOne, dim3(sums), 256, one);
+        else e = follow(l.stream, combineTable, dim3(sums, (unsigned)viewCount), 256, p.views);
     }
-    if (combinePixels > 0) {
-        const unsigned blocks = (unsigned)((combinePixels + 255) / 256);
-        if (single) combineOne<<<blocks, 256, 0, l.stream>>>(one);
-        else combineTable<<<dim3(blocks, (unsigned)viewCount), 256, 0, l.stream>>>(p.views);
-    }
+    if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
