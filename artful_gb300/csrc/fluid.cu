@@ -271,6 +271,9 @@ __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 3
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int tid = (int)threadIdx.x, j = (int)blockIdx.x, rank = j % RINGS;
     const bool helper = tid >= RING_THREADS;
+    /* (this block has started: the others hear of it, and wait for it, before they write to its shared memory; the
+     * step before hides it: as fast without, where a block's memory read after the next barrier takes 224 us) */
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const Ring g = rings[j];
     const uint32_t row = (uint32_t)(j * FW);
     if (helper) {
@@ -287,6 +290,9 @@ __global__ void __cluster_dims__(RINGS, 1, 1) __launch_bounds__(RING_THREADS + 3
             const int i = tid + c * RING_THREADS;
             ringFlow[i] = velocitiesAt(s, flow, g, j, i);
         }
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (!helper) {
         /* this block's share of the rings below and above the cluster, where there are any (found whole by the
          * outer blocks they cost 1.3 us a step) */
         if (tid < 2 * SHARE) {
