@@ -592,21 +592,18 @@ extern "C" int artfCudaHoleRender(ArtfCuda* ctx, const ArtfCudaHoleFrame* frame,
     ctx->drawnPixels = 0; /* (the light buffer is this path's from here on) */
     if ((status = hostInputs(ctx, hostMap, mapVersion, hostFluid, fluidVersion))) return status;
     const size_t pixels = (size_t)frame->size[0] * frame->size[1];
-    /* A host buffer that the device addresses takes the frame straight from the trace's kernels, over the
-     * link as they write it: a page-locked one, or, where the device goes through the host's page tables
-     * (Grace), any one whose pixels are aligned as the kernels store them (1080p, a ray a pixel: 678 us with a
-     * copy after the trace, 500 so, the trace alone 462).  Any other buffer gets a copy of the device's
-     * frame. */
+    /* A host buffer that the device addresses, its pixels aligned as the kernels store them, takes the frame
+     * straight from the trace's kernels, over the link as they write it: a page-locked one, or, where the device
+     * goes through the host's page tables (Grace), any (1080p, a ray a pixel: 678 us with a copy after the trace,
+     * 500 so, the trace alone 462).  Any other buffer gets a copy of the device's frame. */
     cudaPointerAttributes where;
     float* direct = nullptr;
     if (cudaPointerGetAttributes(&where, hostHdr) == cudaSuccess) {
-        if (where.type == cudaMemoryTypeHost) {
-            direct = (float*)where.devicePointer;
-        } else if (where.type == cudaMemoryTypeUnregistered && ctx->hostPages && (uintptr_t)hostHdr % sizeof(float4) == 0) {
-            touchPages(hostHdr, sizeof(float4) * pixels);
-            direct = hostHdr;
-        }
+        if (where.type == cudaMemoryTypeHost) direct = (float*)where.devicePointer;
+        else if (where.type == cudaMemoryTypeUnregistered && ctx->hostPages) direct = hostHdr;
     }
+    if ((uintptr_t)direct % sizeof(float4)) direct = nullptr;
+    if (direct && where.type == cudaMemoryTypeUnregistered) touchPages(hostHdr, sizeof(float4) * pixels);
     if (direct) {
         if ((status = artfCudaHoleTrace(ctx, frame, frame64, nullptr, nullptr, options, direct, nullptr, stats)))
             return status;

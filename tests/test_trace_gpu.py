@@ -337,3 +337,24 @@ def test_host_path_at_any_alignment(lib, ctx, offset, jitter):
     hdr, _ = g.trace(lib, ctx, frame, frame64, capi.MIXED, jitter=jitter, seed=9, persistent=1)
     assert np.array_equal(raw[base:base + floats].view(np.uint32), hdr.ravel().view(np.uint32))
     assert np.all(raw[:base] == 7.0) and np.all(raw[base + floats:] == 7.0)
+
+
+@pytest.mark.parametrize("precision,jitter", [(capi.EXACT, 0), (capi.MIXED, 3)])
+@pytest.mark.parametrize("offset", [1, 2, 3, 0])
+def test_host_path_into_page_locked_memory_at_any_alignment(lib, ctx, offset, precision, jitter):
+    """Into page-locked memory, at an address the kernels may store whole pixels to or a float off: the device
+    path's bits (a misaligned buffer takes them by a copy), and nothing beside the frame written."""
+    import torch
+    scene, frame, frame64, m, fluid = _scene_inputs(lib, "odd_101x67")
+    opts = capi.TraceOptions(precision, jitter, 9, 1.0, 0.0, 0, 0, 1)
+    floats = scene.width * scene.height * 4
+    locked = torch.full((floats + 16,), 7.0, dtype=torch.float32).pin_memory()
+    assert locked.data_ptr() % 16 == 0
+    raw = locked.numpy()
+    base = 8 + offset
+    capi.check(lib.artfCudaHoleRender(ctx, C.byref(frame), C.byref(frame64), m.ctypes.data, 0, fluid.ctypes.data, 0,
+                                      C.byref(opts), locked.data_ptr() + 4 * base, None))
+    g.set_inputs(lib, ctx, m, fluid)
+    hdr, _ = g.trace(lib, ctx, frame, frame64, precision, jitter=jitter, seed=9, persistent=1)
+    assert np.array_equal(raw[base:base + floats].view(np.uint32), hdr.ravel().view(np.uint32))
+    assert np.all(raw[:base] == 7.0) and np.all(raw[base + floats:] == 7.0)
