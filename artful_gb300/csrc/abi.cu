@@ -605,9 +605,11 @@ extern "C" int artfCudaHoleRender(ArtfCuda* ctx, const ArtfCudaHoleFrame* frame,
     if ((uintptr_t)direct % sizeof(float4)) direct = nullptr;
     if (direct && where.type == cudaMemoryTypeUnregistered) touchPages(hostHdr, sizeof(float4) * pixels);
     if (direct) {
-        if ((status = artfCudaHoleTrace(ctx, frame, frame64, nullptr, nullptr, options, direct, nullptr, stats)))
-            return status;
-        CUDA_OR(ARTF_CUDA_ELAUNCH, cudaStreamSynchronize(ctx->stream));
+        status = artfCudaHoleTrace(ctx, frame, frame64, nullptr, nullptr, options, direct, nullptr, stats);
+        /* (waited for after a failure too: no kernel of the call outlives it, with the caller's buffer) */
+        const cudaError_t done = cudaStreamSynchronize(ctx->stream);
+        if (status) return status;
+        CUDA_OR(ARTF_CUDA_ELAUNCH, done);
         return ARTF_CUDA_OK;
     }
     cudaGetLastError(); /* (a pointer the runtime does not know is no error to keep) */

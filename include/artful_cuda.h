@@ -363,9 +363,11 @@ int artfCudaAutotune(ArtfCuda* ctx, const ArtfCudaView* views, int count, const 
                      ArtfCudaTuning* result);
 
 /* The same from host memory to host memory: copies the map and fluid (when their versions changed; NULL:
- * the context's own), traces, and brings width * height float4 back to `hostHdr`: a page-locked buffer
- * (cudaHostAlloc, or registered) is written by the trace's kernels directly, any other is copied into
- * from the device's frame.  Synchronous. */
+ * the context's own), traces, and brings width * height float4 back to `hostHdr`.  A buffer aligned to 16
+ * bytes that the device addresses is written by the trace's kernels directly, and holds part of a frame
+ * when an error is returned: a page-locked one (cudaHostAlloc, or registered), and, where the device goes
+ * through the host's page tables, any (its pages are touched first).  Any other is copied into from the
+ * device's frame.  Synchronous: nothing writes to the buffer after the call, failed or not. */
 int artfCudaHoleRender(ArtfCuda* ctx, const ArtfCudaHoleFrame* frame, const ArtfCudaHoleFrame64* frame64,
                        const float* hostMap, uint64_t mapVersion, const float* hostFluid, uint64_t fluidVersion,
                        const ArtfCudaTraceOptions* options, float* hostHdr, ArtfCudaTraceStats* stats);
