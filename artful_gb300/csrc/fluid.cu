@@ -33,11 +33,12 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <mutex>
-
 namespace artf {
 int contextStream(ArtfCuda* ctx, cudaStream_t* stream);
 int contextFluid(ArtfCuda* ctx, float** fluid);
+struct GasStore;
+cudaError_t takeGas(ArtfCuda* ctx, size_t bytes, void** block, GasStore** store);
+void giveGas(GasStore* store, void* block, bool idle);
 int failWith(int status, const char* message);
 }  // namespace artf
 
@@ -385,6 +386,7 @@ struct ArtfCudaFluid {
     cudaStream_t stream;
     float inner, outer;
     float* block;          /* the seven fields and the rings' terms, one allocation */
+    artf::GasStore* store; /* where it goes back to */
     float* dens[2];
     float2* flow[2];       /* velocities along the radius and the orbit, side by side: read together */
     float* field;
@@ -397,55 +399,17 @@ struct ArtfCudaFluid {
 
 namespace {
 
-/* Where gases' memory comes from: a pool a device, which keeps up to two gases' worth when they are freed, so
- * that a disc that changes does not map and unmap its gas each time (0.2 ms of a new gas's 0.9), until a
- * context is destroyed (trimGases).  NULL where the device has no pools. */
 constexpr size_t GAS_BYTES = sizeof(float) * FIELD * 7 + sizeof(Ring) * FH;
-constexpr int MOST_DEVICES = 64;
-std::mutex poolLock;
-cudaMemPool_t pools[MOST_DEVICES];
 
-cudaMemPool_t poolOf(int device) {
-    if (device < 0 || device >= MOST_DEVICES) return nullptr;
-    std::lock_guard<std::mutex> hold(poolLock);
-    if (!pools[device]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        uint64_t keep = 2 * (GAS_BYTES + ((size_t)2 << 20));
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return nullptr;
-        }
-        pools[device] = pool;
-    }
-    return pools[device];
-}
-
-/* A gas's memory, its use by the stream's work to come; and given back, once the device is done with it (work
- * on other streams that reads the field among it). */
-cudaError_t takeGas(ArtfCudaFluid* f) {
-    const cudaMemPool_t pool = poolOf(f->device);
-    const cudaError_t e = pool ? cudaMallocFromPoolAsync((void**)&f->block, GAS_BYTES, pool, f->stream)
-                               : cudaMalloc((void**)&f->block, GAS_BYTES);
-    if (e != cudaSuccess) {
-        (void)cudaGetLastError(); /* (or the next launch's check would report it) */
-        f->block = nullptr;
-    }
-    return e;
-}
-
+/* A gas's memory given back, once the device is done with it (work on other streams that reads the field among
+ * it). */
 void giveGas(ArtfCudaFluid* f) {
     if (!f->block) return;
     int current = 0;
     const bool known = cudaGetDevice(&current) == cudaSuccess;
     cudaSetDevice(f->device);
-    cudaDeviceSynchronize();
-    if (poolOf(f->device)) cudaFreeAsync(f->block, cudaStreamLegacy); /* (its context may be gone) */
-    else cudaFree(f->block);
+    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+    artf::giveGas(f->store, f->block, idle);
     if (known) cudaSetDevice(current);
 }
 
@@ -537,14 +501,6 @@ int advanceSteps(ArtfCudaFluid* f, int64_t steps) {
 
 }  // namespace
 
-namespace artf {
-/* The memory the device's pool holds beyond the gases that live, given back (a context was destroyed). */
-void trimGases(int device) {
-    std::lock_guard<std::mutex> hold(poolLock);
-    if (device >= 0 && device < MOST_DEVICES && pools[device]) cudaMemPoolTrimTo(pools[device], 0);
-}
-}  // namespace artf
-
 extern "C" void artfCudaFluidFree(ArtfCudaFluid* f) {
     if (!f) return;
     giveGas(f);
@@ -564,7 +520,8 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
     if (!f) return artf::failWith(ARTF_CUDA_ENOMEM, "host allocation");
     f->ctx = ctx, f->stream = stream, f->inner = inner, f->outer = outer;
     f->state = 0x9E3779B9u, f->time = time;
-    if (cudaGetDevice(&f->device) != cudaSuccess || takeGas(f) != cudaSuccess) {
+    if (cudaGetDevice(&f->device) != cudaSuccess ||
+        artf::takeGas(ctx, GAS_BYTES, (void**)&f->block, &f->store) != cudaSuccess) {
         artfCudaFluidFree(f);
         return artf::failWith(ARTF_CUDA_ENOMEM, "fluid: device allocation");
     }

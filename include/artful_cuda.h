@@ -466,7 +466,8 @@ const float* artfCudaFluidField(const ArtfCudaFluid* f);
 double artfCudaFluidTime(const ArtfCudaFluid* f);
 /* The field copied to host memory.  Synchronous. */
 int artfCudaFluidRead(const ArtfCudaFluid* f, float* host);
-/* fluid.c:243 */
+/* fluid.c:243.  The device is waited for; the gas's memory stays with its context for the next gas (that of two
+ * at most, until the context is destroyed), or goes at once where the context has gone before. */
 void artfCudaFluidFree(ArtfCudaFluid* f);
 
 /* ---- measurement ------------------------------------------------------------------------------- */

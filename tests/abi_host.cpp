@@ -27,6 +27,7 @@ static int launches = 0, pendingLaunches = 0; /* in all; and since the stream wa
 static int failLaunch = -1;                   /* this one (from 0) fails */
 static int events = 0, failEvent = -1;        /* event records of a call; the one (from 0) that fails */
 static std::vector<float*> frames;            /* where each launch was to write its frame */
+static bool failMalloc = false;
 static std::set<void*> live;                  /* device allocations */
 
 static cudaError_t launched(float4* hdr) {
@@ -44,6 +45,7 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { return *
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return events++ == failEvent ? cudaErrorInvalidValue : cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t bytes) {
+    if (failMalloc) return cudaErrorMemoryAllocation;
     *p = aligned_alloc(256, (bytes + 255) / 256 * 256);
     live.insert(*p);
     return cudaSuccess;
@@ -122,7 +124,11 @@ cudaError_t launchAdjoint(const void*, int, int, int, int, unsigned long long*, 
     return cudaSuccess;
 }
 cudaError_t launchTangents(const TraceLaunch&, const double*, double, double*) { return cudaSuccess; }
-void trimGases(int) {}
+
+/* (the gas's side of its memory: abi.cu) */
+struct GasStore;
+cudaError_t takeGas(ArtfCuda* ctx, size_t bytes, void** block, GasStore** store);
+void giveGas(GasStore* store, void* block, bool idle);
 }  // namespace artf
 
 /* ---- the checks ---------------------------------------------------------------------------------- */
@@ -179,11 +185,41 @@ static void failedCalls() {
     free(buffer);
 }
 
+/* Gases' memory: plain device memory, kept for the context's next gases up to two, its own context's alone, and
+ * all given back whichever goes first. */
+static void gasMemory() {
+    ArtfCuda *a = nullptr, *b = nullptr;
+    check(artfCudaCreate(0, &a) == ARTF_CUDA_OK && artfCudaCreate(0, &b) == ARTF_CUDA_OK, "two contexts");
+    const size_t before = live.size();
+    void *block[4], *again, *other, *late;
+    artf::GasStore *store[4], *s, *so, *sl;
+    for (int k = 0; k < 4; ++k)
+        check(artf::takeGas(a, 1024, &block[k], &store[k]) == cudaSuccess && live.count(block[k]), "a gas's memory");
+    for (int k = 0; k < 4; ++k) artf::giveGas(store[k], block[k], true);
+    check(live.size() == before + 2, "two gases' memory kept");
+    check(artf::takeGas(b, 1024, &other, &so) == cudaSuccess && live.size() == before + 3, "another context's is its own");
+    check(artf::takeGas(a, 1024, &again, &s) == cudaSuccess && live.size() == before + 3, "kept memory taken again");
+    check(artf::takeGas(a, 1024, &late, &sl) == cudaSuccess && late != again && live.size() == before + 3, "and the other");
+    artf::giveGas(s, again, false);
+    check(live.count(again) == 0 && live.size() == before + 2, "memory that may be in use is not kept");
+    artfCudaDestroy(a);
+    check(live.count(late) == 1, "a context gives back what it keeps, not what a gas holds");
+    artf::giveGas(sl, late, true); /* (its context is gone) */
+    check(live.count(late) == 0, "a gas that outlived its context gives its memory back");
+    artf::giveGas(so, other, true);
+    artfCudaDestroy(b);
+    check(live.count(other) == 0, "nothing left");
+    failMalloc = true;
+    check(artf::takeGas(ctx, 1024, &late, &sl) == cudaErrorMemoryAllocation && !late, "a failed allocation is reported");
+    failMalloc = false;
+}
+
 int main() {
     inputs = (float*)calloc(ARTF_CUDA_MAP_FLOATS, sizeof(float));
     check(artfCudaCreate(0, &ctx) == ARTF_CUDA_OK, "a context");
     hostFrames();
     failedCalls();
+    gasMemory();
     artfCudaDestroy(ctx);
     check(live.empty(), "device memory left after the context");
     free(inputs);
