@@ -565,6 +565,9 @@ extern "C" int artfCudaFluidNew(ArtfCuda* ctx, float inner, float outer, float s
     }
     int status = e == cudaSuccess ? stirStart(f) : artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
     if (!status) status = advanceSteps(f, WARM_STEPS);
+    /* (the gas is there for any stream when the call returns) */
+    if (!status && (e = cudaStreamSynchronize(stream)) != cudaSuccess)
+        status = artf::failWith(ARTF_CUDA_ELAUNCH, cudaGetErrorString(e));
     if (status) {
         artfCudaFluidFree(f);
         return status;

@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import ctypes as C
 import hashlib
+from types import SimpleNamespace
 
 import numpy as np
 import pytest
@@ -191,3 +192,23 @@ def test_gases_come_and_go(lib, ctx):
     a = GpuFluid(lib, ctx, *discs[1], 0.0)
     assert np.array_equal(a.read()[0], want[discs[1]])
     a.free()
+
+
+def test_a_new_gas_is_there_when_its_call_returns(lib, ctx):
+    """artfCudaFluidNew is synchronous: nothing of the gas's start is still to run, and its field may be read from
+    another stream at once."""
+    import torch
+    own = torch.cuda.ExternalStream(lib.artfCudaStream(ctx))
+    other = torch.cuda.Stream()
+    for _ in range(3):
+        a = GpuFluid(lib, ctx, 2.4, 20.0, 0.8, 0.0)
+        assert own.query()
+        with torch.cuda.stream(other):
+            raw = torch.empty(capi.FLUID_FLOATS, dtype=torch.float32, pin_memory=True)
+            field = torch.as_tensor(SimpleNamespace(__cuda_array_interface__={
+                "data": (lib.artfCudaFluidField(a.handle), False), "typestr": "<f4", "version": 2,
+                "shape": (capi.FLUID_FLOATS,), "strides": None}), device="cuda")
+            raw.copy_(field, non_blocking=True)
+        other.synchronize()
+        assert np.array_equal(raw.numpy(), a.read()[0].ravel())
+        a.free()
