@@ -42,23 +42,11 @@
 #define ARTF_FP64_NEWTON_STEPS 1 /* one refinement: ~40 bits, far below float's rounding (3.4 % faster) */
 #include "lensKernel.cuh"
 #include "lensMixed.h"
+#include "lensPairs.cuh"
 
 #include <string.h>
 
 namespace artf {
-
-/* A value as the unevaluated sum hi + lo of two floats, |lo| at most half an ulp of hi: Dekker's
- * double-length arithmetic (1971), about 48 significant bits from FP32 instructions, which this GPU
- * issues 64 times as fast as FP64 ones. */
-struct Ff {
-    float hi, lo;
-};
-
-/* What a ray's set-up under the MOTION guard takes from the view, in double-float: the eye's basis, the
- * metric's four factors, rho, a and the start terms. */
-struct MotionTermsFf {
-    Ff forward[3], right[3], up[3], metric[4], rho, a, a2, mu0Squared, minusTwoA2;
-};
 
 /* A view as the kernels read it, from the device view table or as a parameter. */
 struct MixedView {
@@ -158,61 +146,8 @@ __device__ __noinline__ float narrow(double d) {
     return __uint_as_float(sign | bits);
 }
 
-/* ---- double-float arithmetic --------------------------------------------------------------------------
- * A sum is Knuth's error-free TwoSum of the high parts, a product's error an FMA's residual; the reciprocal
- * and the reciprocal square root are the float estimates refined by one Newton-Raphson step.  The low part of
- * a result gathers what its operation left over and is not folded back into the high part (ffNorm, Dekker's
- * fast two-sum) until a value is kept or rounded to float: what that would save in low bits lies beyond
- * 2^-44 (artfCudaCheckPairs measures it), and it cost three of every ten instructions (a wide motion 277 ->
- * 188, a set-up some 400 -> 250).  No step contracts: every product is its own or an explicit FMA's. */
-__device__ __forceinline__ Ff ffNorm(Ff a) {
-    const float hi = __fadd_rn(a.hi, a.lo);
-    return Ff{hi, __fadd_rn(a.lo, -__fadd_rn(hi, -a.hi))};
-}
-__device__ __forceinline__ float ffRound(Ff a) { return __fadd_rn(a.hi, a.lo); }
-/* a + b of floats: the rounded sum and its error */
-__device__ __forceinline__ Ff ffSum(float a, float b) {
-    const float s = __fadd_rn(a, b), bb = __fadd_rn(s, -a);
-    return Ff{s, __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -bb)), __fadd_rn(b, -bb))};
-}
-__device__ __forceinline__ Ff ffProd(float a, float b) {
-    const float p = __fmul_rn(a, b);
-    return Ff{p, __fmaf_rn(a, b, -p)};
-}
-__device__ __forceinline__ Ff ffAdd(Ff a, Ff b) {
-    const Ff s = ffSum(a.hi, b.hi);
-    return Ff{s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo))};
-}
-__device__ __forceinline__ Ff ffAddF(Ff a, float b) {
-    const Ff s = ffSum(a.hi, b);
-    return Ff{s.hi, __fadd_rn(s.lo, a.lo)};
-}
-__device__ __forceinline__ Ff ffNeg(Ff a) { return Ff{-a.hi, -a.lo}; }
-__device__ __forceinline__ Ff ffSub(Ff a, Ff b) { return ffAdd(a, ffNeg(b)); }
-__device__ __forceinline__ Ff ffMul(Ff a, Ff b) {
-    const Ff p = ffProd(a.hi, b.hi);
-    return Ff{p.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, p.lo))};
-}
-__device__ __forceinline__ Ff ffMulF(Ff a, float b) {
-    const Ff p = ffProd(a.hi, b);
-    return Ff{p.hi, __fmaf_rn(a.lo, b, p.lo)};
-}
-__device__ __forceinline__ Ff ffSquare(Ff a) {
-    const Ff p = ffProd(a.hi, a.hi);
-    return Ff{p.hi, __fmaf_rn(a.hi, a.lo + a.lo, p.lo)};
-}
-__device__ __forceinline__ Ff ffScale(Ff a, float powerOfTwo) { return Ff{a.hi * powerOfTwo, a.lo * powerOfTwo}; }
-__device__ __forceinline__ Ff ffRecip(Ff x) {
-    const float y = __fdividef(1.f, x.hi);
-    const float r = __fmaf_rn(-x.lo, y, __fmaf_rn(-x.hi, y, 1.f)); /* 1 - x y */
-    return Ff{y, __fmul_rn(y, r)};
-}
-__device__ __forceinline__ Ff ffRsqrt(Ff x) {
-    const float y = rsqrtf(x.hi);
-    const Ff yy = ffProd(y, y);
-    const Ff q = ffMul(x, yy); /* x y^2, within an ulp or two of 1 */
-    return Ff{y, __fmul_rn(.5f * y, __fadd_rn(__fadd_rn(1.f, -q.hi), -q.lo))};
-}
+/* ---- pairs (lensPairs.cuh) to and from double ---------------------------------------------------------- */
+
 /* hi + lo as a double: exact, since the pair holds at most 48 significant bits. */
 __device__ __forceinline__ double ffWide(Ff a) { return widen(a.hi) + widen(a.lo); }
 __device__ __forceinline__ Ff ffSplit(double x) {
@@ -220,63 +155,10 @@ __device__ __forceinline__ Ff ffSplit(double x) {
     return Ff{hi, narrow(x - widen(hi))};
 }
 
-/* x (A + x (B + x C)): what u'' is of u, and n_z'' of n_z with B = 0 and C = -2 a^2
- * (a^2 n_z - (K + 2 a^2 n_z^2) n_z, and A is a^2 - K for both). */
-struct Cubic {
-    Ff A, B, C;
-};
-__device__ __forceinline__ Ff ffCubic(const Cubic& f, Ff x) {
-    return ffMul(x, ffAdd(f.A, ffMul(x, ffAdd(f.B, ffMul(x, f.C)))));
-}
-__device__ __forceinline__ Ff ffCubicF(const Cubic& f, float x) {
-    return ffMulF(ffAdd(f.A, ffMulF(ffAdd(f.B, ffMulF(f.C, x)), x)), x);
-}
-/* One Nystrom step (lens.inc:165-192) of x'' = cubic(x) in double-float, from x and its rate v in float:
- * the motion of u at a radial turning point and of n_z at a polar one are this same step, so a warp runs
- * it once for the lanes at either.  Rounded to float: the next x and v, and the first stage. */
-__device__ __forceinline__ void motionFf(const Cubic& f, float step, float x, float v, float& nextX, float& nextV,
-                                         float& first) {
-    const Ff step2 = ffProd(step, step);
-    const Ff k1 = ffCubicF(f, x);
-    const Ff mid = ffAdd(ffAddF(ffProd(step * .5f, v), x), ffMul(ffScale(step2, .125f), k1));
-    const Ff k2 = ffCubic(f, mid);
-    const Ff xv = ffAddF(ffProd(step, v), x);
-    const Ff k3 = ffCubic(f, ffAdd(xv, ffMul(ffScale(step2, .5f), k2)));
-    nextX = ffRound(ffAdd(xv, ffMul(ffMulF(step2, 1.f / 6.f), ffAdd(k1, ffScale(k2, 2.f)))));
-    nextV = ffRound(ffAddF(ffMul(ffProd(step, 1.f / 6.f), ffAdd(ffAdd(k1, k3), ffScale(k2, 4.f))), v));
-    first = ffRound(k1);
-}
-
 /* The wide coefficients, their high halves the FP32 ones. */
 __device__ __forceinline__ void setWide(MixedRay& r, Ff uA, Ff uB, Ff uC, Ff xiA) {
-    uA = ffNorm(uA), uB = ffNorm(uB), uC = ffNorm(uC), xiA = ffNorm(xiA);
     r.c.uA = uA.hi, r.c.uB = uB.hi, r.c.uC = uC.hi, r.c.xiA = xiA.hi;
     r.uALo = uA.lo, r.uBLo = uB.lo, r.uCLo = uC.lo, r.xiALo = xiA.lo;
-}
-
-/* The constants of motion alone, for an eye at rest (lens.inc:125-142 without the aberration of
- * 110-122), in double-float, in rayStartWith's order of operations with the direction normalised first: E,
- * the axial momentum xi, eta and K = eta + xi^2 and the radial equation's coefficients, rounded to float
- * into r.c, the low halves of those the wide sub-steps take
- * into r, and the factors the first state is made of (d_x, 1 / (|d| E), across and the axial component
- * of the direction over E), which the caller forms in FP32 as the reference's integrator has them. */
-__device__ __forceinline__ void motionConstantsFf(const MotionTermsFf& t, float nx, float ny, MixedRay& r,
-                                                  float& dx, float& over, float& across, float& xiAxis) {
-    Ff d[3];
-    for (int k = 0; k < 3; ++k) d[k] = ffAdd(ffAdd(t.forward[k], ffMulF(t.right[k], nx)), ffMulF(t.up[k], ny));
-    const Ff invLength = ffRsqrt(ffAdd(ffAdd(ffSquare(d[0]), ffSquare(d[1])), ffSquare(d[2])));
-    const Ff dz = ffMul(d[2], invLength);
-    const Ff invEnergy = ffRecip(ffNorm(ffSub(t.metric[0], ffMul(t.metric[1], dz))));
-    const Ff overFf = ffMul(invLength, invEnergy);
-    const Ff xi = ffNeg(ffMul(ffMul(t.metric[2], dz), invEnergy));
-    const Ff xiAxisFf = ffMul(ffMul(t.metric[3], d[2]), overFf);
-    const Ff acrossFf = ffMul(ffMul(t.rho, d[1]), overFf);
-    const Ff eta = ffAdd(ffSquare(acrossFf), ffMul(t.mu0Squared, ffSub(ffSquare(xiAxisFf), t.a2)));
-    const Ff big = ffAdd(eta, ffSquare(xi));
-    r.c.invEnergy = ffRound(invEnergy), r.c.xi = ffRound(xi), r.c.moved = 1.f, r.c.big = ffRound(big);
-    setWide(r, ffSub(t.a2, big), ffMulF(ffAdd(eta, ffSquare(ffSub(xi, t.a))), 3.f), ffMul(t.minusTwoA2, eta),
-            ffMul(xi, t.a));
-    dx = ffRound(d[0]), over = ffRound(overFf), across = ffRound(acrossFf), xiAxis = ffRound(xiAxisFf);
 }
 
 /* The helpers below take the guards apart from the parameters, so that a kernel built for all of them
@@ -298,15 +180,17 @@ __device__ __forceinline__ void mixedStart(const MixedParams& p, uint32_t guards
         r.s.u = v.startNarrow[3], r.s.w = narrow(sd.w);
         for (int k = 0; k < 3; ++k) r.s.n[k] = v.startNarrow[k], r.s.v[k] = narrow(sd.v[k]);
     } else if (guards & ARTF_CUDA_GUARD_MOTION) {
-        float dx, over, across, xiAxis;
-        motionConstantsFf(v.motion, nx, ny, r, dx, over, across, xiAxis);
+        /* in double-float; the first state and the step, the integrator's FP32 quantities, from them in FP32 */
+        const MotionFf m = motionConstantsFf(v.motion, nx, ny);
+        r.c.invEnergy = m.invEnergy.hi, r.c.xi = m.xi.hi, r.c.moved = 1.f, r.c.big = m.big.hi;
+        setWide(r, m.uA, m.uB, m.uC, m.xiA);
         r.c.step = divSqrtR(v.stepBaseNarrow, maxX(r.c.big, 4.f));
         r.stepLo = 0.f;
         /* (u and n start at the eye's: the view's, narrowed once) */
         r.s.u = v.startNarrow[3];
-        r.s.w = v.wScaleNarrow * dx * over;
+        r.s.w = v.wScaleNarrow * m.dx.hi * m.over.hi;
         for (int k = 0; k < 3; ++k)
-            r.s.n[k] = v.startNarrow[k], r.s.v[k] = sum2(across, v.f.etheta[k], xiAxis, v.f.ephi[k]);
+            r.s.n[k] = v.startNarrow[k], r.s.v[k] = sum2(m.across.hi, v.f.etheta[k], m.xiAxis.hi, v.f.ephi[k]);
     } else {
         rayStart(v.f, nx, ny, time, p.stepScale, r.c, r.s);
         r.stepLo = r.uALo = r.uBLo = r.uCLo = r.xiALo = 0.f;
@@ -348,15 +232,14 @@ __device__ __forceinline__ void mixedGuards(const MixedView& v, MixedRay& r, boo
         o.k1 = narrow(k1);
     }
     while (turnR || turnP) {
-        Cubic f{Ff{r.c.uA, r.uALo}, Ff{0.f, 0.f}, ffScale(v.motion.a2, -2.f)};
+        Cubic f{Ff{r.c.uA, r.uALo}, Ff{0.f, 0.f}, Ff{-2.f * v.motion.a2.hi, -2.f * v.motion.a2.lo}};
         if (turnR) f.B = Ff{r.c.uB, r.uBLo}, f.C = Ff{r.c.uC, r.uCLo};
-        float x, rate, k1;
-        motionFf(f, r.c.step, turnR ? r.s.u : r.s.n[2], turnR ? r.s.w : r.s.v[2], x, rate, k1);
+        const Motion m = motionFf(f, r.c.step, turnR ? r.s.u : r.s.n[2], turnR ? r.s.w : r.s.v[2]);
         if (turnR) {
-            o.next.u = x, o.next.w = rate, o.k1 = k1;
+            o.next.u = m.x.hi, o.next.w = m.v.hi, o.k1 = m.first.hi;
             turnR = false;
         } else {
-            o.next.n[2] = x, o.next.v[2] = rate, o.a1[2] = k1;
+            o.next.n[2] = m.x.hi, o.next.v[2] = m.v.hi, o.a1[2] = m.first.hi;
             turnP = false;
         }
     }
@@ -1025,8 +908,8 @@ __global__ void checkPairs(const float4* in, float* out, int count) {
     if (i >= count) return;
     const float4 r = in[i];
     const Ff a{r.x, r.y}, b{r.z, r.w};
-    const Ff sum = ffNorm(ffAdd(a, b)), product = ffNorm(ffMul(a, b)), recip = ffNorm(ffRecip(a));
-    const Ff root = ffNorm(ffRsqrt(Ff{fabsf(a.hi), a.hi < 0.f ? -a.lo : a.lo}));
+    const Ff sum = ffAdd(a, b), product = ffMul(a, b), recip = ffRecip(a);
+    const Ff root = ffRsqrt(Ff{fabsf(a.hi), a.hi < 0.f ? -a.lo : a.lo});
     float* o = out + (size_t)i * 8;
     o[0] = sum.hi, o[1] = sum.lo, o[2] = product.hi, o[3] = product.lo;
     o[4] = recip.hi, o[5] = recip.lo, o[6] = root.hi, o[7] = root.lo;
