@@ -209,8 +209,8 @@ __device__ __forceinline__ void mixedStart(const MixedParams& p, uint32_t guards
  * whole sub-step in FP64 (the frame-drag rate's Delta / r^2 cancels there, and it divides).  At a turning
  * point, of u or of n_z, that coordinate's motion in double-float: psi and its rate, and the components
  * about the axis, smooth there, stay the FP32 step's.  A step that turns both runs the motion twice. */
-__device__ __forceinline__ void mixedGuards(const MixedView& v, MixedRay& r, bool band, bool turnR, bool turnP,
-                                            StepOut<float>& o, unsigned& rounds) {
+__device__ __forceinline__ void mixedGuards(uint32_t guards, const MixedView& v, MixedRay& r, bool band, bool turnR,
+                                            bool turnP, StepOut<float>& o, unsigned& rounds) {
     if (!(band || turnR || turnP)) return;
     turnR = turnR && !band;
     r.wide += 1u | (band ? 0x10000u : 0u);
@@ -232,8 +232,8 @@ __device__ __forceinline__ void mixedGuards(const MixedView& v, MixedRay& r, boo
         o.k1 = narrow(k1);
     }
     while (turnR || turnP) {
-        Cubic f{Ff{r.c.uA, r.uALo}, Ff{0.f, 0.f}, Ff{-2.f * v.motion.a2.hi, -2.f * v.motion.a2.lo}};
-        if (turnR) f.B = Ff{r.c.uB, r.uBLo}, f.C = Ff{r.c.uC, r.uCLo};
+        Cubic f = axisCubic(v.motion.a2, Ff{r.c.uA, r.uALo}, r.c.big, guards & ARTF_CUDA_GUARD_MOTION);
+        if (turnR) f = Cubic{Ff{r.c.uA, r.uALo}, Ff{r.c.uB, r.uBLo}, Ff{r.c.uC, r.uCLo}};
         const Motion m = motionFf(f, r.c.step, turnR ? r.s.u : r.s.n[2], turnR ? r.s.w : r.s.v[2]);
         if (turnR) {
             o.next.u = m.x.hi, o.next.w = m.v.hi, o.k1 = m.first.hi;
@@ -331,7 +331,7 @@ __device__ __forceinline__ unsigned traceRayMixed(const MixedParams& p, const Mi
         const bool turnR = (guards & ARTF_CUDA_GUARD_RADIAL) && ((r.s.w > 0.f) != (o.next.w > 0.f));
         const bool turnP = (guards & ARTF_CUDA_GUARD_POLAR) && ((r.s.v[2] > 0.f) != (o.next.v[2] > 0.f));
         if (band | turnR | turnP | (r.s.n[2] * o.next.n[2] < 0.f) | (0.f > o.next.u) | (o.next.u > v.f.uHorizon)) {
-            mixedGuards(v, r, band, turnR, turnP, o, rounds);
+            mixedGuards(guards, v, r, band, turnR, turnP, o, rounds);
             if (const unsigned met = mixedMeets(compensated, v, r, o, end)) {
                 ended = met;
                 break;

@@ -133,6 +133,12 @@ ARTF_PAIR Motion motionFf(const Cubic& f, float step, float x, float v) {
     return Motion{nextX, nextV, k1};
 }
 
+/* n_z's cubic.  A = a^2 - K is the constants' uA; where the constants are float (no MOTION guard) uA carries a
+ * float's rounding of that difference, and A is formed from a^2 and the float K. */
+ARTF_PAIR Cubic axisCubic(Ff a2, Ff uA, float K, bool pairedConstants) {
+    return Cubic{pairedConstants ? uA : ffSub(a2, Ff{K, 0.f}), Ff{0.f, 0.f}, Ff{-2.f * a2.hi, -2.f * a2.lo}};
+}
+
 /* What a ray's set-up takes from the view: the eye's basis, the metric's four factors, rho, a and the start
  * terms. */
 struct MotionTermsFf {

@@ -95,6 +95,7 @@ struct Errors {
 static Errors invEnergy{"invEnergy"}, xi{"xi"}, big{"big"}, uA{"uA"}, uB{"uB"}, uC{"uC"}, xiA{"xiA"};
 static Errors step[2][3] = {{{"radial_x"}, {"radial_v"}, {"radial_first"}}, {{"polar_x"}, {"polar_v"}, {"polar_first"}}};
 static long loose = 0;
+static L axis = 0; /* the worst error of n_z's cubic */
 
 static void kept(Ff a) { loose += (float)((double)a.hi + (double)a.lo) != a.hi; }
 
@@ -137,12 +138,18 @@ int main() {
             for (int k = 0; k < 3; ++k)
                 d[k] = value(t.forward[k]) + value(t.right[k]) * nx + value(t.up[k]) * ny, length2 += d[k] * d[k];
             const L inv = 1 / sqrtl(length2), dz = d[2] * inv, e = 1 / (value(t.metric[0]) - value(t.metric[1]) * dz);
-            const L x = -value(t.metric[2]) * dz * e, axis = value(t.metric[3]) * dz * e, across = value(t.rho) * d[1] * inv * e;
-            const L eta = across * across + value(t.mu0Squared) * (axis * axis - value(t.a2)), K = eta + x * x;
+            const L x = -value(t.metric[2]) * dz * e, xiAxis = value(t.metric[3]) * dz * e, across = value(t.rho) * d[1] * inv * e;
+            const L eta = across * across + value(t.mu0Squared) * (xiAxis * xiAxis - value(t.a2)), K = eta + x * x;
             const L off = x - value(t.a), A = value(t.a2) - K, B = 3 * (eta + off * off), C = value(t.minusTwoA2) * eta;
             invEnergy.add(m.invEnergy, y.invEnergy, e, fabsl(e)), xi.add(m.xi, y.xi, x, fabsl(x));
             big.add(m.big, y.big, K, fabsl(K)), uA.add(m.uA, y.uA, A, fabsl(A)), uB.add(m.uB, y.uB, B, fabsl(B));
             uC.add(m.uC, y.uC, C, fabsl(C)), xiA.add(m.xiA, y.xiA, x * value(t.a), fabsl(x * value(t.a)));
+            /* n_z's cubic with constants in pairs, and with float ones, as the ray has them without that guard */
+            const float floatK = m.big.hi, floatA = (float)(a2 - (double)floatK);
+            const Cubic paired = axisCubic(t.a2, m.uA, m.big.hi, true), plain = axisCubic(t.a2, Ff{floatA, 0.f}, floatK, false);
+            axis = fmaxl(axis, fabsl(value(paired.A) - value(m.uA)) / fabsl(A));
+            axis = fmaxl(axis, fabsl(value(plain.A) - (value(t.a2) - floatK)) / (value(t.a2) + fabsl((L)floatK)));
+            axis = fmaxl(axis, fabsl(value(paired.C) + 2 * value(t.a2)) + fabsl(value(paired.B)));
             /* the ray in float, to where its rates turn */
             RayConst<float> c;
             RayState<float> s;
@@ -152,7 +159,7 @@ int main() {
                 nystromStep((float)a, c, s, o);
                 if ((s.w > 0) != (o.next.w > 0)) turn(step[0], Cubic{m.uA, m.uB, m.uC}, c.step, s.u, s.w);
                 if ((s.v[2] > 0) != (o.next.v[2] > 0))
-                    turn(step[1], Cubic{m.uA, Ff{0.f, 0.f}, Ff{-2.f * t.a2.hi, -2.f * t.a2.lo}}, c.step, s.n[2], s.v[2]);
+                    turn(step[1], paired, c.step, s.n[2], s.v[2]);
                 if (o.next.u < 0 || o.next.u > frame.uHorizon) break;
                 s = o.next;
             }
@@ -161,6 +168,6 @@ int main() {
     for (Errors* e : {&invEnergy, &xi, &big, &uA, &uB, &uC, &xiA}) e->print();
     for (auto& kind : step)
         for (Errors& e : kind) e.print();
-    printf("loose %ld\n", loose);
+    printf("loose %ld\naxis_log2 %.2f\n", loose, axis > 0 ? (double)log2l(axis) : -99.);
     return 0;
 }

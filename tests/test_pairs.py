@@ -44,3 +44,9 @@ def test_errors_are_the_renormalised_pairs(measured, name):
 
 def test_kept_values_are_normalised(measured):
     assert measured["loose"] == 0
+
+
+def test_the_axis_cubic_keeps_its_bits(measured):
+    """a^2 - K as a pair, whether the ray's constants are pairs or float: one renormalised difference of values of
+    48 and 24 bits, 2^-47 of their size."""
+    assert measured["axis_log2"] <= -47.0
