@@ -18,6 +18,8 @@
 #pragma once
 
 #include <math.h>
+#include <stdint.h>
+#include <string.h>
 
 #if defined(__CUDACC__)
 #define ARTF_PAIR __host__ __device__ __forceinline__
@@ -102,6 +104,26 @@ ARTF_PAIR Ff ffRsqrt(Ff x) {
     const Ff q = ffMulOpen(x, ffProd(y, y)); /* x y^2, next to 1 */
     return ffNorm(y, mulF(.5f * y, addF(addF(1.f, -q.hi), -q.lo)));
 }
+
+/* A double as the float it rounds to and what is left of its bits in a word: all 53, where a pair's low float would
+ * keep 48.  restOf: of x beside `wide`, its float widened; withRest: x again. */
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ int64_t bitsOf(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ double ofBits(int64_t b) { return __longlong_as_double(b); }
+#else
+ARTF_PAIR int64_t bitsOf(double x) {
+    int64_t b;
+    memcpy(&b, &x, sizeof b);
+    return b;
+}
+ARTF_PAIR double ofBits(int64_t b) {
+    double x;
+    memcpy(&x, &b, sizeof x);
+    return x;
+}
+#endif
+ARTF_PAIR int32_t restOf(double x, double wide) { return (int32_t)(bitsOf(x) - bitsOf(wide)); }
+ARTF_PAIR double withRest(double wide, int32_t rest) { return ofBits(bitsOf(wide) + rest); }
 
 /* x (A + x (B + x C)): what u'' is of u, and n_z'' of n_z with A = a^2 - K, B = 0 and C = -2 a^2
  * (a^2 n_z - (K + 2 a^2 n_z^2) n_z). */

@@ -113,7 +113,19 @@ static void turn(Errors* e, const Cubic& f, float h, float x, float v) {
     e[2].add(a.first, b.first, k1, size);
 }
 
+/* Doubles from the float they round to and their rest, every exponent a step can have. */
+static long lostBits() {
+    long lost = 0;
+    for (int k = 0; k < 1000000; ++k) {
+        const double x = std::ldexp(uniform(1, 2), (int)uniform(-60, 20));
+        const float f = (float)x;
+        lost += withRest((double)f, restOf(x, (double)f)) != x;
+    }
+    return lost;
+}
+
 int main() {
+    printf("lost %ld\n", lostBits());
     for (int eye = 0; eye < 96; ++eye) {
         ArtfCudaHoleParams p = {};
         p.spin = uniform(-.5, .998), p.inclination = uniform(5, 89) * 3.14159265358979 / 180, p.innerScale = 1;

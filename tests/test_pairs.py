@@ -50,3 +50,7 @@ def test_the_axis_cubic_keeps_its_bits(measured):
     """a^2 - K as a pair, whether the ray's constants are pairs or float: one renormalised difference of values of
     48 and 24 bits, 2^-47 of their size."""
     assert measured["axis_log2"] <= -47.0
+
+
+def test_a_double_is_its_float_and_its_rest(measured):
+    assert measured["lost"] == 0
