@@ -47,13 +47,22 @@ def theta_of(p: capi.HoleParams) -> np.ndarray:
 
 def packed(params) -> C.Array:
     """The parameter records of several views, side by side as the C ABI takes them."""
-    return params if isinstance(params, C.Array) else (capi.HoleParams * len(params))(*params)
+    if isinstance(params, C.Array) and params._type_ is capi.HoleParams:
+        return params
+    params = list(params)
+    return (capi.HoleParams * len(params))(*params)
 
 
 def packed_with_theta(base: C.Array, theta: np.ndarray) -> C.Array:
-    """base's records with their five parameters (the records' first doubles) replaced: (n, 5)."""
-    out = type(base).from_buffer_copy(base)
-    np.frombuffer(out, np.float64).reshape(len(base), -1)[:, :5] = theta
+    """with_theta of base's records and theta's rows in turn, as many as there are of both: a row's values, five at
+    most, in place of the record's first doubles."""
+    if theta.ndim != 2:
+        raise TypeError(f"theta has {theta.ndim} dimensions: a row a view is wanted")
+    n, values = min(len(base), len(theta)), min(len(PARAM_NAMES), theta.shape[1])
+    out = (capi.HoleParams * n)()
+    C.memmove(out, base, C.sizeof(out))
+    if n:
+        np.frombuffer(out, np.float64).reshape(n, -1)[:, :values] = theta[:n, :values]
     return out
 
 
