@@ -326,3 +326,27 @@ def test_bloom_pyramid_equals_its_levels_one_by_one(lib, ctx, width, height):
     for p, w in zip(planes, want):
         np.testing.assert_array_equal(p.cpu().numpy().view(np.uint32), w.view(np.uint32))
     assert bool((bgra != 0).all())
+
+
+@pytest.mark.parametrize("bloom", [0.0, 4.5])
+@pytest.mark.parametrize("width,height", [(1, 1), (2, 1), (1, 2), (3, 2), (7, 9), (61, 40), (130, 65), (257, 511), (1919, 3)])
+def test_tone_mapped_pixels_equal_the_oracle(lib, ctx, width, height, bloom):
+    """The post pass's BGRA words over sizes whose last thread has one pixel and whose glow is clamped at a level
+    one texel wide, dark pixels and bright ones beside one another: the oracle's, word for word."""
+    import torch
+    rng = np.random.default_rng(width * 17 + height)
+    view = scenes.Scene("tone", scenes.hole_desc(0.5), scenes.camera(70.0, 30.0), width, height)
+    view.desc.bloom = bloom
+    frame, _, _ = scenes.frame(view)
+    hdr = np.zeros((height, width, 4), np.float32)
+    hdr[..., :3] = (rng.exponential(1.5, (height, width, 3)) ** 2).astype(np.float32) * (rng.random((height, width, 1)) < 0.7)
+    total = sum(int(frame.bloom[i][1]) * int(frame.bloom[i][2]) for i in range(frame.size[3]))
+    device = torch.from_numpy(hdr).cuda()
+    planes = [torch.zeros(total, dtype=torch.float32, device="cuda") for _ in range(3)]
+    bgra = torch.zeros((height, width), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    pointers = (C.c_void_p * 3)(*[p.data_ptr() for p in planes])
+    capi.check(lib.artfCudaPostLaunch(C.byref(frame), device.data_ptr(), pointers, bgra.data_ptr(),
+                                      lib.artfCudaStream(ctx)))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(bgra.cpu().numpy().view(np.uint32), binding.post(frame, hdr))
