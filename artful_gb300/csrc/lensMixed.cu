@@ -43,6 +43,7 @@
 #include "lensKernel.cuh"
 #include "lensMixed.h"
 #include "lensPairs.cuh"
+#include "lensParts.h"
 
 #include <string.h>
 
@@ -406,7 +407,7 @@ __device__ __forceinline__ int viewOf(const MixedParams& p, int unit) {
 constexpr int kWeightClasses = 9; /* steps / 8 up to 64: the probe stops there (all heavier tiles, class 8) */
 constexpr int kProbeSteps = 64;
 constexpr int kHeavyClass = 5; /* 40 steps or more at a corner */
-constexpr int kHeavyRaysLog2 = 3, kCornersLog2 = 2;
+constexpr int kCornersLog2 = 2;
 
 /* The view a batch-wide tile belongs to: the last whose first tile is at or below it. */
 __device__ __forceinline__ int tileView(const MixedParams& p, int tile) {
@@ -538,22 +539,18 @@ __device__ __forceinline__ void mixedTiles(const MixedParams& p, const MixedView
     unsigned rounds = 0;
     clearMixed(tally);
     chained();
-    unsigned heavy = 0; /* the rays in heavy slots */
-    if (kSplit) {
-        for (int c = kHeavyClass; c < kWeightClasses; ++c) heavy += __ldcg(p.classes + c); /* (not __ldg: a read-only load could move above the wait) */
-        heavy = min(heavy, (unsigned)p.mostHeavy) << 5;
-    }
-    const unsigned heavyParts = heavy >> kHeavyRaysLog2;
-    const unsigned parts = heavyParts + (((unsigned)p.totalUnits - heavy) >> p.lanesLog2); /* 2^lanesLog2 rays each */
+    unsigned heavySlots = 0;
+    if (kSplit)
+        for (int c = kHeavyClass; c < kWeightClasses; ++c) heavySlots += __ldcg(p.classes + c); /* (not __ldg: a read-only load could move above the wait) */
+    const MixedParts q = partsOf<kSplit>((unsigned)p.totalUnits, heavySlots, (unsigned)p.mostHeavy, p.lanesLog2);
     for (;;) {
         unsigned part = 0;
         if (lane == 0) part = (unsigned)atomicAdd(p.counters + CQueue, 1ull);
         part = __shfl_sync(0xFFFFFFFFu, part, 0);
-        if (part >= parts) break;
+        if (part >= q.parts) break;
         /* (a tile's rays row by row: 8 x 4 pixels a part, 8 x 2, 8 x 1, 4 x 1 or 2 x 1) */
-        const bool split = kSplit && part < heavyParts;
-        const int lanesLog2 = split ? kHeavyRaysLog2 : p.lanesLog2;
-        const unsigned first = split ? part << lanesLog2 : heavy + ((part - heavyParts) << lanesLog2);
+        int lanesLog2;
+        const unsigned first = partFirst<kSplit>(q, part, p.lanesLog2, lanesLog2);
         const unsigned within = (first & 31u) + (unsigned)lane;
         const int slot = (int)(first >> 5);
         const MixedView* v = kOne ? one : p.views;
@@ -798,40 +795,11 @@ size_t mixedOrderBytes(int totalTiles, int totalUnits) {
     return kOrderHead + weights + (size_t)(totalUnits / 32) * sizeof(uint2);
 }
 
-/* The persistent grid, and how many rays a warp takes at a time: all of a slot's 32 while that gives every
- * resident warp one; for a frame too small for that, half as many, and so on, down to two, so that more
- * warps share the rays and each has fewer that part ways (a warp runs what any of its rays needs, and
- * rays of a small frame's neighbouring pixels part early: a 101 x 67 frame took 119 us by 32 rays, 84 by
- * 8, 80 by 4 or 2; at 1920 x 1080 a warp's 32 rays stay together, 30.2 of 32 lanes busy).  refillBatch
- * sets the most.
- * Heavy slots are split where warps take whole slots of 32, the fewer the more slots there are: a quarter of
- * the warps' number at three slots a warp, none from six on (us, whole slots against split: 320 x 180 99 and
- * 79, 384 x 216 104 and 80, 512 x 288 126 and 101, 640 x 360 114 and 97, 320 x 180 x 4 rays 155 and 115, 768 x
- * 432 180 and 156; at 960 x 540, 6.7 slots a warp, 143 and 150; at 1280 x 720, 11.8, splitting 304 slots 181
- * and 188). */
-struct MixedGrid {
-    int blocks, most, lanesLog2; /* the launch's blocks, and as many as are resident at once */
-    bool resident; /* every part has a warp at once: the order they start in makes no difference */
-    int mostHeavy; /* the heavy slots that are split at most, for a trace that orders its slots */
-};
-
 static MixedGrid mixedGrid(const TraceLaunch& l, int totalUnits, const void* kernel) {
     const int block = l.blockSize > 0 ? l.blockSize : 128;
     int perSm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, block, 0);
-    const long long grid = (long long)(perSm > 0 ? perSm : 1) * l.smCount, warps = grid * (block / 32);
-    MixedGrid g;
-    g.lanesLog2 = 5;
-    while (l.refillBatch > 0 && 1 << g.lanesLog2 > l.refillBatch) --g.lanesLog2;
-    while (g.lanesLog2 > 1 && (long long)(totalUnits >> g.lanesLog2) * 2 <= warps) --g.lanesLog2;
-    const long long parts = totalUnits >> g.lanesLog2, needed = (parts * 32 + block - 1) / block;
-    const long long slots = totalUnits >> 5, room = (6 * warps - slots) / 12;
-    g.mostHeavy = room > 0 && g.lanesLog2 == 5 ? (int)room : 0;
-    g.resident = parts <= warps;
-    g.most = (int)grid;
-    g.blocks = (int)(grid > needed ? needed : grid);
-    if (g.blocks < 1) g.blocks = 1;
-    return g;
+    return mixedGridOf(totalUnits, block, perSm, l.smCount, l.refillBatch);
 }
 
 /* A launch that may start while the stream's work before it drains: kernels that wait in chained(). */
