@@ -12,9 +12,9 @@
  * reference computes them, as a kernel parameter.
  *
  * Three launches: paintRows, a block a row of the gas, the sky or the dust; scaleGas; and the tables.
- * What bounds it is issue: a lattice lookup is four hashes of eleven integer instructions.  A row's slow lattices (ten of the gas's 21 lookups) have a few dozen columns, so their values
- * are hashed once a row into shared memory; columns wrap by a comparison, not a division; every period and
- * seed is a constant.  paintRows 97 us (86 % of the issue slots), the whole call 270 -> 126 us; before, one
+ * What bounds it is issue: a lattice lookup is four hashes of eleven integer instructions.  A row's slow
+ * lattices (ten of the gas's 21 lookups) have a few dozen columns, so their values are hashed once a row into
+ * shared memory; columns wrap by a comparison, not a division; every period and seed is a constant.  paintRows 97 us (86 % of the issue slots), the whole call 270 -> 126 us; before, one
  * thread added the sums (1024 dependent double additions) and the tables and scratch were copied and
  * allocated in every call. */
 #include "nvtxRange.h"

@@ -140,11 +140,12 @@ template <> __device__ __forceinline__ float apart(float a, float b) { return __
 
 /* ---- the debug build's bounds checks -------------------------------------------------------------
  * Built with ARTF_CUDA_DEBUG_BOUNDS, every table row or entry the shading reads is checked against its
- * own region of the map or fluid (not only the buffer, which the clamps below keep every read inside),
- * and every write against the frame or buffer it goes to.  The first index found outside is recorded in
- * the fault word a frame carries (the launch's CBoundsKind, CBoundsIndex counters) and the C ABI
- * returns ARTF_CUDA_EBOUNDS; the read still goes through the clamp, as in the release build, and the
- * write is skipped.  In the release build the checks compile to nothing. */
+ * own region of the map or fluid (not only the buffer), and every write against the frame or buffer it
+ * goes to.  The first index found outside is recorded in the fault word a frame carries (the launch's
+ * CBoundsKind, CBoundsIndex counters) and the C ABI returns ARTF_CUDA_EBOUNDS; the read is made as in the
+ * release build, inside the buffer (its index is held where it is formed, by placeOf, a NaN's too, or
+ * clamped, for the sky's rows and the colours and in units that define ARTF_CLAMP_ROWS), and the write is
+ * skipped.  In the release build the checks compile to nothing. */
 enum BoundsKind : uint32_t {
     kBoundsGasRow = 1, kBoundsFluidRow, kBoundsDustRow, kBoundsSkyRow, kBoundsRingRow, kBoundsColour,
     kBoundsPixel, kBoundsRayPlane, kBoundsRayEnd

@@ -31,7 +31,7 @@
  * one another, so a wide step serves most of a warp at a time, and a ray's step costs nothing for the
  * schedule's sake.  (Lanes that waited for full rounds of wide steps and were refilled one by one, as an
  * FP64 wide step wanted, paid 80 thread instructions a step in votes and flags: 2.15 against 1.61 ms for the
- * 1080p x 4 frame, 7.63 against 5.51 for 64 views.)  What a step costs is issue slots (76 % of them used, FMA
+ * 1080p x 4 frame, 7.63 against 5.51 for 64 views.)  What a step costs is issue slots (75 % of them used, FMA
  * pipe 55 % busy), so the FP32 step runs its coordinates in pairs with packed instructions (nystromStep: 1.86
  * -> 1.76 ms), the wide step is one code path (1.74 -> 1.61 with the counts out of registers) and each float
  * rounding is written out or pinned (ARTF_PINNED_FMA): whatever registers a kernel is given, its images are

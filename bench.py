@@ -44,16 +44,16 @@ WORKLOAD = "kerr-hole 1920x1080, 4 jittered rays/px, a=0.998, r_obs=50 M, i=85 d
 # Kernels one mixed frame launches: the tile probe, the heavy-first order, the trace, the ray-plane sum.
 LAUNCHES_PER_MIXED_FRAME = 4
 # DRAM bytes (read + write) of one launch of the mixed trace kernel at this workload, from one ncu
-# capture (dram__bytes_read.sum 17.23 MB + dram__bytes_write.sum 73.36 MB): the map read once, and the
+# capture (dram__bytes_read.sum 17.34 MB + dram__bytes_write.sum 73.65 MB): the map read once, and the
 # part of the 133 MB of ray planes that leaves L2 before the sum reads it back.
-TRACE_TRAFFIC_BYTES = 90_593_280
+TRACE_TRAFFIC_BYTES = 90_991_360
 TRACE_TRAFFIC_GEODESICS = 1920 * 1080 * 4
 FLOPS_WIDE_RADIAL = 61  # lensFlops.h: a whole radial sub-step in the horizon's band (spin != 0)
 # How busy the mixed trace keeps its pipes, from one ncu --set full capture of its kernel at 960x540 x 4
 # (the counted work above counts a double-float operation, some 3 to 10 FP32 instructions, as one): the
 # FP64 pipe's instructions, the FP32 FMA pipe's cycles, the integer pipe's instructions and the
 # schedulers' issue slots, of peak.
-MIXED_PIPES_BUSY = {"fp64": 0.184, "fp32_fma": 0.523, "alu": 0.424, "issue": 0.734,
+MIXED_PIPES_BUSY = {"fp64": 0.170, "fp32_fma": 0.518, "alu": 0.404, "issue": 0.718,
                     "source": "ncu sm__inst_executed_pipe_fp64, sm__pipe_fma_cycles_active, sm__inst_executed_pipe_alu, "
                               "smsp__issue_active "
                               "of traceMixedOneAll at 960x540 x 4"}
