@@ -462,7 +462,9 @@ cudaError_t follow(ArtfCudaFluid* f, void (*kernel)(P...), unsigned blocks, unsi
     early.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(blocks), c.blockDim = dim3(threads), c.stream = f->stream, c.attrs = &early, c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, P(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError(); /* (or the next launch's check would report it) */
+    return e;
 }
 
 static_assert(START_EDDIES % EDDIES_A_LAUNCH + EDDIES_A_STEP <= EDDIES_A_LAUNCH, "the last launch holds both");

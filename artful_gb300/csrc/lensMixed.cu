@@ -810,7 +810,9 @@ static cudaError_t follow(cudaStream_t stream, void (*kernel)(P...), dim3 grid, 
     early.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c = {};
     c.gridDim = grid, c.blockDim = dim3((unsigned)block), c.stream = stream, c.attrs = &early, c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, P(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError(); /* (or the next launch's check would report it) */
+    return e;
 }
 
 cudaError_t launchMixedTable(const TraceLaunch& l, const void* deviceTable, int viewCount, int totalUnits,

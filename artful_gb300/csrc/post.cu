@@ -47,7 +47,9 @@ cudaError_t follow(cudaStream_t stream, void (*kernel)(P...), dim3 grid, int blo
     early.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c = {};
     c.gridDim = grid, c.blockDim = dim3((unsigned)block), c.stream = stream, c.attrs = &early, c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, P(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError(); /* (or the next launch's check would report it) */
+    return e;
 }
 
 /* software.c:334-351: level 0 from the frame's light. */

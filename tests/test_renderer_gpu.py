@@ -350,3 +350,25 @@ def test_tone_mapped_pixels_equal_the_oracle(lib, ctx, width, height, bloom):
                                       lib.artfCudaStream(ctx)))
     torch.cuda.synchronize()
     np.testing.assert_array_equal(bgra.cpu().numpy().view(np.uint32), binding.post(frame, hdr))
+
+
+def test_a_refused_launch_is_reported_once(lib, ctx):
+    """A frame taller than a launch's grid may be: the post pass reports it, and what is called next is none the
+    worse."""
+    import torch
+    width, height = 1, 70000
+    view = scenes.Scene("tall", scenes.hole_desc(0.5), scenes.camera(70.0, 30.0), width, height)
+    tall, _, _ = scenes.frame(view)
+    hdr = torch.zeros((height, width, 4), dtype=torch.float32, device="cuda")
+    planes = [torch.zeros(int(tall.bloom[0][1]) * int(tall.bloom[0][2]), dtype=torch.float32, device="cuda") for _ in range(3)]
+    bgra = torch.zeros((height, width), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    pointers = (C.c_void_p * 3)(*[p.data_ptr() for p in planes])
+    assert tall.size[3] == 1
+    assert lib.artfCudaPostLaunch(C.byref(tall), hdr.data_ptr(), pointers, bgra.data_ptr(), lib.artfCudaStream(ctx)) != 0
+    small = scenes.Scene("small", scenes.hole_desc(0.5), scenes.camera(70.0, 30.0), 16, 9)
+    frame, frame64, clamped = scenes.frame(small)
+    g.set_inputs(lib, ctx, scenes.synth_map(lib, clamped, 1, 3.0), scenes.unit_fluid())
+    for precision in (capi.EXACT, capi.MIXED):
+        light, _ = g.trace(lib, ctx, frame, frame64, precision)
+        assert np.isfinite(light).all()
