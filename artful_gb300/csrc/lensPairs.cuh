@@ -11,7 +11,7 @@
  * two of the high one) only where the value goes on into a sum it is a small part of, or meets roundings larger than
  * it would save: there the error against exact values is the same with and without, to a per cent in every quantile
  * from the median (2^-46.9 for the coefficients) to 99.9 %, over spins, inclinations and distances of the scenes'
- * range (the host test measures it).  A 1080p x 4 frame takes 1364 us so, 64 views 4790; with every result
+ * range (the host test measures it).  A 1080p x 4 frame takes 1364 us so, 64 views 4600-4700; with every result
  * renormalised and the sums in their plain form 1451 and 5200.  Left out everywhere it was 1306 and 4480, and the
  * coefficients' errors half as large again in the median and twice at 99.9 %.
  * Compiles on the host too, where the test runs it. */
